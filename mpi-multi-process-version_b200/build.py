@@ -42,7 +42,7 @@ UNITS = [
     ("unet.o", "unet_kernels.cu", []),
 ]
 
-HEADERS = ["lbm_internal.h", "lbm_handle.h", "lbm_march.cuh"]
+HEADERS = ["lbm_internal.h", "lbm_handle.h", "lbm_march.cuh", "lbm_march2d.cuh", "lbm_node2d.cuh"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:
@@ -57,7 +57,7 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
     cc = nvcc()
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", h)
                                                         for h in ("lbm_b200.h", "lbm_surrogate.h")]
-    objs = []
+    objs, cmds = [], []
     for obj, src, extra in UNITS:
         o = os.path.join(BUILD, obj)
         s = os.path.join(CSRC, src)
@@ -68,7 +68,12 @@ def build(verbose: bool = False, force: bool = False, ptxas_info: bool = False) 
                 cmd.insert(1, "-Xptxas=-v")
             if verbose:
                 print(" ".join(cmd), file=sys.stderr)
-            subprocess.check_call(cmd)
+            cmds.append(cmd)
+    # the units compile side by side
+    running = [subprocess.Popen(cmd) for cmd in cmds]
+    failed = [cmd for cmd, p in zip(cmds, running) if p.wait() != 0]
+    if failed:
+        raise subprocess.CalledProcessError(1, failed[0])
     if force or _stale(LIB, objs):
         cmd = [cc, *ARCH, "-shared", "-o", LIB, *objs]
         if verbose:

@@ -8,7 +8,8 @@
 //     that splits the total work into equal contiguous shares, one per block;
 //     the per-cavity geometry, TMA descriptors and buffers come from tables
 //     in device memory;
-//   * steps between checks are replayed from 2-step CUDA graphs;
+//   * a launch advances up to four steps (2D, fast build) and launches between
+//     checks are replayed in pairs from CUDA graphs;
 //   * lbm_batch_run applies the reference's stop test per cavity (errorU and
 //     errorT at most eps at a check, 2M:307) and drops stopped cavities
 //     from the work list;
@@ -56,6 +57,7 @@ struct lbm_batch {
     int use_graphs = 1;
     double growth = 0.0;           // residual growth factor that stops a member in lbm_batch_run (0: off)
     int storages = 0;              // LBM_BATCH_OPT_STORAGES: storages lbm_batch_tune may pick (0: the current)
+    int levels = 1;                // time steps a 2D multi-step launch advances (fast build)
     int pdl = 1;                   // LBM_BATCH_OPT_PDL: programmatic dependent launch of the step kernels
     Geo *d_geo = nullptr;
     TmapSet *d_maps = nullptr;
@@ -80,12 +82,30 @@ struct lbm_batch {
     cudaGraphExec_t run_graph[2] = {nullptr, nullptr};  // check periods of lbm_batch_run from cur = 0 / 1
     int run_graph_period = 0;
     int64_t run_graph_launches = 0;  // kernels one replay of a check-period graph launches
-    int64_t graph_launches = 0;      // kernels one replay of a 2-step graph launches
+    int64_t graph_launches = 0;      // kernels one replay of a step graph launches
     int64_t active_nodes = 0;
     RunCtl *d_ctl = nullptr;       // run state of every member (member i's bufs.ctl = d_ctl + i)
     int *d_idx = nullptr;          // the members of a run (its mask), for the batched check
     int nidx = 0;
 };
+
+// time steps of a multi-step launch of the 2D kernel (the exact build and 3D: 1).
+// Four levels share the launch and a segment's pipeline fill; large FP32 batches,
+// bound by issue rather than by HBM, do better with the narrower halo of two.
+// Measured, us a step at 1 / 2 / 4 levels (64 columns): FP64 sweep of 32 cavities
+// 390 / 237 / 206, 16 squares 25.1 / 20.3 / 19.2, one 7.27 / 5.26 / 4.78; FP32
+// 244 / 158 / 165, 17.5 / 15.9 / 15.5, 7.26 / 4.76 / 4.02.
+static int batch_levels(const lbm_batch *b)
+{
+    if (b->dim != 2 || b->mode == LBM_MODE_EXACT) return 1;
+    int64_t nodes = 0;
+    for (const lbm_handle *h : b->cav) nodes += h->geo.nnode;
+    return b->storage == LBM_STORE_F32 && nodes >= (1 << 21) ? 2 : 4;
+}
+
+// the kernel's columns for a tile width: the fast build's rows have 64 or 128
+// (tile 32 caps the strips at 32 of the 64)
+static int W_cols(int tile) { return tile < 64 ? 64 : tile; }
 
 static void drop_graphs(lbm_batch *b)
 {
@@ -218,7 +238,7 @@ static int build_tables(lbm_batch *b)
     const int TX = d3 ? 32 : b->tile;
     std::vector<TmapSet> maps(2 * (size_t)b->n);
     for (int i = 0; i < b->n; ++i)
-        if (!encode_maps_tx(b->cav[i], d3 ? 0 : TX, &maps[2 * (size_t)i]))
+        if (!encode_maps_tx(b->cav[i], d3 ? 0 : (b->mode == LBM_MODE_EXACT ? TX : W_cols(TX)), &maps[2 * (size_t)i]))
             return set_error(LBM_ERR_UNSUPPORTED, "batch: TMA descriptors for cavity %d could not be encoded", i);
     BCU(cudaMemcpyAsync(b->d_maps, maps.data(), sizeof(TmapSet) * maps.size(), cudaMemcpyHostToDevice, b->stream));
     {
@@ -228,15 +248,24 @@ static int build_tables(lbm_batch *b)
         BCU(cudaMemcpyAsync(b->d_bufs, bufs.data(), sizeof(Bufs) * b->n, cudaMemcpyHostToDevice, b->stream));
     }
 
+    const bool fast2d = !d3 && b->mode != LBM_MODE_EXACT;
+    b->levels = batch_levels(b);
     struct Col {
         int cav, pos, ny;  // pos: 2D the strip's x-offset, 3D the tile index; ny: items (rows or slices)
     };
     std::vector<Col> cols;
+    std::vector<Strip2> strips;
     size_t ncols_all = 0;  // the columns of every member, active or not: the lists' capacity
     b->active_nodes = 0;
     for (int i = 0; i < b->n; ++i) {
         const Geo &g = b->cav[i]->geo;
-        const int nc = d3 ? ((g.nx + 31) / 32) * ((g.ny + kBatchTileY - 1) / kBatchTileY) : (g.nx + TX - 1) / TX;
+        int nc = d3 ? ((g.nx + 31) / 32) * ((g.ny + kBatchTileY - 1) / kBatchTileY) : (g.nx + TX - 1) / TX;
+        if (fast2d) {
+            const size_t n0 = strips.size();
+            strips_march2d(i, g.nx, 0, g.ny, g.ny, TX, b->levels, strips);
+            nc = (int)(strips.size() - n0);
+            if (!b->active[i]) strips.resize(n0);
+        }
         ncols_all += nc;
         if (!b->active[i]) continue;
         for (int c = 0; c < nc; ++c) cols.push_back({i, d3 ? c : c * TX, d3 ? g.nz : g.ny});
@@ -264,16 +293,24 @@ static int build_tables(lbm_batch *b)
         }
         const int bps = d3 ? (b->mode == LBM_MODE_EXACT ? exact::march_batch3d_blocks_per_sm(sto)
                                                          : fast::march_batch3d_blocks_per_sm(sto))
-                           : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(sto, TX)
-                                                        : fast::march_batch_blocks_per_sm(sto, TX));
+                           : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(sto, TX, 1)
+                                                        : fast::march_batch_blocks_per_sm(sto, W_cols(TX), b->levels));
         if (bps <= 0) return set_error(LBM_ERR_UNSUPPORTED, "batch kernel with tile %d cannot be resident", TX);
         const int64_t G = b->nblocks_opt > 0 ? b->nblocks_opt : (int64_t)bps * sms;
         // equal contiguous shares of the (column, item) items; blocks past the work get none
         std::vector<int4> segs;
         std::vector<int> off(G + 1, 0);
+        if (fast2d) {
+            std::vector<Strip2> mine;
+            for (const Strip2 &st : strips)
+                if (b->cav[st.cav]->p.storage == sto) mine.push_back(st);
+            plan_march2d(mine, b->levels, (int)G, segs, off);
+            sc.clear();
+            stotal = 0;
+        }
         size_t c = 0;
         int64_t colbase = 0;  // first item of column c
-        for (int64_t blk = 0; blk < G; ++blk) {
+        for (int64_t blk = 0; blk < G && !fast2d; ++blk) {
             off[blk] = (int)segs.size();
             const int64_t lo = stotal * blk / G, hi = stotal * (blk + 1) / G;
             int64_t u = lo;
@@ -323,52 +360,77 @@ static int build_tables(lbm_batch *b)
 // one step of every member on the work lists: one persistent kernel per
 // population storage present; pdl: launched as a programmatic dependent of the
 // stream's previous kernel
-static cudaError_t launch_list(lbm_batch *b, int sto, int cur, int wm, bool pdl, cudaStream_t s)
+static cudaError_t launch_list(lbm_batch *b, int sto, int cur, int wm, int levels, bool pdl, cudaStream_t s)
 {
     const lbm_batch::WorkList &W = b->wl[sto];
     if (b->dim == 3)
         return b->mode == LBM_MODE_EXACT ? exact::march_batch3d(sto, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s)
                                          : fast::march_batch3d(sto, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s);
-    return b->mode == LBM_MODE_EXACT ? exact::march_batch(sto, W.tx, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s)
-                                     : fast::march_batch(sto, W.tx, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s);
+    return b->mode == LBM_MODE_EXACT ? exact::march_batch(sto, W.tx, W.dev, W.nblocks, cur, wm, b->d_err, pdl, 1, s)
+                                     : fast::march_batch(sto, W_cols(W.tx), W.dev, W.nblocks, cur, wm, b->d_err, pdl,
+                                                         levels, s);
 }
 
 // with both storages present the two kernels run side by side (a fork onto
 // the second stream and a join), so a step costs one kernel's latency; a
 // single list's kernels follow one another as programmatic dependents
-static cudaError_t launch_step(lbm_batch *b, int cur, int wm)
+static cudaError_t launch_step(lbm_batch *b, int cur, int wm, int levels = 1)
 {
     const bool a = b->wl[0].nblocks > 0, c = b->wl[1].nblocks > 0;
     if (a && c) {
         cudaError_t e = cudaEventRecord(b->ev_fork, b->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream2, b->ev_fork, 0);
-        if (e == cudaSuccess) e = launch_list(b, 1, cur, wm, false, b->stream2);
-        if (e == cudaSuccess) e = launch_list(b, 0, cur, wm, false, b->stream);
+        if (e == cudaSuccess) e = launch_list(b, 1, cur, wm, levels, false, b->stream2);
+        if (e == cudaSuccess) e = launch_list(b, 0, cur, wm, levels, false, b->stream);
         if (e == cudaSuccess) e = cudaEventRecord(b->ev_join, b->stream2);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->ev_join, 0);
         return e;
     }
-    if (a) return launch_list(b, 0, cur, wm, b->pdl != 0, b->stream);
-    if (c) return launch_list(b, 1, cur, wm, b->pdl != 0, b->stream);
+    if (a) return launch_list(b, 0, cur, wm, levels, b->pdl != 0, b->stream);
+    if (c) return launch_list(b, 1, cur, wm, levels, b->pdl != 0, b->stream);
     return cudaSuccess;
 }
 
-// a 2-step graph starting from buffer `cur`
+// n steps from buffer `cur`, which ends at (cur + n) & 1: pairs of multi-step
+// launches (each flips the buffers once for its even number of steps), then
+// single steps, the last one alone with the macroscopic fields if with_macro
+static cudaError_t launch_steps(lbm_batch *b, int cur, int n, bool with_macro)
+{
+    int left = with_macro ? n - 1 : n;
+    const int group = 2 * b->levels;
+    cudaError_t e = cudaSuccess;
+    if (b->levels > 1)
+        for (; left >= group && e == cudaSuccess; left -= group)
+            for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+                e = launch_step(b, cur, 0, b->levels);
+                cur = 1 - cur;
+            }
+    for (; left > 0 && e == cudaSuccess; --left) {
+        e = launch_step(b, cur, 0);
+        cur = 1 - cur;
+    }
+    if (with_macro && e == cudaSuccess) e = launch_step(b, cur, 1);
+    return e;
+}
+
+// steps per replayed graph (two launches; even, so a replay leaves `cur` as it was)
+static int graph_steps(const lbm_batch *b) { return 2 * b->levels; }
+
+// a graph of graph_steps(b) steps starting from buffer `cur`
 static int get_graph(lbm_batch *b, int cur, cudaGraphExec_t *out)
 {
     if (!b->graph[cur]) {
         cudaGraph_t g = nullptr;
         const int64_t launches0 = g_launches;
         BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e1 = launch_step(b, cur, 0);
-        cudaError_t e2 = launch_step(b, 1 - cur, 0);
-        cudaError_t e3 = cudaStreamEndCapture(b->stream, &g);
+        const cudaError_t e1 = launch_steps(b, cur, graph_steps(b), false);
+        const cudaError_t e3 = cudaStreamEndCapture(b->stream, &g);
         b->graph_launches = g_launches - launches0;
         g_launches = launches0;  // counted when replayed
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
+        if (e1 != cudaSuccess || e3 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             return set_error(LBM_ERR_CUDA, "batch graph capture failed: %s",
-                             cudaGetErrorString(e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3)));
+                             cudaGetErrorString(e1 != cudaSuccess ? e1 : e3));
         }
         cudaError_t e = cudaGraphInstantiate(&b->graph[cur], g, 0);
         cudaGraphDestroy(g);
@@ -410,24 +472,20 @@ extern "C" int lbm_batch_step(lbm_batch *b, int32_t nsteps)
         if (st) return st;
     }
     int done = 0;
-    // whole 2-step graphs for all but the last step, then the last step with the macroscopic output
+    // whole graphs for all but the last step, then the last ones, the very last with the macroscopic output
     if (b->use_graphs) {
-        while (nsteps - done > 2) {
+        const int gs = graph_steps(b);
+        while (nsteps - done > gs) {
             cudaGraphExec_t g;
             int st = get_graph(b, cur, &g);
             if (st) return st;
             BCU(cudaGraphLaunch(g, b->stream));
             g_launches += b->graph_launches;
-            done += 2;
+            done += gs;
         }
     }
-    while (done < nsteps) {
-        BCU(launch_step(b, cur, done == nsteps - 1));
-        cur = 1 - cur;
-        ++done;
-    }
-    // each graph replay flips the buffers twice, each single launch once
-    const int final_cur = cur;
+    BCU(launch_steps(b, cur, nsteps - done, true));
+    const int final_cur = (cur + nsteps - done) & 1;
     for (int i = 0; i < b->n; ++i)
         if (b->active[i]) {
             b->cav[i]->cur = final_cur;
@@ -519,8 +577,7 @@ static int batch_period_graph(lbm_batch *b, int cur, int period, cudaGraphExec_t
         cudaGraph_t g = nullptr;
         const int64_t launches0 = g_launches;
         BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaSuccess;
-        for (int i = 0; i < period && e == cudaSuccess; ++i) e = launch_step(b, (cur + i) & 1, i == period - 1);
+        cudaError_t e = launch_steps(b, cur, period, true);
         if (e == cudaSuccess) e = run_check_batch(b->dev, b->d_idx, b->nidx, period, b->stream);
         const cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
         b->run_graph_launches = g_launches - launches0;
@@ -642,12 +699,12 @@ static int batch_run(lbm_batch *b, const int32_t *mask, int32_t max_steps, int32
                 }
                 g_launches += b->run_graph_launches;
             } else {
-                for (int i = 0; i < k && !st; ++i) {
-                    cudaError_t e = launch_step(b, (cur + i) & 1, i == k - 1);
-                    if (e != cudaSuccess) st = set_error(LBM_ERR_CUDA, "batch step: %s", cudaGetErrorString(e));
+                cudaError_t e = launch_steps(b, cur, k, true);
+                if (e != cudaSuccess) {
+                    st = set_error(LBM_ERR_CUDA, "batch step: %s", cudaGetErrorString(e));
+                    break;
                 }
-                if (st) break;
-                cudaError_t e = run_check_batch(b->dev, b->d_idx, b->nidx, k, b->stream);
+                e = run_check_batch(b->dev, b->d_idx, b->nidx, k, b->stream);
                 if (e != cudaSuccess) {
                     st = set_error(LBM_ERR_CUDA, "batch check: %s", cudaGetErrorString(e));
                     break;
@@ -861,9 +918,10 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
     BCU(cudaSetDevice(b->device));
     int sms = 0;
     BCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
-    const int tiles2[3] = {32, 64, 128}, tiles3[1] = {32};  // 3D: the tile is fixed at 32 x kBatchTileY
+    // 3D: the tile is fixed at 32 x kBatchTileY; the fast build's 2D rows have 64 or 128 columns
+    const int tiles2[3] = {64, 128, 32}, tiles3[1] = {32};
     const int *tiles = b->dim == 3 ? tiles3 : tiles2;
-    const int ntile = b->dim == 3 ? 1 : 3;
+    const int ntile = b->dim == 3 ? 1 : (b->mode == LBM_MODE_EXACT ? 3 : 2);
     double best = -1.0;
     int best_tile = b->tile, best_nb = 0;
     cudaEvent_t e0, e1;
@@ -874,8 +932,8 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
         const int t = tiles[ti];
         const int bps = b->dim == 3 ? (b->mode == LBM_MODE_EXACT ? exact::march_batch3d_blocks_per_sm(b->storage)
                                                                  : fast::march_batch3d_blocks_per_sm(b->storage))
-                                    : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(b->storage, t)
-                                                                 : fast::march_batch_blocks_per_sm(b->storage, t));
+                                    : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(b->storage, t, 1)
+                                                                 : fast::march_batch_blocks_per_sm(b->storage, W_cols(t), batch_levels(b)));
         if (bps <= 0) continue;
         const int cands[2] = {bps, bps > 1 ? bps / 2 : 0};
         for (int c : cands) {

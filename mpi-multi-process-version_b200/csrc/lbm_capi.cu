@@ -323,6 +323,8 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
     if (!enc) return false;
     const Geo &g = h->geo;
     const MarchShape ms = march_shape(g.dim, h->p.storage, tx, h->tiley);
+    // the fast build's 2D march: one box of all planes per row
+    const int wb = g.dim == 2 && h->p.mode != LBM_MODE_EXACT ? march2d_box(h->p.storage, tx ? tx : h->nt) : 0;
     const CUtensorMapDataType dtype =
         h->p.storage == LBM_STORE_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const cuuint64_t es = h->esize;
@@ -347,7 +349,7 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
                 const int cc = c & 1;
                 const cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)nplanes};
                 const cuuint64_t strides[2] = {(cuuint64_t)g.pitch * es, (cuuint64_t)g.plane * es};
-                const cuuint32_t box[3] = {(cuuint32_t)ms.bx[cc], 1, 1};
+                const cuuint32_t box[3] = {(cuuint32_t)(wb ? wb : ms.bx[cc]), 1, (cuuint32_t)(wb ? nplanes : 1)};
                 const cuuint32_t estr[3] = {1, 1, 1};
                 r = enc(m, dtype, 3, h->bufs.pop[buf], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -369,7 +371,7 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
         } else {
             const cuuint64_t dims[2] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny};
             const cuuint64_t strides[1] = {(cuuint64_t)g.pitch * cs};
-            const cuuint32_t box[2] = {(cuuint32_t)ms.TX, 1};
+            const cuuint32_t box[2] = {(cuuint32_t)(wb ? wb : ms.TX), 1};
             const cuuint32_t estr[2] = {1, 1};
             r = enc(&out[buf].fmap, ftype, 2, h->bufs.F[buf], dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -465,20 +467,80 @@ int lbm::plan_march3d(int ntiles, int nz, int nblocks, int kind, std::vector<int
     return (int)off.size() - 1;
 }
 
-// plan the 3D march for grid G and upload it; sets h->nblocks
-static int upload_plan3d(lbm_handle *h, int G)
+// ---------------------------------------------------------------------------
+// 2D march work plan (fast build)
+// ---------------------------------------------------------------------------
+void lbm::strips_march2d(int cav, int nx, int lo, int hi, int ny, int nt, int levels, std::vector<Strip2> &out)
+{
+    const int halo = levels - 1;
+    // cuts on 8-element boundaries: a strip's rows then start and end on whole
+    // 32-byte sectors in either storage, so no sector is written in two parts
+    // (measured at 2048^2 FP64, 58-column strips: 157 us a step, on sector boundaries 107 us)
+    auto cut = [&](int k, int n) {
+        if (k <= 0) return 0;
+        if (k >= n) return nx;
+        return std::min((int)(((int64_t)k * nx / n + 4) / 8 * 8), (nx - 2) / 2 * 2);
+    };
+    auto fits = [&](int n) {
+        for (int k = 0; k < n; ++k) {
+            const int a = cut(k, n), b = cut(k + 1, n);
+            if (b - a < 2 || std::min(b + halo, nx) - std::max(a - halo, 0) > nt) return false;
+        }
+        return true;
+    };
+    int S = std::max(1, nx / nt);
+    while (!fits(S)) ++S;
+    for (int k = 0; k < S; ++k) out.push_back({cav, cut(k, S), cut(k + 1, S) - cut(k, S), lo, hi, ny});
+}
+
+int lbm::plan_march2d(const std::vector<Strip2> &strips, int levels, int nblocks, std::vector<int4> &segs,
+                      std::vector<int> &off)
+{
+    const int64_t ov = 3 * levels - 1;
+    // blocks needed with at most `budget` iterations each; min_rows: a segment
+    // is not worth its overhead below that.  A wall row's one-sided stencil
+    // needs two more rows of its own segment's level below, so no cut leaves
+    // the first or the last row of a cavity alone.
+    auto fill = [&](int64_t budget, bool emit) -> int64_t {
+        int64_t blocks = 0, left = 0;
+        for (const Strip2 &st : strips) {
+            int r = st.lo;
+            while (r < st.hi) {
+                if (left < ov + std::min(4, st.hi - r)) {
+                    if (emit && blocks < nblocks) off[blocks] = (int)segs.size();
+                    ++blocks;
+                    left = budget;
+                }
+                int e = (int)std::min<int64_t>(st.hi, r + std::max<int64_t>(left - ov, 4));
+                if (st.hi - e == 1) e = e - r > 3 ? e - 1 : st.hi;
+                if (emit) segs.push_back(make_int4(st.cav | (int)((uint32_t)st.w << 24), st.x0, r, e));
+                left -= (e - r) + ov;
+                r = e;
+            }
+        }
+        return blocks;
+    };
+    segs.clear();
+    off.assign((size_t)nblocks + 1, 0);
+    int64_t total = 0, tall = 1;
+    for (const Strip2 &st : strips) {
+        total += st.hi - st.lo + ov;
+        tall = std::max<int64_t>(tall, st.hi - st.lo);
+    }
+    int64_t a = std::max<int64_t>(ov + 4, total / nblocks), b = total + ov + 4;
+    while (a < b) {
+        const int64_t m = (a + b) / 2;
+        if (fill(m, false) <= nblocks) b = m;
+        else a = m + 1;
+    }
+    const int64_t used = fill(a, true);
+    for (int64_t k = used; k <= nblocks; ++k) off[k] = (int)segs.size();
+    return (int)used;
+}
+
+static int upload_segs(lbm_handle *h, const std::vector<int4> &segs, const std::vector<int> &off)
 {
     CU(cudaStreamSynchronize(h->stream));  // no launch in flight reads the old plan
-    const MarchShape ms = march_shape(3, h->p.storage, 0, h->tiley);
-    const int ntiles = ((h->geo.nx + ms.TX - 1) / ms.TX) * ((h->geo.ny + ms.TY - 1) / ms.TY);
-    std::vector<int4> segs;
-    std::vector<int> off;
-    // the slices the handle computes: all of them, or a slab's own [klo, khi)
-    const int nb = lbm::plan_march3d(ntiles, h->geo.khi - h->geo.klo, G, h->plan_opt, segs, off);
-    for (int4 &s : segs) {
-        s.y += h->geo.klo;
-        s.z += h->geo.klo;
-    }
     if (segs.size() > h->msegs_cap) {
         if (h->d_msegs) cudaFree(h->d_msegs);
         h->d_msegs = nullptr;
@@ -497,8 +559,75 @@ static int upload_plan3d(lbm_handle *h, int G)
     }
     CU(cudaMemcpy(h->d_msegs, segs.data(), sizeof(int4) * segs.size(), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(h->d_msegoff, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
+    return LBM_OK;
+}
+
+// plan the 3D march for grid G and upload it; sets h->nblocks
+static int upload_plan3d(lbm_handle *h, int G)
+{
+    const MarchShape ms = march_shape(3, h->p.storage, 0, h->tiley);
+    const int ntiles = ((h->geo.nx + ms.TX - 1) / ms.TX) * ((h->geo.ny + ms.TY - 1) / ms.TY);
+    std::vector<int4> segs;
+    std::vector<int> off;
+    // the slices the handle computes: all of them, or a slab's own [klo, khi)
+    const int nb = lbm::plan_march3d(ntiles, h->geo.khi - h->geo.klo, G, h->plan_opt, segs, off);
+    for (int4 &s : segs) {
+        s.y += h->geo.klo;
+        s.z += h->geo.klo;
+    }
+    int st = upload_segs(h, segs, off);
+    if (st) return st;
     h->nblocks = nb;
     return LBM_OK;
+}
+
+// The fast build's 2D march: levels per launch, columns per block, work plan.
+// Few nodes: four levels, which share the launch and the pipeline's fill; from
+// 2^19 on two levels, whose halo is narrower (the state no longer fits L2, and
+// two already halve its traffic).  Measured, FP64, us a step (columns x levels
+// 64x4 / 128x2 / 64x2): 384^2 6.9 / 7.8 / 7.2, 700x900 18.4 / 18.5 / 19.7, 1024^2
+// 29.0 / 28.2 / 30.1, 2048^2 108 / 112 / 106; FP32: 512^2 7.7 / 8.0 / 8.2, 1023x771
+// 17.3 / 16.9 / 17.7, 2048^2 89 / 77 / 79.
+static int resolve_2d(lbm_handle *h)
+{
+    const Geo &g = h->geo;
+    const bool slab = g.jlo > 0 || g.jhi < g.ny;  // ghost rows are good for one step only
+    const bool f64 = h->p.storage == LBM_STORE_F64;
+    const int levels = slab ? 1 : (g.nnode < (1 << 19) ? 4 : 2);
+    const int nt = g.nnode < (1 << 19) || (f64 && g.nnode >= (1 << 21)) ? 64 : 128;
+    const int bps = fast::march_blocks_per_sm(g, h->p.storage, h->tiley, nt, levels);
+    if (bps <= 0 || fast::march_blocks_per_sm(g, h->p.storage, h->tiley, nt, 1) <= 0) {
+        h->levels = 0;
+        return LBM_OK;
+    }
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    h->nt = nt;
+    h->levels = levels;
+    h->slots = h->nblocks_opt > 0 ? h->nblocks_opt : bps * sms;
+    h->segs2.clear();
+    h->plan_dirty = true;  // planned by the init call or the first launch: a batch's members never need it
+    h->march_ok = lbm::encode_maps_tx(h, 0, h->tmaps);
+    return LBM_OK;
+}
+
+// the plan on the host
+static void plan_2d(lbm_handle *h)
+{
+    if (!h->plan_dirty || !h->segs2.empty()) return;
+    const Geo &g = h->geo;
+    std::vector<lbm::Strip2> strips;
+    lbm::strips_march2d(0, g.nx, g.jlo, g.jhi, g.ny, h->nt, h->levels, strips);
+    h->nblocks = lbm::plan_march2d(strips, h->levels, h->slots, h->segs2, h->segoff2);
+}
+
+static int ensure_plan(lbm_handle *h)
+{
+    if (!h->plan_dirty) return LBM_OK;
+    plan_2d(h);
+    int st = upload_segs(h, h->segs2, h->segoff2);
+    if (!st) h->plan_dirty = false;
+    return st;
 }
 
 extern "C" int lbm_march_plan3d(int32_t ntiles, int32_t nz, int32_t nblocks, int32_t kind, int32_t *seg_count,
@@ -530,9 +659,21 @@ static int resolve_path(lbm_handle *h)
     if (h->kernel_opt == 2 && !ok)
         return fail(LBM_ERR_UNSUPPORTED, "march kernel not available for this shape / device");
     h->use_march = h->kernel_opt == 2 || (h->kernel_opt == 0 && ok && h->geo.nnode >= (1 << 15));
-    if (h->use_march) {
-        const int bps = h->p.mode == LBM_MODE_EXACT ? exact::march_blocks_per_sm(h->geo, h->p.storage, h->tiley)
-                                                   : fast::march_blocks_per_sm(h->geo, h->p.storage, h->tiley);
+    h->levels = 1;
+    h->plan_dirty = false;
+    const bool fast2d = h->p.dim == 2 && h->p.mode != LBM_MODE_EXACT;
+    if (fast2d && ok && h->kernel_opt != 1) {
+        int st = resolve_2d(h);
+        if (st) return st;
+        if (!h->levels || !h->march_ok) {
+            if (h->kernel_opt == 2) return fail(LBM_ERR_UNSUPPORTED, "march kernel cannot be resident");
+            h->levels = 1;
+            h->use_march = 0;
+        }
+    } else if (h->use_march) {
+        const int bps = h->p.mode == LBM_MODE_EXACT
+                            ? exact::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 128, 1)
+                            : fast::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 128, 1);
         if (bps <= 0) {
             if (h->kernel_opt == 2) return fail(LBM_ERR_UNSUPPORTED, "march kernel cannot be resident");
             h->use_march = 0;
@@ -632,6 +773,7 @@ extern "C" int lbm_create(const lbm_params *p, const double *x, const double *y,
     g.Snu = h->d.Snu; g.Sq = h->d.Sq; g.sig_k = h->d.sig_k; g.gbeta = h->d.gbeta;
     g.dt = p->dt; g.Thot = p->Thot; g.Tcold = p->Tcold; g.T0 = 0.5 * (p->Thot + p->Tcold);
     g.length_LB = p->length_LB;
+    relax_setup(g);
     tc_setup(g, c[p->dim == 2 ? 0 : 1]);
 
     // coordinates, weights, cell widths
@@ -755,6 +897,7 @@ extern "C" int lbm_init_reference(lbm_handle *h)
     if (st) return st;
     CU(launch_equilibrium(h, h->bufs.pop[h->cur]));
     if ((st = reset_run(h))) return st;
+    if (h->owns_stream && (st = ensure_plan(h))) return st;  // so that stepping itself uploads nothing
     CU(cudaStreamSynchronize(h->stream));
     h->phase = 1;
     return LBM_OK;
@@ -775,6 +918,7 @@ extern "C" int lbm_init_equilibrium(lbm_handle *h, const double *rho, const doub
     if (st) return st;
     CU(launch_equilibrium(h, h->bufs.pop[h->cur]));
     if ((st = reset_run(h))) return st;
+    if (h->owns_stream && (st = ensure_plan(h))) return st;  // so that stepping itself uploads nothing
     CU(cudaStreamSynchronize(h->stream));
     h->phase = 1;
     return LBM_OK;
@@ -799,6 +943,7 @@ extern "C" int lbm_init_warm(lbm_handle *h, const double *rho, const double *u, 
     if (st) return st;
     CU(launch_equilibrium(h, h->bufs.pop[h->cur], 1));
     if ((st = reset_run(h))) return st;
+    if (h->owns_stream && (st = ensure_plan(h))) return st;  // so that stepping itself uploads nothing
     CU(cudaStreamSynchronize(h->stream));
     h->phase = 1;
     return LBM_OK;
@@ -818,19 +963,43 @@ int lbm::first_collision(lbm_handle *h)
     return LBM_OK;
 }
 
-// one fused step from buffer `cur` (asynchronous)
-static cudaError_t launch_one(lbm_handle *h, int cur, int wm)
+// `levels` fused steps from buffer `cur` in one launch (asynchronous)
+static cudaError_t launch_one(lbm_handle *h, int cur, int wm, int levels = 1)
 {
     const bool ex = h->p.mode == LBM_MODE_EXACT;
     Bufs &b = h->bufs;
     const int nxt = 1 - cur;
-    if (h->use_march)
+    if (h->use_march || levels > 1)
         return ex ? exact::march(h->geo, h->p.storage, h->tmaps[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm,
-                                 h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->stream)
+                                 h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->nt, 1, h->stream)
                   : fast::march(h->geo, h->p.storage, h->tmaps[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm,
-                                h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->stream);
+                                h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->nt, levels, h->stream);
     return ex ? exact::step(h->geo, h->p.storage, b.pop[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm, h->stream)
               : fast::step(h->geo, h->p.storage, b.pop[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm, h->stream);
+}
+
+// n steps from buffer `cur`, which ends at (cur + n) & 1: several steps per
+// launch, as many launches (modulo 2) as steps.  with_macro: the last step runs
+// alone and writes the macroscopic fields (it also leaves the state one step
+// older in the other buffer, where lbm_get_populations streams from).
+static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
+{
+    int left = with_macro ? n - 1 : n;
+    cudaError_t e = cudaSuccess;
+    if (h->levels > 1 && !h->resident) {
+        // an even number of levels: launches in pairs
+        for (; left >= 2 * h->levels && e == cudaSuccess; left -= 2 * h->levels)
+            for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+                e = launch_one(h, cur, 0, h->levels);
+                cur = 1 - cur;
+            }
+    }
+    for (; left > 0 && e == cudaSuccess; --left) {
+        e = launch_one(h, cur, 0);
+        cur = 1 - cur;
+    }
+    if (with_macro && e == cudaSuccess) e = launch_one(h, cur, 1);
+    return e;
 }
 
 void lbm::drop_graphs(lbm_handle *h)
@@ -847,27 +1016,40 @@ void lbm::drop_graphs(lbm_handle *h)
         }
 }
 
-// steps per replayed graph in lbm_step (even: a replay leaves `cur` as it was);
-// inside a graph consecutive march steps are programmatic dependents
-static constexpr int kGraphSteps = 8;
+// steps per replayed graph in lbm_step (even: a replay leaves `cur` as it was):
+// eight launches; inside a graph consecutive march steps are programmatic
+// dependents
+static int graph_steps(const lbm_handle *h) { return 8 * h->levels; }
 
-// a kGraphSteps-step graph starting from buffer `cur`, captured once per kernel choice
+// end the capture begun on h's stream: *out holds the instantiated graph and
+// *launches the kernels one replay launches.  e: the captured launches' status,
+// launches0: g_launches before them
+static int end_capture(lbm_handle *h, cudaError_t e, int64_t launches0, cudaGraphExec_t *out, int64_t *launches,
+                       const char *what)
+{
+    cudaGraph_t g = nullptr;
+    const cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
+    *launches = lbm::g_launches - launches0;
+    lbm::g_launches = launches0;  // counted when replayed
+    if (e != cudaSuccess || e2 != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return fail(LBM_ERR_CUDA, "%s graph capture: %s", what, cudaGetErrorString(e != cudaSuccess ? e : e2));
+    }
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "%s graph instantiate: %s", what, cudaGetErrorString(e));
+    return LBM_OK;
+}
+
+// a graph of graph_steps(h) steps starting from buffer `cur`, captured once per kernel choice
 static int step_graph(lbm_handle *h, int cur, cudaGraphExec_t *out)
 {
     if (!h->graph[cur]) {
-        cudaGraph_t g = nullptr;
+        const int64_t l0 = lbm::g_launches;
         CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e1 = cudaSuccess;
-        for (int k = 0; k < kGraphSteps && e1 == cudaSuccess; ++k) e1 = launch_one(h, (cur + k) & 1, 0);
-        const cudaError_t e3 = cudaStreamEndCapture(h->stream, &g);
-        lbm::g_launches -= kGraphSteps;  // counted when replayed
-        if (e1 != cudaSuccess || e3 != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            return fail(LBM_ERR_CUDA, "step graph capture: %s", cudaGetErrorString(e1 != cudaSuccess ? e1 : e3));
-        }
-        const cudaError_t e = cudaGraphInstantiate(&h->graph[cur], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "step graph instantiate: %s", cudaGetErrorString(e));
+        const cudaError_t e = launch_steps(h, cur, graph_steps(h), false);
+        int st = end_capture(h, e, l0, &h->graph[cur], &h->graph_launches, "step");
+        if (st) return st;
     }
     *out = h->graph[cur];
     return LBM_OK;
@@ -880,6 +1062,7 @@ extern "C" int lbm_step(lbm_handle *h, int32_t nsteps)
     if (h->phase == 0) return fail(LBM_ERR_STATE, "lbm_step before an init call");
     if (nsteps == 0) return LBM_OK;
     int st = lbm::first_collision(h);
+    if (!st) st = ensure_plan(h);
     if (st) return st;
     int done = 0;
     if (h->resident && nsteps > 4) {
@@ -893,22 +1076,21 @@ extern "C" int lbm_step(lbm_handle *h, int32_t nsteps)
         h->itc += nsteps;
         return LBM_OK;
     }
-    // replay kGraphSteps-step graphs for all but the last step(s) (small
-    // domains are launch-bound), then single launches; the last step writes
-    // the macroscopic fields
+    // replay graphs for all but the last step(s) (small domains are
+    // launch-bound), then plain launches; the last step writes the macroscopic
+    // fields
     if (h->use_graphs) {
-        while (nsteps - done > kGraphSteps) {
+        const int gs = graph_steps(h);
+        while (nsteps - done > gs) {
             cudaGraphExec_t g;
             if ((st = step_graph(h, h->cur, &g))) return st;
             CU(cudaGraphLaunch(g, h->stream));
-            lbm::g_launches += kGraphSteps;
-            done += kGraphSteps;
+            lbm::g_launches += h->graph_launches;
+            done += gs;
         }
     }
-    for (; done < nsteps; ++done) {
-        CU(launch_one(h, h->cur, done == nsteps - 1));
-        h->cur = 1 - h->cur;
-    }
+    CU(launch_steps(h, h->cur, nsteps - done, true));
+    h->cur = (h->cur + nsteps - done) & 1;
     h->itc += nsteps;
     return LBM_OK;
 }
@@ -968,20 +1150,12 @@ static int period_graph(lbm_handle *h, int cur, int period, cudaGraphExec_t *out
         h->run_graph_period = period;
     }
     if (!h->run_graph[cur]) {
-        cudaGraph_t g = nullptr;
+        const int64_t l0 = lbm::g_launches;
         CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = cudaSuccess;
-        for (int i = 0; i < period && e == cudaSuccess; ++i) e = launch_one(h, (cur + i) & 1, i == period - 1);
+        cudaError_t e = launch_steps(h, cur, period, true);
         if (e == cudaSuccess) e = run_check(h->geo, h->bufs, period, h->stream);
-        const cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
-        lbm::g_launches -= period + 2;  // counted when replayed
-        if (e != cudaSuccess || e2 != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            return fail(LBM_ERR_CUDA, "check-period graph capture: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
-        }
-        e = cudaGraphInstantiate(&h->run_graph[cur], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) return fail(LBM_ERR_CUDA, "check-period graph instantiate: %s", cudaGetErrorString(e));
+        int st = end_capture(h, e, l0, &h->run_graph[cur], &h->run_graph_launches, "check-period");
+        if (st) return st;
     }
     *out = h->run_graph[cur];
     return LBM_OK;
@@ -994,6 +1168,7 @@ extern "C" int lbm_run(lbm_handle *h, int64_t max_steps, int32_t check_every, do
     if (max_steps < 0 || check_every < 1) return fail(LBM_ERR_PARAM, "need max_steps >= 0 and check_every >= 1");
     if (h->phase == 0) return fail(LBM_ERR_STATE, "lbm_run before an init call");
     int st = lbm::first_collision(h);
+    if (!st) st = ensure_plan(h);
     if (st) return st;
     if ((st = lbm::run_begin(h, eps, 0.0, 0))) return st;
     const int64_t itc0 = h->itc;
@@ -1014,7 +1189,7 @@ extern "C" int lbm_run(lbm_handle *h, int64_t max_steps, int32_t check_every, do
                 st = fail(LBM_ERR_CUDA, "cudaGraphLaunch: %s", cudaGetErrorString(e));
                 break;
             }
-            lbm::g_launches += k + 2;
+            lbm::g_launches += h->run_graph_launches;
             h->cur = (int)((h->cur + k) & 1);
             h->itc += k;
         } else {
@@ -1456,7 +1631,10 @@ extern "C" int lbm_get_option(const lbm_handle *h, int32_t option, int64_t *valu
     if (!h || !value) return fail(LBM_ERR_PARAM, "NULL argument");
     switch (option) {
     case LBM_OPT_KERNEL: *value = h->use_march ? 2 : 1; return LBM_OK;
-    case LBM_OPT_NBLOCKS: *value = h->use_march ? h->nblocks : 0; return LBM_OK;
+    case LBM_OPT_NBLOCKS:
+        if (h->use_march) plan_2d(const_cast<lbm_handle *>(h));
+        *value = h->use_march ? h->nblocks : 0;
+        return LBM_OK;
     case LBM_OPT_L2PROMO: *value = h->l2promo; return LBM_OK;
     case LBM_OPT_GRAPHS: *value = h->use_graphs; return LBM_OK;
     case LBM_OPT_RESIDENT: *value = h->resident > 0; return LBM_OK;

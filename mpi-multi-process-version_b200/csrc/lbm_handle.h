@@ -50,14 +50,22 @@ struct lbm_handle {
     int4 *d_msegs = nullptr;     // 3D march work plan: segments (tile, z0, z1, -)
     int *d_msegoff = nullptr;    // and each block's first segment
     size_t msegs_cap = 0, msegoff_cap = 0;
+    int nt = 128;                // 2D, fast build: columns per row of the march kernel
+    int levels = 1;              // and the time steps its multi-step launches advance
+    int slots = 0;               // blocks the march plan may use
+    std::vector<int4> segs2;     // the march's work plan
+    std::vector<int> segoff2;
+    bool plan_dirty = false;     // it is not on the device yet (the first launch plans and uploads it)
     int l2promo = 0;             // LBM_OPT_L2PROMO
     int use_graphs = 1;          // LBM_OPT_GRAPHS
     int resident_opt = 0;        // LBM_OPT_RESIDENT as set (opt-in)
     int resident = 0;            // resolved: blocks of the resident multi-step launch (0: off)
     unsigned *d_bar = nullptr;   // grid barrier of the resident launch (two counters)
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // 8-step graphs (kGraphSteps) from cur = 0 / 1
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // multi-step graphs of lbm_step from cur = 0 / 1
+    int64_t graph_launches = 0;  // kernels one replay launches
     cudaGraphExec_t run_graph[2] = {nullptr, nullptr};  // check periods of lbm_run from cur = 0 / 1
     int run_graph_period = 0;    // their length
+    int64_t run_graph_launches = 0;  // kernels one replay launches
     int cur = 0;                 // buffer holding the newest populations
     int phase = 0;               // 0: not initialised, 1: pre-collision, 2: post-collision
     int64_t itc = 0;

@@ -21,6 +21,7 @@ struct Geo {
     int64_t plane;   // elements between population planes
     int64_t nnode;   // nx*ny*nz: packed macro arrays, x fastest
     double Snu, Sq, sig_k, gbeta, dt, Thot, Tcold, T0, length_LB;
+    double relax[8];         // constants of the fast build's collision (relax_setup)
     double tc_lo, tc_grad;   // conduction profile: hot wall position and dTc per lattice unit (tc_setup)
     const double *wgt[3];    // per axis: weights [n][2 signs][3], sign 0 = +1, 1 = -1
     const double *coord[3];  // per axis: coordinates c(0:n+1)
@@ -37,6 +38,15 @@ inline void tc_setup(Geo &G, const double *c_heated)
     const int n = G.dim == 2 ? G.nx : G.ny;
     G.tc_lo = c_heated[1] - 0.5 * G.dt;
     G.tc_grad = (G.Tcold - G.Thot) / ((c_heated[n] + 0.5 * G.dt) - G.tc_lo);
+}
+
+// The constants of the fast build's collision in the order of its Relax: Snu,
+// Sq, sig_k, gbeta, dt, dt/2 and the forcing factors (1 - Sq/2) dt, (2 - Snu) dt.
+inline void relax_setup(Geo &G)
+{
+    const double r[8] = {G.Snu, G.Sq, G.sig_k, G.gbeta, G.dt, 0.5 * G.dt, (1.0 - 0.5 * G.Sq) * G.dt,
+                         (2.0 - G.Snu) * G.dt};
+    for (int k = 0; k < 8; ++k) G.relax[k] = r[k];
 }
 
 __host__ __device__ inline double tc_gradient(const Geo &G) { return G.tc_grad; }
@@ -92,7 +102,8 @@ struct BatchDev {
     const Geo *geo;          // [ncav]
     const TmapSet *maps;     // [ncav][2]: descriptors of pop[0], pop[1] (+ their force arrays)
     const Bufs *bufs;        // [ncav]
-    const int4 *segs;        // all segments: 2D (cavity, i0, ja, jb); 3D (tile, z0, z1, cavity)
+    const int4 *segs;        // all segments: 2D (cavity, i0, ja, jb), the fast build's from plan_march2d;
+                             // 3D (tile, z0, z1, cavity)
     const int *seg_off;      // [nblocks + 1]
 };
 
@@ -133,16 +144,20 @@ constexpr int kBatchTileY = 4;
                             void *pop_out, const Bufs &b, cudaStream_t s);                    \
     /* fused step through the TMA-fed persistent march kernel; 3D: tile rows ty (4 or 8)  */ \
     /* and the blocks' segment lists segs[segoff[b] .. segoff[b+1]) (device memory);       */ \
-    /* pdl: programmatic dependent launch (overlaps the previous kernel's tail)            */ \
+    /* pdl: programmatic dependent launch (overlaps the previous kernel's tail);           */ \
+    /* 2D, fast build: segments of plan_march2d, rows of nt columns (64 or 128), levels    */ \
+    /* time steps in the one launch (1, 2 or 4; write_macro needs 1)                       */ \
     cudaError_t march(const Geo &g, int store, const TmapSet &src, const void *F_in,          \
                       void *pop_out, void *F_out, const Bufs &b, int write_macro, int nblocks,\
-                      int ty, const int4 *segs, const int *segoff, bool pdl, cudaStream_t s); \
+                      int ty, const int4 *segs, const int *segoff, bool pdl, int nt,          \
+                      int levels, cudaStream_t s);                                            \
     /* resident blocks per SM of the march kernel (0 if it cannot launch) */                  \
-    int march_blocks_per_sm(const Geo &g, int store, int ty);                                 \
-    /* one step of every cavity of a 2D batch (tile width TX = 32, 64 or 128) */              \
+    int march_blocks_per_sm(const Geo &g, int store, int ty, int nt, int levels);             \
+    /* `levels` steps of every cavity of a 2D batch (tile width TX = 32, 64 or 128; the   */  \
+    /* exact build: one step) */                                                              \
     cudaError_t march_batch(int store, int TX, const BatchDev &D, int nblocks, int cur,       \
-                            int write_macro, int *err, bool pdl, cudaStream_t s);             \
-    int march_batch_blocks_per_sm(int store, int TX);                                         \
+                            int write_macro, int *err, bool pdl, int levels, cudaStream_t s); \
+    int march_batch_blocks_per_sm(int store, int TX, int levels);                             \
     /* one step of every cavity of a 3D batch (segments: tile, z0, z1, cavity; 32 x 4 tiles) */\
     cudaError_t march_batch3d(int store, const BatchDev &D, int nblocks, int cur,             \
                               int write_macro, int *err, bool pdl, cudaStream_t s);           \
@@ -185,6 +200,8 @@ int set_error(int code, const char *fmt, ...);
 // selects the tile width of the 2D kernels (0: the single-cavity default),
 // ty the tile rows of the 3D kernel (4 or 8; 0: 8)
 MarchShape march_shape(int dim, int store, int tx = 0, int ty = 0);
+// elements of a row box of the fast build's 2D march (tile width nt)
+int march2d_box(int store, int nt);
 
 // Work plan of the 3D march kernel: for `nblocks` persistent blocks over
 // `ntiles` tile columns of nz slices, the segments (tile, z0, z1, 0) of each
@@ -193,5 +210,20 @@ MarchShape march_shape(int dim, int store, int tx = 0, int ty = 0);
 // take the chunks' last slices in lockstep rounds); 1: contiguous equal
 // shares of the (tile-major, slice-minor) items.  Returns the blocks used.
 int plan_march3d(int ntiles, int nz, int nblocks, int kind, std::vector<int4> &segs, std::vector<int> &off);
+
+// A march of the fast build's 2D kernel: rows [lo, hi) of columns [x0, x0 + w)
+// of cavity cav (ny rows in all).
+struct Strip2 {
+    int cav, x0, w, lo, hi, ny;
+};
+// The strips of a cavity nx nodes wide for rows of nt columns and `levels` time
+// levels per launch: as few as fit, of nearly equal width.
+void strips_march2d(int cav, int nx, int lo, int hi, int ny, int nt, int levels, std::vector<Strip2> &out);
+// Work plan: the strips' rows cut into segments (cav | w << 24, x0, ja, jb) for
+// at most `nblocks` blocks so that the busiest block runs as few iterations as
+// possible (a segment costs its rows and 3 levels - 1 more).  off: each block's
+// first segment, nblocks + 1 entries; returns the blocks that have work.
+int plan_march2d(const std::vector<Strip2> &strips, int levels, int nblocks, std::vector<int4> &segs,
+                 std::vector<int> &off);
 
 }  // namespace lbm

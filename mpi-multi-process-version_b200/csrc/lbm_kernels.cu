@@ -216,6 +216,10 @@ __device__ __forceinline__ void collide2d(const C f[9], const C gg[5], C rho, C 
     gp[4] = -DV(np[2],2.0)+DV(np[3],4.0)-DV(np[4],4.0);
 }
 
+#if !LBM_EXACT
+#include "lbm_node2d.cuh"
+#endif
+
 // One node (i, j) of the fused 2D step.  KIND 0: fused step; KIND 1: stream
 // + walls + macro only.  COHERENT: read the source through L2 (ld.global.cg)
 // instead of the read-only path, for a kernel that wrote it itself earlier.
@@ -229,19 +233,21 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
     using C = typename Tr<ST>::C;
     const int64_t P = G.plane;
     const int64_t id = (int64_t)j * G.pitch + i;
+    auto LD = [&](int q, int64_t off) -> C {
+        return tocomp(COHERENT ? __ldcg(src + q * P + id + off) : __ldg(src + q * P + id + off));
+    };
+    C f[9], gg[5];
+    const C Fy0 = COHERENT ? __ldcg(Fin + id) : Fin[id];  // the force of the collision that produced src
+#if LBM_EXACT
     const int xa = off_a(i, G.nx), xb = off_b(i, G.nx);
     const int64_t ya = (int64_t)off_a(j, G.ny) * G.pitch, yb = (int64_t)off_b(j, G.ny) * G.pitch;
     C xp[3], xm[3], yp[3], ym[3];
     load_w(G.wgt[0], i, xp, xm);
     load_w(G.wgt[1], j, yp, ym);
 
-    auto LD = [&](int q, int64_t off) -> C {
-        return tocomp(COHERENT ? __ldcg(src + q * P + id + off) : __ldg(src + q * P + id + off));
-    };
     // y-interpolation of plane q on the column at x-offset c
     auto YI = [&](int q, const C w[3], int64_t c) -> C { return ip(w, LD(q, c + ya), LD(q, c), LD(q, c + yb)); };
 
-    C f[9], gg[5];
     f[0] = LD(0, 0);
     f[1] = ip(xp, LD(1, xa), LD(1, 0), LD(1, xb));
     f[2] = ip(yp, LD(2, ya), LD(2, 0), LD(2, yb));
@@ -256,25 +262,16 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
     gg[2] = ip(yp, LD(11, ya), LD(11, 0), LD(11, yb));
     gg[3] = ip(xm, LD(12, xa), LD(12, 0), LD(12, xb));
     gg[4] = ip(ym, LD(13, ya), LD(13, 0), LD(13, yb));
-    // deviation from the conduction profile: the departure point of g1 / g3
-    // lies dt behind / ahead along x
-    C Tc = C(0.0);
-    if (Tr<ST>::kDevT) {
-        Tc = C(tc_value(G, i));
-        const C sT = C(0.125 * G.dt * tc_gradient(G));
-        gg[1] -= sT;
-        gg[3] += sT;
-    }
 
     // walls: bounceback_u (2B:731-768), bounceback_T (2B:770-801)
     const C two_wT = C(2.0) * C(0.125);
     if (i == 0) {
         f[1] = LD(3, 0); f[5] = LD(7, 0); f[8] = LD(6, 0);
-        gg[1] = -LD(12, 0) + two_wT * (Tr<ST>::kDevT ? C(G.Thot) - Tc : C(G.Thot));
+        gg[1] = -LD(12, 0) + two_wT * C(G.Thot);
     }
     if (i == G.nx - 1) {
         f[3] = LD(1, 0); f[6] = LD(8, 0); f[7] = LD(5, 0);
-        gg[3] = -LD(10, 0) + two_wT * (Tr<ST>::kDevT ? C(G.Tcold) - Tc : C(G.Tcold));
+        gg[3] = -LD(10, 0) + two_wT * C(G.Tcold);
     }
     if (j == G.ny - 1) {
         f[4] = LD(2, 0); f[7] = LD(5, 0); f[8] = LD(6, 0);
@@ -285,20 +282,55 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
         gg[2] = LD(13, 0);
     }
 
-    // macro_u / macro_t (2M:726-753); the force is the one of the collision
-    // that produced src
-    const C Fy0 = COHERENT ? __ldcg(Fin + id) : Fin[id];
+    // macro_u / macro_t (2M:726-753)
     const C dt = C(G.dt);
-    const C rho = (Tr<ST>::kShift ? C(1.0) : C(0.0)) + (f[0]+f[1]+f[2]+f[3]+f[4]+f[5]+f[6]+f[7]+f[8]);
-#if LBM_EXACT
+    const C rho = f[0]+f[1]+f[2]+f[3]+f[4]+f[5]+f[6]+f[7]+f[8];
     const C u = ( f[1]-f[3]+f[5]-f[6]-f[7]+f[8]+C(0.5)*dt*C(0.0))/rho;
     const C v = ( f[2]-f[4]+f[5]+f[6]-f[7]-f[8]+C(0.5)*dt*Fy0)/rho;
+    const C T = gg[0]+gg[1]+gg[2]+gg[3]+gg[4];
 #else
-    const C rinv = C(1.0) / rho;
-    const C u = (f[1]-f[3]+f[5]-f[6]-f[7]+f[8])*rinv;
-    const C v = (f[2]-f[4]+f[5]+f[6]-f[7]-f[8]+C(0.5)*dt*Fy0)*rinv;
+    // the window form of lbm_node2d.cuh: x first on each row, then y
+    const int xo = win_lo(i, G.nx) - i;
+    const int64_t yo = (int64_t)(win_lo(j, G.ny) - j) * G.pitch;
+    C xp[3], xm[3], yp[3], ym[3];
+    window_weights<C>(G.wgt[0] + (int64_t)i * 6, i, G.nx, xp, xm);
+    window_weights<C>(G.wgt[1] + (int64_t)j * 6, j, G.ny, yp, ym);
+    auto XI = [&](int q, const C w[3], int64_t r) -> C {
+        return lin3(w, LD(q, r + xo), LD(q, r + xo + 1), LD(q, r + xo + 2));
+    };
+    auto YI = [&](int q, const C w[3]) -> C {
+        return lin3(w, LD(q, yo), LD(q, yo + G.pitch), LD(q, yo + 2 * G.pitch));
+    };
+    auto XY = [&](int q, const C wx[3], const C wy[3]) -> C {
+        return lin3(wy, XI(q, wx, yo), XI(q, wx, yo + G.pitch), XI(q, wx, yo + 2 * G.pitch));
+    };
+    f[0] = LD(0, 0);
+    f[1] = XI(1, xp, 0);
+    f[2] = YI(2, yp);
+    f[3] = XI(3, xm, 0);
+    f[4] = YI(4, ym);
+    f[5] = XY(5, xp, yp);
+    f[6] = XY(6, xm, yp);
+    f[7] = XY(7, xm, ym);
+    f[8] = XY(8, xp, ym);
+    gg[0] = LD(9, 0);
+    gg[1] = XI(10, xp, 0);
+    gg[2] = YI(11, yp);
+    gg[3] = XI(12, xm, 0);
+    gg[4] = YI(13, ym);
+    // deviation from the conduction profile: the departure point of g1 / g3
+    // lies dt behind / ahead along x
+    C Tc = C(0.0);
+    if (Tr<ST>::kDevT) {
+        Tc = C(tc_value(G, i));
+        const C sT = C(0.125 * G.dt * tc_gradient(G));
+        gg[1] = sub_(gg[1], sT);
+        gg[3] = add_(gg[3], sT);
+    }
+    walls2d<C, Tr<ST>::kDevT>(i, j, G.nx, G.ny, C(G.Thot), C(G.Tcold), Tc, [&](int q) -> C { return LD(q, 0); }, f, gg);
+    C fp[9], gp[5], Fy, rho, u, v, T;
+    node2d<C, Tr<ST>::kShift, Tr<ST>::kDevT>(f, gg, Fy0, relax_of<C>(G), Tc, fp, gp, Fy, rho, u, v, T);
 #endif
-    const C T = Tr<ST>::kDevT ? Tc + (gg[0]+gg[1]+gg[2]+gg[3]+gg[4]) : gg[0]+gg[1]+gg[2]+gg[3]+gg[4];
 
     if (write_macro || KIND == 1) {
         const int64_t mid = (int64_t)j * G.nx + i;
@@ -316,8 +348,10 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
         return;
     }
 
+#if LBM_EXACT
     C fp[9], gp[5], Fy;
     collide2d<C, Tr<ST>::kShift, Tr<ST>::kDevT>(f, gg, rho, u, v, T, G, fp, gp, Fy);
+#endif
     Fout[id] = Fy;
 #pragma unroll
     for (int q = 0; q < 9; ++q) ST_(q, fp[q]);
@@ -1059,6 +1093,9 @@ __global__ void k_collide(const Geo G, const typename Tr<ST>::S *__restrict__ in
 }
 
 #include "lbm_march.cuh"
+#if !LBM_EXACT
+#include "lbm_march2d.cuh"
+#endif
 
 // ---------------------------------------------------------------------------
 // launchers
@@ -1230,6 +1267,7 @@ static cudaError_t prepare_march3d()
     return cudaSuccess;
 }
 
+#if LBM_EXACT
 template <int ST, class L>
 static cudaError_t prepare_march2d()
 {
@@ -1242,6 +1280,32 @@ static cudaError_t prepare_march2d()
     }
     return cudaSuccess;
 }
+#else
+template <int ST, int COLS, int T>
+static cudaError_t prepare_march2d()
+{
+    static bool done = false;
+    if (!done) {
+        cudaError_t e = cudaFuncSetAttribute(k_march2d<ST, COLS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             M2<ST, COLS, T>::SMEM);
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    return cudaSuccess;
+}
+
+// CALLT(columns, levels) of the variant asked for
+#define LBM_MARCH2D_CASES(cols, levels, CALLT)   \
+    switch ((cols) * 8 + (levels)) {             \
+    case 64 * 8 + 1: return CALLT(64, 1);        \
+    case 64 * 8 + 2: return CALLT(64, 2);        \
+    case 64 * 8 + 4: return CALLT(64, 4);        \
+    case 128 * 8 + 1: return CALLT(128, 1);      \
+    case 128 * 8 + 2: return CALLT(128, 2);      \
+    case 128 * 8 + 4: return CALLT(128, 4);      \
+    default: break;                              \
+    }
+#endif
 
 template <int ST, int TY>
 static int mbps3(void)
@@ -1254,6 +1318,7 @@ static int mbps3(void)
                : 0;
 }
 
+#if LBM_EXACT
 template <int ST, class L>
 static int mbps2(void)
 {
@@ -1264,15 +1329,43 @@ static int mbps2(void)
 }
 
 template <int ST>
-static int mbps(const Geo &g, int ty)
+static int mbps2d(const Geo &g, int, int)
 {
-    if (g.dim == 3) return ty == 4 ? mbps3<ST, 4>() : mbps3<ST, 8>();
     return g.nnode >= kDeepRingNodes ? mbps2<ST, L2d<ST>>() : mbps2<ST, L2s<ST>>();
 }
-
-int march_blocks_per_sm(const Geo &g, int store, int ty)
+#else
+template <int ST, int COLS, int T>
+static int mbps2(void)
 {
-#define CALL(ST) mbps<ST>(g, ty)
+    if (prepare_march2d<ST, COLS, T>() != cudaSuccess) return 0;
+    using M = M2<ST, COLS, T>;
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d<ST, COLS, T>, M::COLS * T, M::SMEM) ==
+                   cudaSuccess
+               ? n
+               : 0;
+}
+
+template <int ST>
+static int mbps2d(const Geo &, int nt, int levels)
+{
+#define CALLT(COLS, T) (mbps2<ST, COLS, T>())
+    LBM_MARCH2D_CASES(nt, levels, CALLT)
+#undef CALLT
+    return 0;
+}
+#endif
+
+template <int ST>
+static int mbps(const Geo &g, int ty, int nt, int levels)
+{
+    if (g.dim == 3) return ty == 4 ? mbps3<ST, 4>() : mbps3<ST, 8>();
+    return mbps2d<ST>(g, nt, levels);
+}
+
+int march_blocks_per_sm(const Geo &g, int store, int ty, int nt, int levels)
+{
+#define CALL(ST) mbps<ST>(g, ty, nt, levels)
     LBM_DISPATCH(store, CALL)
 #undef CALL
 }
@@ -1290,6 +1383,7 @@ static cudaError_t launch_march3d(const Geo &g, const TmapSet &m, const void *Fi
                     (S *)pout, (C *)Fout, b, wm, segs, segoff, b.err);
 }
 
+#if LBM_EXACT
 template <int ST, class L>
 static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
                                   const Bufs &b, int wm, int nblocks, bool pdl, cudaStream_t s)
@@ -1305,100 +1399,140 @@ static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, const void *Fi
 }
 
 template <int ST>
-static cudaError_t launch_march(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
-                                const Bufs &b, int wm, int nblocks, int ty, const int4 *segs, const int *segoff,
-                                bool pdl, cudaStream_t s)
+static cudaError_t launch_2d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout, const Bufs &b,
+                             int wm, int nblocks, const int4 *, const int *, bool pdl, int, int, cudaStream_t s)
+{
+    return g.nnode >= kDeepRingNodes ? launch_march2d<ST, L2d<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s)
+                                     : launch_march2d<ST, L2s<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s);
+}
+#else
+template <int ST, int COLS, int T>
+static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, void *pout, void *Fout, const Bufs &b, int wm,
+                                  int nblocks, const int4 *segs, const int *segoff, bool pdl, cudaStream_t s)
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
+    using M = M2<ST, COLS, T>;
+    cudaError_t e = prepare_march2d<ST, COLS, T>();
+    if (e != cudaSuccess) return e;
+    return launch_k(k_march2d<ST, COLS, T>, nblocks, M::COLS * T, M::SMEM, s, pdl, m.m[0], m.fmap, g, (S *)pout,
+                    (C *)Fout, b, wm, segs, segoff, b.err);
+}
+
+template <int ST>
+static cudaError_t launch_2d(const Geo &g, const TmapSet &m, const void *, void *pout, void *Fout, const Bufs &b,
+                             int wm, int nblocks, const int4 *segs, const int *segoff, bool pdl, int nt, int levels,
+                             cudaStream_t s)
+{
+#define CALLT(COLS, T) (launch_march2d<ST, COLS, T>(g, m, pout, Fout, b, wm, nblocks, segs, segoff, pdl, s))
+    LBM_MARCH2D_CASES(nt, levels, CALLT)
+#undef CALLT
+    return cudaErrorInvalidValue;
+}
+#endif
+
+template <int ST>
+static cudaError_t launch_march(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
+                                const Bufs &b, int wm, int nblocks, int ty, const int4 *segs, const int *segoff,
+                                bool pdl, int nt, int levels, cudaStream_t s)
+{
     cudaError_t e;
-    if (g.dim == 3) {
+    if (g.dim == 3)
         e = ty == 4 ? launch_march3d<ST, 4>(g, m, Fin, pout, Fout, b, wm, segs, segoff, nblocks, pdl, s)
                     : launch_march3d<ST, 8>(g, m, Fin, pout, Fout, b, wm, segs, segoff, nblocks, pdl, s);
-    } else {
-        e = g.nnode >= kDeepRingNodes ? launch_march2d<ST, L2d<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s)
-                                      : launch_march2d<ST, L2s<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s);
-    }
+    else
+        e = launch_2d<ST>(g, m, Fin, pout, Fout, b, wm, nblocks, segs, segoff, pdl, nt, levels, s);
     ++g_launches;
     return e;
 }
 
 cudaError_t march(const Geo &g, int store, const TmapSet &src, const void *F_in, void *pop_out, void *F_out,
                   const Bufs &b, int write_macro, int nblocks, int ty, const int4 *segs, const int *segoff,
-                  bool pdl, cudaStream_t s)
+                  bool pdl, int nt, int levels, cudaStream_t s)
 {
-#define CALL(ST) launch_march<ST>(g, src, F_in, pop_out, F_out, b, write_macro, nblocks, ty, segs, segoff, pdl, s)
+#define CALL(ST) \
+    launch_march<ST>(g, src, F_in, pop_out, F_out, b, write_macro, nblocks, ty, segs, segoff, pdl, nt, levels, s)
     LBM_DISPATCH(store, CALL)
 #undef CALL
 }
 
-template <int ST, int TX>
-static cudaError_t prepare_batch()
-{
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march2d_batch<ST, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             L2<ST, TX>::smem());
+// the 2D batch kernel of COLS columns advancing T time levels (the exact build: one level)
+template <int ST, int COLS, int T>
+struct BatchK {
+#if LBM_EXACT
+    static constexpr int threads = COLS, smem = L2<ST, COLS>::smem();
+    static auto kernel() { return k_march2d_batch<ST, COLS>; }
+#else
+    static constexpr int threads = COLS * T, smem = M2<ST, COLS, T>::SMEM;
+    static auto kernel() { return k_march2d_batch<ST, COLS, T>; }
+#endif
+    static cudaError_t prepare()
+    {
+        static bool done = false;
+        if (!done) {
+            cudaError_t e = cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e != cudaSuccess) return e;
+            done = true;
+        }
+        return cudaSuccess;
+    }
+    static cudaError_t launch(const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl, cudaStream_t s)
+    {
+        cudaError_t e = prepare();
         if (e != cudaSuccess) return e;
-        done = true;
+        ++g_launches;
+        return launch_k(kernel(), nblocks, threads, smem, s, pdl, D, cur, wm, err);
     }
-    return cudaSuccess;
-}
+    static int blocks()
+    {
+        if (prepare() != cudaSuccess) return 0;
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel(), threads, smem) == cudaSuccess ? n : 0;
+    }
+};
 
-template <int ST, int TX>
-static cudaError_t launch_batch(const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl, cudaStream_t s)
-{
-    cudaError_t e = prepare_batch<ST, TX>();
-    if (e != cudaSuccess) return e;
-    ++g_launches;
-    return launch_k(k_march2d_batch<ST, TX>, nblocks, TX, L2<ST, TX>::smem(), s, pdl, D, cur, wm, err);
-}
+#if LBM_EXACT
+#define LBM_BATCH_CASES(cols, levels, CALLB) \
+    switch (cols) {                              \
+    case 32: return CALLB(32, 1);             \
+    case 64: return CALLB(64, 1);             \
+    case 128: return CALLB(128, 1);           \
+    default: break;                              \
+    }
+#else
+#define LBM_BATCH_CASES(cols, levels, CALLB) LBM_MARCH2D_CASES(cols, levels, CALLB)
+#endif
 
-template <int ST, int TX>
-static int batch_bps()
+template <int ST>
+static cudaError_t launch_batch_tx(int cols, int levels, const BatchDev &D, int nblocks, int cur, int wm,
+                                   int *err, bool pdl, cudaStream_t s)
 {
-    if (prepare_batch<ST, TX>() != cudaSuccess) return 0;
-    int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d_batch<ST, TX>, TX, L2<ST, TX>::smem()) ==
-                   cudaSuccess
-               ? n
-               : 0;
+#define CALLB(X, T) (BatchK<ST, X, T>::launch(D, nblocks, cur, wm, err, pdl, s))
+    LBM_BATCH_CASES(cols, levels, CALLB)
+#undef CALLB
+    return cudaErrorInvalidValue;
 }
 
 template <int ST>
-static cudaError_t launch_batch_tx(int TX, const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl,
-                                   cudaStream_t s)
+static int batch_bps_tx(int cols, int levels)
 {
-    switch (TX) {
-    case 32: return launch_batch<ST, 32>(D, nblocks, cur, wm, err, pdl, s);
-    case 64: return launch_batch<ST, 64>(D, nblocks, cur, wm, err, pdl, s);
-    case 128: return launch_batch<ST, 128>(D, nblocks, cur, wm, err, pdl, s);
-    default: return cudaErrorInvalidValue;
-    }
+#define CALLB(X, T) (BatchK<ST, X, T>::blocks())
+    LBM_BATCH_CASES(cols, levels, CALLB)
+#undef CALLB
+    return 0;
 }
 
-template <int ST>
-static int batch_bps_tx(int TX)
+cudaError_t march_batch(int store, int cols, const BatchDev &D, int nblocks, int cur, int write_macro, int *err,
+                        bool pdl, int levels, cudaStream_t s)
 {
-    switch (TX) {
-    case 32: return batch_bps<ST, 32>();
-    case 64: return batch_bps<ST, 64>();
-    case 128: return batch_bps<ST, 128>();
-    default: return 0;
-    }
-}
-
-cudaError_t march_batch(int store, int TX, const BatchDev &D, int nblocks, int cur, int write_macro, int *err,
-                        bool pdl, cudaStream_t s)
-{
-#define CALL(ST) launch_batch_tx<ST>(TX, D, nblocks, cur, write_macro, err, pdl, s)
+#define CALL(ST) launch_batch_tx<ST>(cols, levels, D, nblocks, cur, write_macro, err, pdl, s)
     LBM_DISPATCH(store, CALL)
 #undef CALL
 }
 
-int march_batch_blocks_per_sm(int store, int TX)
+int march_batch_blocks_per_sm(int store, int cols, int levels)
 {
-#define CALL(ST) batch_bps_tx<ST>(TX)
+#define CALL(ST) batch_bps_tx<ST>(cols, levels)
     LBM_DISPATCH(store, CALL)
 #undef CALL
 }
@@ -1462,6 +1596,8 @@ cudaError_t set_wait_limit(long long cycles)
 }  // namespace LBM_NS
 
 #if !LBM_EXACT
+int march2d_box(int store, int nt) { return nt + 2 * (store == kF64 ? 2 : 4); }
+
 // tile shapes of the march kernels, for the host's tensor-map encoding
 MarchShape march_shape(int dim, int store, int tx, int ty)
 {

@@ -95,6 +95,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, long lon
     return true;
 }
 
+// the same with the limit of a step's waits, read only where the first test fails
+__device__ __forceinline__ bool mbar_wait_lim(uint64_t *b, uint32_t parity)
+{
+    if (mbar_probe(b, parity)) return true;
+    return mbar_wait(b, parity, *(volatile long long *)&g_wait_limit);
+}
+
 __device__ __forceinline__ void tma_load4(void *dst, const CUtensorMap *m, uint64_t *bar, int c0, int c1, int c2,
                                           int c3)
 {
@@ -168,7 +175,7 @@ __device__ __forceinline__ int need_hi(int k, int n) { return k == 0 ? 2 : (k ==
 // miss the small L1 left beside the rings (each one an L2 round trip on the
 // critical path of the step).  Single-cavity kernels take Geo as a kernel
 // parameter and read it from the constant bank instead.
-constexpr int kGeoStage = 256;
+constexpr int kGeoStage = 320;
 static_assert(sizeof(Geo) <= kGeoStage && sizeof(Geo) % 8 == 0, "staged Geo must fit its shared-memory slot");
 
 // every thread of the CTA: copy *src into the shared slot dst (8-byte words),
@@ -629,6 +636,10 @@ using L2d = L2<ST, 128, 6, 4>;
 // nodes from which the single-cavity 2D kernel uses the deep ring
 constexpr int64_t kDeepRingNodes = int64_t(1) << 20;
 
+#if LBM_EXACT
+// The exact build's 2D march: one time level per pass, every node interpolated in
+// the reference's operand order from a ring of rows in shared memory.
+
 // One node of the 2D march at row j, from the ring slots in shared memory:
 // interpolation, walls, macro, collision, stores.
 template <int ST, class L>
@@ -739,7 +750,6 @@ __device__ __forceinline__ void march2d_run(int nseg, SegFn seg, CavFn cavity, i
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
-    constexpr int TX = L::TX;
     constexpr int HX = L::HX;
     extern __shared__ unsigned char sm_raw[];
     unsigned char *sm = sm_raw + ((128u - (saddr(sm_raw) & 127u)) & 127u);
@@ -935,3 +945,4 @@ k_march2d_batch(const BatchDev D, int cur, int write_macro, int *err)
     };
     march2d_run<ST, L2<ST, TX>, true>(s1 - s0, seg, cavity, write_macro, err);
 }
+#endif  // LBM_EXACT
