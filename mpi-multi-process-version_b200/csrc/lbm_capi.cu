@@ -538,6 +538,65 @@ int lbm::plan_march2d(const std::vector<Strip2> &strips, int levels, int nblocks
     return (int)used;
 }
 
+// The tile kernel's plan: of the tilings and step counts that fit shared memory
+// the one with the least time per step, from a fit to measured launches (48x40 to
+// 256^2, within 15 %): 3.3 us for launch, load and store; a level 0.4 us plus
+// 0.15 us (FP32 0.10) per warp of its region; one block per SM at a time.  A longer
+// launch spreads its fixed cost over more steps but widens the halo every tile
+// computes: 128^2 takes 2.82, 2.11, 2.19, 2.45 us a step at 2, 4, 6, 8 steps.
+// T = 0 where the march kernel's launch of four levels is the faster (with a tenth
+// in hand for the fit): measured, march against tiles, FP64 4.63 / 3.0 us a step at
+// 192^2, 5.02 / 4.4 at 256^2, 5.6 / 6.5 at 300^2; FP32 4.11 / 3.35 at 256^2,
+// 5.49 / 5.25 at 384^2, 7.77 / 7.98 at 512^2.
+lbm::TilePlan lbm::plan_tile2d(int nx, int ny, int esize, int sms)
+{
+    TilePlan best{};
+    double bc = 1e30;
+    const double per_warp = esize == 8 ? 0.15 : 0.10;
+    for (int ntx = 1; ntx <= (nx + 7) / 8; ++ntx) {
+        int cx = 0;
+        bool okx = true;
+        for (int a = 0; a < ntx; ++a) {
+            const int w = tile_cut(a + 1, ntx, nx, 8) - tile_cut(a, ntx, nx, 8);
+            okx = okx && w >= 2;
+            cx = std::max(cx, w);
+        }
+        if (!okx || cx > 64) continue;
+        for (int nty = 1; nty <= (ny + 3) / 4; ++nty) {
+            if ((int64_t)ntx * nty > 2 * sms) break;
+            int cy = 0;
+            bool oky = true;
+            for (int a = 0; a < nty; ++a) {
+                const int w = tile_cut(a + 1, nty, ny, 1) - tile_cut(a, nty, ny, 1);
+                oky = oky && w >= 2;
+                cy = std::max(cy, w);
+            }
+            if (!oky || cy > 64) continue;
+            for (int T = 1; T <= 8; ++T) {
+                const int ew = std::min(cx + 2 * T, nx), eh = std::min(cy + 2 * T, ny), en = ew * eh;
+                const int smem = (2 * en * 15 + (ew + eh) * kTileWeights) * esize;
+                if (smem > kTileSmem) continue;
+                const int waves = (ntx * nty + sms - 1) / sms;
+                double c = 3.3;
+                int most = 0;
+                for (int l = 1; l <= T; ++l) {
+                    const int n = std::min(cx + 2 * (T - l), nx) * std::min(cy + 2 * (T - l), ny);
+                    most = std::max(most, n);
+                    c += 0.4 + per_warp * ((n + 31) / 32);
+                }
+                c = c * waves / T;
+                if (c < bc) {
+                    bc = c;
+                    best = {ntx, nty, T, en, std::max(64, std::min(512, (most + 31) / 32 * 32)), std::max(smem, kTileAlone)};
+                }
+            }
+        }
+    }
+    const double n = (double)nx * ny;
+    if (bc > 0.9 * (esize == 8 ? 3.9 + 2.06e-5 * n : 3.0 + 1.75e-5 * n)) best.T = 0;
+    return best;
+}
+
 static int upload_segs(lbm_handle *h, const std::vector<int4> &segs, const std::vector<int> &off)
 {
     CU(cudaStreamSynchronize(h->stream));  // no launch in flight reads the old plan
@@ -605,6 +664,7 @@ static int resolve_2d(lbm_handle *h)
     h->nt = nt;
     h->levels = levels;
     h->slots = h->nblocks_opt > 0 ? h->nblocks_opt : bps * sms;
+    h->sms = sms;
     h->segs2.clear();
     h->plan_dirty = true;  // planned by the init call or the first launch: a batch's members never need it
     h->march_ok = lbm::encode_maps_tx(h, 0, h->tmaps);
@@ -619,12 +679,15 @@ static void plan_2d(lbm_handle *h)
     std::vector<lbm::Strip2> strips;
     lbm::strips_march2d(0, g.nx, g.jlo, g.jhi, g.ny, h->nt, h->levels, strips);
     h->nblocks = lbm::plan_march2d(strips, h->levels, h->slots, h->segs2, h->segoff2);
+    if (g.jlo == 0 && g.jhi == g.ny && g.nnode <= (1 << 18))
+        h->tile = lbm::plan_tile2d(g.nx, g.ny, (int)h->esize, h->sms);
 }
 
 static int ensure_plan(lbm_handle *h)
 {
     if (!h->plan_dirty) return LBM_OK;
     plan_2d(h);
+    if (h->tile.T > 1 && !h->use_march) return LBM_OK;  // tiles and direct-load single steps only
     int st = upload_segs(h, h->segs2, h->segoff2);
     if (!st) h->plan_dirty = false;
     return st;
@@ -660,6 +723,7 @@ static int resolve_path(lbm_handle *h)
         return fail(LBM_ERR_UNSUPPORTED, "march kernel not available for this shape / device");
     h->use_march = h->kernel_opt == 2 || (h->kernel_opt == 0 && ok && h->geo.nnode >= (1 << 15));
     h->levels = 1;
+    h->tile.T = 0;
     h->plan_dirty = false;
     const bool fast2d = h->p.dim == 2 && h->p.mode != LBM_MODE_EXACT;
     if (fast2d && ok && h->kernel_opt != 1) {
@@ -986,7 +1050,18 @@ static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
 {
     int left = with_macro ? n - 1 : n;
     cudaError_t e = cudaSuccess;
-    if (h->levels > 1 && !h->resident) {
+    if (h->tile.T > 1 && !h->resident && left > 0) {
+        int k = (left + h->tile.T - 1) / h->tile.T;
+        k += (k ^ left) & 1;
+        for (; k > 0 && e == cudaSuccess; --k) {
+            const int T = (left + k - 1) / k;
+            Bufs &b = h->bufs;
+            e = fast::tile2d(h->geo, h->p.storage, b.pop[cur], b.F[cur], b.pop[1 - cur], b.F[1 - cur], b, h->tile, T,
+                             h->pdl != 0, h->stream);
+            left -= T;
+            cur = 1 - cur;
+        }
+    } else if (h->levels > 1 && !h->resident) {
         // an even number of levels: launches in pairs
         for (; left >= 2 * h->levels && e == cudaSuccess; left -= 2 * h->levels)
             for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
@@ -1019,7 +1094,7 @@ void lbm::drop_graphs(lbm_handle *h)
 // steps per replayed graph in lbm_step (even: a replay leaves `cur` as it was):
 // eight launches; inside a graph consecutive march steps are programmatic
 // dependents
-static int graph_steps(const lbm_handle *h) { return 8 * h->levels; }
+static int graph_steps(const lbm_handle *h) { return 8 * (h->tile.T > 1 ? h->tile.T : h->levels); }
 
 // end the capture begun on h's stream: *out holds the instantiated graph and
 // *launches the kernels one replay launches.  e: the captured launches' status,

@@ -52,7 +52,8 @@ struct lbm_handle {
     size_t msegs_cap = 0, msegoff_cap = 0;
     int nt = 128;                // 2D, fast build: columns per row of the march kernel
     int levels = 1;              // and the time steps its multi-step launches advance
-    int slots = 0;               // blocks the march plan may use
+    lbm::TilePlan tile{};        // T > 1: small domains step T at a time through the tile kernel instead
+    int slots = 0, sms = 0;      // blocks the march plan may use, SMs of the device
     std::vector<int4> segs2;     // the march's work plan
     std::vector<int> segoff2;
     bool plan_dirty = false;     // it is not on the device yet (the first launch plans and uploads it)

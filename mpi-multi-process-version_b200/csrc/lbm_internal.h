@@ -169,6 +169,36 @@ constexpr int kBatchTileY = 4;
 LBM_DECLARE_LAUNCHERS(fast)
 LBM_DECLARE_LAUNCHERS(exact)
 
+// Small 2D domains of the fast build (lbm_tile2d.cuh): ntx x nty tiles, each
+// advanced up to T steps per launch in shared memory.  plan_tile2d chooses them;
+// T = 0: the domain is better off with the march kernel.
+struct TilePlan {
+    int ntx, nty;       // tiles: columns [tile_cut(a), tile_cut(a + 1)), rows likewise
+    int T;              // steps of a launch (at most)
+    int en;             // nodes a patch has room for
+    int threads, smem;  // of a block
+};
+constexpr int kTileSmem = 227 * 1024;  // a block's shared memory limit
+// a block takes at least this much, so that no two share an SM: the next launch's blocks, scheduled early
+// (programmatic dependent launch), would otherwise gather on some SMs and leave others idle
+constexpr int kTileAlone = 116 * 1024;
+constexpr int kTileWeights = 7;        // elements per column and per row of its weight table (6, and odd: no bank conflicts)
+// the first column (row) of tile a of nt on an axis of n nodes: cuts on
+// multiples of m, the last tile at least two wide
+__host__ __device__ inline int tile_cut(int a, int nt, int n, int m)
+{
+    if (a <= 0) return 0;
+    if (a >= nt) return n;
+    const int c = int(((int64_t)a * n / nt + m / 2) / m * m);
+    return c < n - 2 ? c : n - 2;
+}
+TilePlan plan_tile2d(int nx, int ny, int esize, int sms);
+namespace fast {
+// T <= plan.T steps of the domain in one launch
+cudaError_t tile2d(const Geo &g, int store, const void *pop_in, const void *F_in, void *pop_out, void *F_out,
+                   const Bufs &b, const TilePlan &pl, int T, bool pdl, cudaStream_t s);
+}
+
 // mode-independent kernels (lbm_reduce.cu)
 cudaError_t reduce_check(const Geo &g, const Bufs &b, cudaStream_t s);      // scal[0..3]
 cudaError_t reduce_nusselt(const Geo &g, const Bufs &b, cudaStream_t s);    // scal[4..6]

@@ -1095,6 +1095,7 @@ __global__ void k_collide(const Geo G, const typename Tr<ST>::S *__restrict__ in
 #include "lbm_march.cuh"
 #if !LBM_EXACT
 #include "lbm_march2d.cuh"
+#include "lbm_tile2d.cuh"
 #endif
 
 // ---------------------------------------------------------------------------
@@ -1455,6 +1456,35 @@ cudaError_t march(const Geo &g, int store, const TmapSet &src, const void *F_in,
     LBM_DISPATCH(store, CALL)
 #undef CALL
 }
+
+#if !LBM_EXACT
+template <int ST>
+static cudaError_t launch_tile2d(const Geo &g, const void *pin, const void *Fin, void *pout, void *Fout,
+                                 const Bufs &b, const TilePlan &pl, int T, bool pdl, cudaStream_t s)
+{
+    using S = typename Tr<ST>::S;
+    using C = typename Tr<ST>::C;
+    static bool done = false;
+    if (!done) {
+        cudaError_t e = cudaFuncSetAttribute(k_tile2d<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    TilePlan q = pl;
+    q.T = T;
+    ++g_launches;
+    return launch_k(k_tile2d<ST>, pl.ntx * pl.nty, pl.threads, pl.smem, s, pdl, g, (const S *)pin, (const C *)Fin,
+                    (S *)pout, (C *)Fout, (const RunCtl *)b.ctl, q);
+}
+
+cudaError_t tile2d(const Geo &g, int store, const void *pop_in, const void *F_in, void *pop_out, void *F_out,
+                   const Bufs &b, const TilePlan &pl, int T, bool pdl, cudaStream_t s)
+{
+#define CALL(ST) launch_tile2d<ST>(g, pop_in, F_in, pop_out, F_out, b, pl, T, pdl, s)
+    LBM_DISPATCH(store, CALL)
+#undef CALL
+}
+#endif
 
 // the 2D batch kernel of COLS columns advancing T time levels (the exact build: one level)
 template <int ST, int COLS, int T>
