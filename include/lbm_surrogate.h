@@ -60,6 +60,12 @@ int lbm_nn_colsum(const void *a, int64_t P, int32_t C, float *ws, float *out, vo
 int lbm_nn_silu_backward(const float *da, int64_t das, int32_t dao, const float *z,
                          int64_t P, int32_t C, void *dz, void *stream);
 
+/* lbm_nn_silu_backward and the bias gradient db[c] = sum over rows of dz[p][c]
+ * in one pass (the values lbm_nn_colsum(dz) gives up to the order of the sum);
+ * ws: FP32 scratch of lbm_nn_colsum_workspace(P, C). */
+int lbm_nn_silu_backward_bias(const float *da, int64_t das, int32_t dao, const float *z, int64_t P, int32_t C,
+                              void *dz, float *ws, float *db, void *stream);
+
 /* 2x2 average pooling of x (B, H, W even) into y (B, H/2, W/2); bf16. */
 int lbm_nn_pool2(const void *x, int64_t xs, int32_t xo, int32_t B, int32_t H, int32_t W, int32_t C,
                  void *y, int64_t ys, int32_t yo, void *stream);

@@ -44,6 +44,7 @@ _SIGS = {
     "lbm_nn_colsum_workspace": [_i64, _i32],
     "lbm_nn_colsum": [_dp, _i64, _i32, _dp, _dp, _dp],
     "lbm_nn_silu_backward": [_dp, _i64, _i32, _dp, _i64, _i32, _dp, _dp],
+    "lbm_nn_silu_backward_bias": [_dp, _i64, _i32, _dp, _i64, _i32, _dp, _dp, _dp, _dp],
     "lbm_nn_pool2": [_dp, _i64, _i32, _i32, _i32, _i32, _i32, _dp, _i64, _i32, _dp],
     "lbm_nn_pool2_backward": [_dp, _i64, _i32, _i32, _i32, _i32, _i32, _dp, _i64, _i32, _dp],
     "lbm_nn_up2": [_dp, _i64, _i32, _i32, _i32, _i32, _i32, _dp, _i64, _i32, _dp],
@@ -340,11 +341,10 @@ class Net:
             H = b["res"][name]
             P = B * H * H
             dz = b["dz_" + name]
-            _chk(lib.lbm_nn_silu_backward(da_ptr, das, dao, b["z_" + name].data_ptr(), P, co, dz.data_ptr(), s),
-                 "silu backward")
+            _chk(lib.lbm_nn_silu_backward_bias(da_ptr, das, dao, b["z_" + name].data_ptr(), P, co, dz.data_ptr(), ws,
+                                               self._gb(name), s), f"silu backward {name}")
             _chk(lib.lbm_nn_conv3x3_wgrad(dz.data_ptr(), x_ptr, xs, xo, B, H, H, ci, co, ws, wsn, self._gw(name), s),
                  f"wgrad {name}")
-            _chk(lib.lbm_nn_colsum(dz.data_ptr(), P, co, ws, self._gb(name), s), f"bias grad {name}")
             if dx_ptr is not None:
                 self._conv(B, name, dz.data_ptr(), co, 0, dx_ptr, dxs, dxo, dx_acc, None, 0, 0, 0, False, True, H, co, ci)
 
@@ -369,7 +369,7 @@ class Net:
         _chk(lib.lbm_nn_pool2_backward(p("dp1"), c1, 0, B, R, R, c1, p("dcat1"), c2 + c1, c2, s), "pool bwd")
         back("e1b", p("dcat1"), c2 + c1, c2, p("a_e1a"), c1, 0, p("da_e1a"), c1, 0)
         back("e1a", p("da_e1a"), c1, 0, p("x"), IN_CH, 0)
-        self.launches += 14 + 3 + 13 * 6 + 5 + 3 + 3
+        self.launches += 14 + 3 + 13 * 5 + 4 + 3 + 3
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8, wd=0.0):
         self.t += 1

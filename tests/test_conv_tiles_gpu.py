@@ -1,0 +1,70 @@
+"""The network's tiled kernels at the sizes where a tile ends: images smaller
+than a pixel tile, one row or column past it, channel counts with a remainder,
+strides and addresses that allow no wide stores.
+
+Reference: the float64 oracle on the same bfloat16 operands.  A sum of n products
+accumulated in FP32 in any order, truncating or rounding, is off by at most
+n 2^-23 sum |x_i| |w_i|; that is the tolerance, element by element."""
+import numpy as np
+import pytest
+
+import unet_oracle as U
+
+pytestmark = pytest.mark.gpu
+
+
+def up(torch, a, dtype=None):
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda().to(dtype or torch.float32)
+
+
+def down(t):
+    return t.float().cpu().numpy().astype(np.float64)
+
+
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [(1, 1, 1, 32, 8), (2, 8, 16, 32, 32), (2, 9, 17, 64, 40), (1, 7, 33, 96, 72),
+                                            (5, 24, 31, 32, 64), (40, 3, 2, 64, 32)])
+def test_weight_gradient_tile_edges(pkg, B, H, W, Cin, Cout):
+    import torch
+    lib = pkg.surrogate.nn()
+    rng = np.random.default_rng(B * H * W + Cin + Cout)
+    x = U.bf16_round(rng.normal(size=(B, H, W, Cin + 8)))
+    dz = U.bf16_round(rng.normal(size=(B, H, W, Cout)))
+    xd, dzd = up(torch, x, torch.bfloat16), up(torch, dz, torch.bfloat16)
+    n = lib.lbm_nn_wgrad_workspace(B, H, W, Cin, Cout)
+    ws = torch.full((n,), float("nan"), device="cuda")
+    dw = torch.zeros(Cout * 9 * Cin, device="cuda")
+    assert lib.lbm_nn_conv3x3_wgrad(dzd.data_ptr(), xd.data_ptr(), Cin + 8, 8, B, H, W, Cin, Cout, ws.data_ptr(), n,
+                                    dw.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    ref = U.conv3x3_wgrad(dz, x[..., 8:])
+    size = U.conv3x3_wgrad(np.abs(dz), np.abs(x[..., 8:]))
+    assert (np.abs(down(dw).reshape(ref.shape) - ref) <= B * H * W * 2.0 ** -23 * size).all()
+
+
+# channels: one 16-byte group, more groups than a block has threads, no multiple of 8; an offset that allows no
+# wide loads
+@pytest.mark.parametrize("P,C,off", [(1, 8, 0), (1000, 32, 0), (4737, 96, 4), (70, 2056, 0), (333, 36, 0), (333, 32, 1)])
+def test_silu_backward_with_bias_gradient(pkg, P, C, off):
+    import torch
+    lib = pkg.surrogate.nn()
+    rng = np.random.default_rng(P + C)
+    da, z = rng.normal(size=(P, C + off)), rng.normal(0, 3, size=(P, C))
+    dad, zd = up(torch, da), up(torch, z)
+    n = max(lib.lbm_nn_colsum_workspace(P, C), 1)
+    outs = []
+    for fused in (True, False):
+        ws = torch.full((n,), float("nan"), device="cuda")
+        dz = torch.zeros(P, C, device="cuda", dtype=torch.bfloat16)
+        db = torch.zeros(C, device="cuda")
+        if fused:
+            assert lib.lbm_nn_silu_backward_bias(dad.data_ptr(), C + off, off, zd.data_ptr(), P, C, dz.data_ptr(),
+                                                 ws.data_ptr(), db.data_ptr(), None) == 0
+        else:
+            assert lib.lbm_nn_silu_backward(dad.data_ptr(), C + off, off, zd.data_ptr(), P, C, dz.data_ptr(), None) == 0
+            assert lib.lbm_nn_colsum(dz.data_ptr(), P, C, ws.data_ptr(), db.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        outs.append((down(dz), down(db)))
+    assert np.array_equal(outs[0][0], outs[1][0])
+    dz = outs[0][0]
+    for _, db in outs:
+        assert (np.abs(db - dz.sum(0)) <= P * 2.0 ** -23 * np.abs(dz).sum(0)).all()
