@@ -502,7 +502,7 @@ def run_unet(args, world, rank, local):
     forward, MSE loss, backward and Adam of the 4-level U-Net (1.95 M
     parameters, bf16 activations, FP32 accumulation) on a batch of 16
     128 x 128 images (seeded random inputs and targets), with the 3x3
-    convolutions on the chosen tensor-core path (--tensor-path 0: mma.sync,
+    convolutions on the chosen tensor-core path (--tensor-path 0: automatic,
     1: tcgen05 with the accumulator in tensor memory).  roofline: the 3x3
     convolutions' FLOPs (forward, data and weight gradients) per step against
     the measured bf16 GEMM peak."""
@@ -552,7 +552,7 @@ def run_unet(args, world, rank, local):
             "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": False, "scaling": "weak",
             "vs_baseline": None, "dtype": "bf16 (FP32 accumulation)", "data": "synthetic",
             "config": {"workload": "unet", "batch": B, "image": R, "params": int(net.n_params),
-                       "tensor_path": ["mma.sync", "tcgen05"][args.tensor_path]},
+                       "tensor_path": ["automatic", "tcgen05"][args.tensor_path]},
             "roofline": {"bound": "tensor", "achieved": tflops, "peak": peak, "unit": "TFLOP/s",
                          "frac": tflops / peak, "traffic": None, "peak_kind": kind,
                          "flops_per_step": flops, "kernel": "3x3 convolutions (fwd, dgrad, wgrad)"},
@@ -659,7 +659,7 @@ def main():
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--workload", default="cavity3d_128",
                     choices=sorted(WORKLOADS) + ["batch256", "steady", "unet"])
-    ap.add_argument("--tensor-path", type=int, default=0, choices=[0, 1], help="unet: 0 mma.sync, 1 tcgen05")
+    ap.add_argument("--tensor-path", type=int, default=0, choices=[0, 1], help="unet: 0 automatic, 1 tcgen05")
     ap.add_argument("--cases", type=int, default=16, help="steady: held-out cavities")
     ap.add_argument("--steady-cases", type=int, default=16,
                     help="cavity workloads: held-out cavities of the time_to_steady object (0: leave it out)")

@@ -937,22 +937,30 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // ---------------------------------------------------------------------------
 // 3x3 convolution on the 5th-generation tensor cores (tcgen05, TMEM)
 // ---------------------------------------------------------------------------
-// Same implicit GEMM as k_conv3x3 (M = pixels, N = Cout, K = 9 Cin), with the
-// accumulator tile (128 pixels x BN channels, FP32) held in tensor memory:
-//   * 4 warps gather the im2col tile and the weight tile of each K chunk (one
-//     tap, 32 input channels) with cp.async into a 4-stage ring, two chunks
-//     ahead, in the no-swizzle K-major core-matrix layout (8 rows x 16 bytes
-//     per core matrix; K-adjacent core matrices 128 B apart, 8-row groups
-//     512 B apart);
-//   * after a generic-to-async proxy fence and a CTA barrier, one thread issues
-//     two tcgen05.mma (K = 16 each) and commits them to the stage's mbarrier,
-//     which frees the stage for the copy of chunk kc + 4;
-//   * the epilogue reads the accumulators back with tcgen05.ld (warp w owns
-//     TMEM lanes 32w..32w+31, i.e. pixels 32w..32w+31 of the tile).
+// The implicit GEMM of k_conv3x3 (M = pixels, N = Cout, K = 9 Cin) on a tile of
+// 8 x 16 pixels, with the accumulators (128 pixels x BN channels, FP32, NM tiles a
+// block) in tensor memory.  The kernel was bound by gathering the im2col matrix,
+// nine copies of every pixel; here a K chunk is 32 input channels and all nine
+// taps, and its pixels are staged once, with a one-pixel border:
+//   * A lies as four panels of 8 channels, [panel][18 x 10 pixels][16 bytes].  The
+//     8 pixels of a tile row are a core matrix (8 rows of 16 bytes), the rows of
+//     the tile 160 bytes apart (stride offset) and the panels 2880 (leading
+//     offset): in this layout without swizzle a tap is a shift of the start
+//     address by whole 16-byte pixels;
+//   * B is the chunk's weights of the nine taps, [tap][panel][BN][16 bytes];
+//   * one thread issues a chunk's 18 tcgen05.mma (K = 16) per tile and commits
+//     them to the stage's mbarrier; the next chunk is copied meanwhile (two
+//     stages; one where Cin = 32 is all there is, then two tiles a block share
+//     the weights);
+//   * the epilogue reads the accumulators with tcgen05.ld, a thread one pixel and
+//     16 channels at a time, and stores whole 32-byte sectors.
+// Measured at batch 16 of 128^2 images, all forward and data-gradient layers of
+// a training step: mma.sync kernel 1.64 ms, this kernel 1.01 ms.
 // Every mbarrier wait is bounded; on timeout the CTA counts the event in
 // g_nn_timeouts (read by lbm_nn_timeouts), waits (bounded) for its own MMAs,
 // frees its tensor memory and returns.
-constexpr int TBM = 128, TBK = 32, TSTAGES = 4, TTHREADS = 128;
+constexpr int TBM = 128, TBK = 32, TTHREADS = 256;
+constexpr int TTW = 8, TTH = 16, THW = TTW + 2, THP = THW * (TTH + 2);  // pixel tile, its border, their pixels
 constexpr long long kNnWaitCycles = 2000000000LL;  // ~1 s at 1.9 GHz
 __device__ int g_nn_timeouts;
 
@@ -1004,44 +1012,52 @@ __host__ __device__ constexpr uint32_t umma_idesc()
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
 }
 
-template <int BN>
+template <int BN, int NM>
 struct TcLayout {
-    static constexpr int A_BYTES = TBM * TBK * 2;  // 8 KB
-    static constexpr int B_BYTES = BN * TBK * 2;
-    static constexpr int STAGE = A_BYTES + B_BYTES;
-    static constexpr int BAR = TSTAGES * STAGE;    // mbarriers, then the TMEM address
-    static_assert(BAR >= TBM * 33 * 4, "the epilogue stages 128 x 33 floats in the ring");
-    static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "TMEM allocations are powers of two >= 32");
-    static constexpr int SMEM = BAR + 64 + 1024;   // + alignment slack
+    static constexpr int PANEL = THP * 16;             // 2880: 8 channels of the tile and its border
+    static constexpr int A_BYTES = 4 * PANEL;
+    static constexpr int TAP = 4 * BN * 16;            // a tap's weights
+    static constexpr int BOFF = NM * A_BYTES;
+    static constexpr int STAGE = BOFF + 9 * TAP;
+    static constexpr int HEAD = 128 + BN * 4;          // mbarriers, the TMEM address, the channels' bias
+    static constexpr int COLS = NM * BN;               // TMEM columns
+    static_assert(COLS == 32 || COLS == 64 || COLS == 128, "TMEM allocations are powers of two >= 32");
+    static constexpr int smem(int stages) { return HEAD + stages * STAGE + 128; }
     // shared memory bounds the CTAs per SM, so their TMEM columns fit the SM's 512
-    static_assert((228 * 1024 / SMEM) * BN <= 512, "TMEM oversubscription");
-    // byte offset of element (row r, 16-byte piece q) in a K-major no-swizzle tile
-    __device__ static int off(int r, int q) { return (r >> 3) * 512 + q * 128 + (r & 7) * 16; }
+    static_assert((228 * 1024 / smem(1)) * COLS <= 512, "TMEM oversubscription");
 };
 
-template <int BN>
-__global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a)
+__device__ __forceinline__ void st_v8(float *p, const float *v)
 {
-    using Lt = TcLayout<BN>;
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+
+// vec: the outputs' channel strides, offsets and addresses allow 32-byte stores
+template <int BN, int NM, int NST>
+__global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a, int ntx, int nty, int ntiles, int vec)
+{
+    using Lt = TcLayout<BN, NM>;
     extern __shared__ unsigned char tc_raw[];
-    unsigned char *sm = tc_raw + ((1024u - (smem_u32(tc_raw) & 1023u)) & 1023u);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm + Lt::BAR);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + TSTAGES);
+    unsigned char *sm = tc_raw + ((128u - (smem_u32(tc_raw) & 127u)) & 127u);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sm);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + NST);
+    float *sbias = reinterpret_cast<float *>(sm + 128);
+    unsigned char *stages = sm + Lt::HEAD;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t M = (int64_t)a.B * a.H * a.W;
-    const int64_t m0 = (int64_t)blockIdx.x * TBM;
     const int n0 = blockIdx.y * BN;
-    const int cchunks = a.Cin / TBK;
-    const int nk = 9 * cchunks;
+    const int nk = a.Cin / TBK;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(BN)
+                     "r"(Lt::COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (tid < BN) sbias[tid] = a.bias && n0 + tid < a.Cout ? a.bias[n0 + tid] : 0.0f;
     if (tid == 0) {
-        for (int s = 0; s < TSTAGES; ++s) nn_mbar_init(&bars[s], 1);
+        for (int k = 0; k < NST; ++k) nn_mbar_init(&bars[k], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tc_fence_before();
@@ -1049,61 +1065,52 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // the four A pieces of this thread: rows r = (tid + 128 i) / 4, 16-byte piece q
-    int ab[4], ay[4], ax[4];
-    bool av[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = (tid + i * TTHREADS) >> 2;
-        const int64_t m = m0 + r;
-        av[i] = m < M;
-        const int64_t mm = av[i] ? m : 0;
-        ax[i] = int(mm % a.W);
-        ay[i] = int((mm / a.W) % a.H);
-        ab[i] = int(mm / ((int64_t)a.W * a.H));
-    }
     auto load = [&](int kc) {
-        unsigned char *st = sm + (kc % TSTAGES) * Lt::STAGE;
-        const int tap = kc / cchunks, c0 = (kc % cchunks) * TBK;
-        const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+        unsigned char *st = stages + (kc % NST) * Lt::STAGE;
+        const int c0 = kc * TBK;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int v = tid + i * TTHREADS, r = v >> 2, q = v & 3;
-            const int yy = ay[i] + dy, xx = ax[i] + dx;
-            const bool ok = av[i] && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-            const bf16 *src = ok ? a.x + ((int64_t)(ab[i] * a.H + yy) * a.W + xx) * a.xs + a.xo + c0 + q * 8 : a.x;
-            cp_async16(st + Lt::off(r, q), src, ok ? 16 : 0);
+        for (int i = 0; i < NM; ++i) {
+            const int t = blockIdx.x * NM + i;
+            const int x0 = (t % ntx) * TTW - 1, y0 = ((t / ntx) % nty) * TTH - 1, b = t / (ntx * nty);
+            for (int v = tid; v < THP * 4; v += TTHREADS) {
+                const int px = v >> 2, q = v & 3;
+                const int xx = x0 + px % THW, yy = y0 + px / THW;
+                const bool ok = t < ntiles && xx >= 0 && xx < a.W && yy >= 0 && yy < a.H;
+                const bf16 *src = a.x + (ok ? (((int64_t)b * a.H + yy) * a.W + xx) * a.xs + a.xo + c0 + q * 8 : 0);
+                cp_async16(st + i * Lt::A_BYTES + q * Lt::PANEL + px * 16, src, ok ? 16 : 0);
+            }
         }
-#pragma unroll
-        for (int i = 0; i < BN / 32; ++i) {
-            const int v = tid + i * TTHREADS, r = v >> 2, q = v & 3;
-            const int n = n0 + r;
-            const bool ok = n < a.Cout;
-            const bf16 *src = ok ? a.w + ((int64_t)n * 9 + tap) * a.Cin + c0 + q * 8 : a.w;
-            cp_async16(st + Lt::A_BYTES + Lt::off(r, q), src, ok ? 16 : 0);
+        for (int v = tid; v < 9 * BN * 4; v += TTHREADS) {
+            const int q = v & 3, n = (v >> 2) % BN, tap = v / (4 * BN);
+            const bool ok = n0 + n < a.Cout;
+            const bf16 *src = a.w + (ok ? ((int64_t)(n0 + n) * 9 + tap) * a.Cin + c0 + q * 8 : 0);
+            cp_async16(st + Lt::BOFF + tap * Lt::TAP + q * (BN * 16) + n * 16, src, ok ? 16 : 0);
         }
     };
 
-    // K-direction core matrices 128 B apart, 8-row groups 512 B apart
-    const uint32_t lbo = 128u, sbo = 512u;
     constexpr uint32_t idesc = umma_idesc<BN>();
     bool fail = false;
     int issued = 0;  // K chunks whose MMAs were issued (uniform over the CTA)
-    // copies run two chunks ahead of the MMAs: the stage refilled at chunk kc
-    // held chunk kc-2, whose MMAs were issued an iteration earlier and have
-    // normally completed, so the wait below rarely stalls
-    constexpr int AHEAD = TSTAGES - 2;
+    // copies run AHEAD chunks in front of the MMAs; the stage refilled for chunk kc + AHEAD held chunk
+    // kc + AHEAD - NST, whose MMAs were issued an iteration or more earlier
+    constexpr int AHEAD = NST - 1;
+    if (NST == 1) {
+        load(0);
+        cp_commit();
+    }
     for (int kc = 0; kc < AHEAD; ++kc) {
         if (kc < nk) load(kc);
         cp_commit();
     }
     for (int kc = 0; kc < nk; ++kc) {
-        const int nxt = kc + AHEAD;
-        if (nxt < nk) {
-            if (kc >= 2 && !nn_mbar_wait(&bars[(kc - 2) % TSTAGES], uint32_t(((kc - 2) / TSTAGES) & 1))) fail = true;
-            if (!fail) load(nxt);
+        if (NST > 1) {
+            const int nx = kc + AHEAD;
+            if (nx < nk) {
+                if (nx >= NST && !nn_mbar_wait(&bars[nx % NST], uint32_t((nx / NST - 1) & 1))) fail = true;
+                if (!fail) load(nx);
+            }
+            cp_commit();
         }
-        cp_commit();
         cp_wait<AHEAD>();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
@@ -1113,21 +1120,30 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a)
         }
         tc_fence_after();
         if (tid == 0) {
-            const uint32_t base = smem_u32(sm + (kc % TSTAGES) * Lt::STAGE);
+            const uint32_t base = smem_u32(stages + (kc % NST) * Lt::STAGE);
+#pragma unroll 1
+            for (int tap = 0; tap < 9; ++tap) {
+                const uint32_t shift = uint32_t((tap / 3) * THW + tap % 3) * 16u;
 #pragma unroll
-            for (int ks = 0; ks < TBK; ks += 16) {
-                const uint64_t da = umma_desc(base + (ks / 8) * 128, lbo, sbo);
-                const uint64_t db = umma_desc(base + Lt::A_BYTES + (ks / 8) * 128, lbo, sbo);
-                const uint32_t accum = (kc > 0 || ks > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(idesc), "r"(accum)
-                    : "memory");
+                for (int ks = 0; ks < TBK; ks += 16) {
+                    const uint64_t db =
+                        umma_desc(base + Lt::BOFF + tap * Lt::TAP + (ks / 8) * (BN * 16), BN * 16, 128);
+                    const uint32_t accum = (kc > 0 || tap > 0 || ks > 0) ? 1u : 0u;
+#pragma unroll
+                    for (int i = 0; i < NM; ++i) {
+                        const uint64_t da = umma_desc(base + i * Lt::A_BYTES + (ks / 8) * Lt::PANEL + shift,
+                                                      Lt::PANEL, THW * 16);
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + i * BN),
+                            "l"(da), "l"(db), "r"(idesc), "r"(accum)
+                            : "memory");
+                    }
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&bars[kc % TSTAGES]))
+                             smem_u32(&bars[kc % NST]))
                          : "memory");
         }
         ++issued;
@@ -1136,60 +1152,112 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a)
     // chunk arrives (bounded: also on the failure path, before the tensor
     // memory is freed)
     bool done = true;
-    if (issued > 0) done = nn_mbar_wait(&bars[(issued - 1) % TSTAGES], uint32_t(((issued - 1) / TSTAGES) & 1));
+    if (issued > 0) done = nn_mbar_wait(&bars[(issued - 1) % NST], uint32_t(((issued - 1) / NST) & 1));
     cp_wait<0>();
     tc_fence_after();
     if (__syncthreads_or(fail || !done)) {
         if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
     } else {
-        // the ring is free now: stage each 32-column slice of the accumulator
-        // (thread = pixel row) and write it out row by row with the lanes on
-        // consecutive channels, so every store instruction is coalesced
-        float *stg = reinterpret_cast<float *>(sm);   // 128 x 33 floats, fits the ring
+        // warp w reads TMEM lanes 32 (w % 4) ..: pixels 4 tile rows; two warpgroups split the tiles (NM = 2) or
+        // the channel slices
+        const int wg = warp >> 2;
+        const int t = blockIdx.x * NM + (NM == 2 ? wg : 0);
+        const int row = (warp & 3) * 32 + lane;
+        const int xx = (t % ntx) * TTW + (row & 7), yy = ((t / ntx) % nty) * TTH + (row >> 3), b = t / (ntx * nty);
+        const bool px = t < ntiles && xx < a.W && yy < a.H;
+        const int64_t m = ((int64_t)b * a.H + yy) * a.W + xx;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-            uint32_t r[32];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+        for (int sl = NM == 2 ? 0 : wg; sl < BN / 16; sl += NM == 2 ? 1 : 2) {
+            uint32_t r[16];
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) +
+                                   (uint32_t)((NM == 2 ? wg * BN : 0) + sl * 16);
             asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15},"
+                " [%16];"
                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                  "=r"(r[15])
                 : "r"(taddr)
                 : "memory");
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int row = warp * 32 + lane;
+            const int n = n0 + sl * 16;
+            if (!px || n >= a.Cout) continue;
+            float z[16];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) stg[row * 33 + j] = __uint_as_float(r[j]);
-            __syncthreads();
-            const int n = n0 + c0 + lane;
-            if (n < a.Cout) {
-                const float bia = a.bias ? a.bias[n] : 0.0f;
-#pragma unroll 4
-                for (int rr = 0; rr < 32; ++rr) {
-                    const int rl = warp * 32 + rr;
-                    const int64_t m = m0 + rl;
-                    if (m >= M) break;
-                    const float z = stg[rl * 33 + lane] + bia;
-                    if (a.of) {
-                        float *p = a.of + m * a.os + a.oo + n;
-                        *p = a.acc ? *p + z : z;
+            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]) + sbias[sl * 16 + j];
+            if (vec && n + 16 <= a.Cout) {
+                if (a.of) {
+                    float *p = a.of + m * a.os + a.oo + n;
+                    st_v8(p, z);
+                    st_v8(p + 8, z + 8);
+                }
+                if (a.oa) {
+                    float h[8];
+#pragma unroll
+                    for (int j = 0; j < 16; j += 2) {
+                        const __nv_bfloat162 v = a.act ? __floats2bfloat162_rn(silu(z[j]), silu(z[j + 1]))
+                                                       : __floats2bfloat162_rn(z[j], z[j + 1]);
+                        h[j / 2] = *reinterpret_cast<const float *>(&v);
                     }
-                    if (a.oa) a.oa[m * a.as + a.ao + n] = __float2bfloat16_rn(a.act ? silu(z) : z);
+                    st_v8(reinterpret_cast<float *>(a.oa + m * a.as + a.ao + n), h);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (n + j >= a.Cout) break;
+                    if (a.of) {
+                        float *p = a.of + m * a.os + a.oo + n + j;
+                        *p = a.acc ? *p + z[j] : z[j];
+                    }
+                    if (a.oa) a.oa[m * a.as + a.ao + n + j] = __float2bfloat16_rn(a.act ? silu(z[j]) : z[j]);
                 }
             }
-            __syncthreads();
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Lt::COLS) : "memory");
 }
 
-int g_use_tc = 0;          // 0: mma.sync (the default, faster on these layer sizes), 1: tcgen05 (lbm_nn_set_tensor_path)
+template <int BN, int NM, int NST>
+void launch_conv_tc(const ConvArgs &a, int vec, cudaStream_t s)
+{
+    using Lt = TcLayout<BN, NM>;
+    const int ntx = (a.W + TTW - 1) / TTW, nty = (a.H + TTH - 1) / TTH, ntiles = a.B * ntx * nty;
+    cudaFuncSetAttribute(k_conv3x3_tc<BN, NM, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lt::smem(NST));
+    dim3 grid(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
+    k_conv3x3_tc<BN, NM, NST><<<grid, TTHREADS, Lt::smem(NST), s>>>(a, ntx, nty, ntiles, vec);
+}
+
+int64_t tc_tiles(const ConvArgs &a) { return (int64_t)a.B * ((a.W + TTW - 1) / TTW) * ((a.H + TTH - 1) / TTH); }
+
+// Tiles and channels per block and stages of the ring: where Cin = 32 is one
+// chunk, one stage, and two tiles share the weights if there are tiles enough
+// for every SM; otherwise two stages, so that two blocks share an SM (four
+// stages, one block an SM: 47 us for 256 channels at 16 x 16, batch 16, against
+// 30 us), and 32 channels a block where 64 would leave SMs idle.
+void conv_tc(const ConvArgs &a, cudaStream_t s)
+{
+    const int64_t tiles = tc_tiles(a);
+    const auto ok32 = [](const void *p) { return ((uintptr_t)p & 31u) == 0; };
+    const int vec = !a.acc && (!a.of || ((a.os | a.oo) % 8 == 0 && ok32(a.of))) &&
+                    (!a.oa || ((a.as | a.ao) % 16 == 0 && ok32(a.oa)));
+    const bool few = tiles * ((a.Cout + 63) / 64) < 148;
+    if (a.Cin == TBK) {
+        const bool two = tiles >= 592;
+        if (a.Cout <= 32 || few)
+            two ? launch_conv_tc<32, 2, 1>(a, vec, s) : launch_conv_tc<32, 1, 1>(a, vec, s);
+        else
+            two ? launch_conv_tc<64, 2, 1>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
+    } else if (a.Cout <= 32 || few) {
+        launch_conv_tc<32, 1, 2>(a, vec, s);
+    } else {
+        launch_conv_tc<64, 1, 2>(a, vec, s);
+    }
+}
+
+int g_path = 0;            // lbm_nn_set_tensor_path: 0 the faster kernel for the tensors at hand, 1 tcgen05
 
 }  // namespace
 
@@ -1216,24 +1284,13 @@ extern "C" int lbm_nn_conv3x3(const void *x, int64_t xs, int32_t xo, const void 
                (bf16 *)oa, as, ao, act};
     const int64_t M = (int64_t)B * H * W;
     cudaStream_t s = (cudaStream_t)stream;
-    if (g_use_tc) {
-        const int bn = Cout <= 32 ? 32 : (Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256));
-        dim3 grid(unsigned((M + TBM - 1) / TBM), unsigned((Cout + bn - 1) / bn));
-        if (bn == 32) {
-            cudaFuncSetAttribute(k_conv3x3_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout<32>::SMEM);
-            k_conv3x3_tc<32><<<grid, TTHREADS, TcLayout<32>::SMEM, s>>>(a);
-        } else if (bn == 64) {
-            cudaFuncSetAttribute(k_conv3x3_tc<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout<64>::SMEM);
-            k_conv3x3_tc<64><<<grid, TTHREADS, TcLayout<64>::SMEM, s>>>(a);
-        } else if (bn == 128) {
-            cudaFuncSetAttribute(k_conv3x3_tc<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout<128>::SMEM);
-            k_conv3x3_tc<128><<<grid, TTHREADS, TcLayout<128>::SMEM, s>>>(a);
-        } else {
-            // 256 TMEM columns per CTA; its 97 KB of shared memory keep at most
-            // two CTAs on an SM, within the SM's 512 columns
-            cudaFuncSetAttribute(k_conv3x3_tc<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcLayout<256>::SMEM);
-            k_conv3x3_tc<256><<<grid, TTHREADS, TcLayout<256>::SMEM, s>>>(a);
-        }
+    // The tcgen05 kernel is the faster on the network's layers (batch 16: 31 us against 59 for 32 -> 32 channels at
+    // 128 x 128, 29 against 55 for 256 -> 256 at 16 x 16) and on any call of few blocks.  mma.sync takes pixels in a
+    // row, across images, and wins where more than two blocks an SM would mostly hold padding (256 images of 9 x 9,
+    // 64 channels: 27 us against 33; of 2 x 2, 256 channels: 53 against 135; a tile half full: 33 against 17).
+    const int64_t tiles = tc_tiles(a);
+    if (g_path == 1 || 8 * M >= 3 * tiles * TTW * TTH || tiles * ((Cout + 63) / 64) <= 296) {
+        conv_tc(a, s);
         return launched("lbm_nn_conv3x3 (tcgen05)");
     }
     if (Cout <= 32) {
@@ -1491,12 +1548,12 @@ extern "C" int lbm_nn_to_bf16(const float *x, void *y, int64_t n, void *stream)
 
 extern "C" int lbm_nn_set_tensor_path(int32_t path)
 {
-    NN_REQUIRE(path == 0 || path == 1, "lbm_nn_set_tensor_path: path must be 0 (mma.sync) or 1 (tcgen05)");
-    g_use_tc = path == 1;
+    NN_REQUIRE(path == 0 || path == 1, "lbm_nn_set_tensor_path: path must be 0 (automatic) or 1 (tcgen05)");
+    g_path = path;
     return LBM_OK;
 }
 
-extern "C" int lbm_nn_get_tensor_path(void) { return g_use_tc ? 1 : 0; }
+extern "C" int lbm_nn_get_tensor_path(void) { return g_path; }
 
 extern "C" int lbm_nn_timeouts(int32_t *count, int32_t reset)
 {

@@ -21,6 +21,52 @@ def down(t):
     return t.float().cpu().numpy().astype(np.float64)
 
 
+# (B, H, W): one pixel; a tile exactly; one past it each way; thin; many images far smaller than a tile
+@pytest.mark.parametrize("path", [0, 1])
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [(1, 1, 1, 32, 8), (2, 16, 8, 32, 32), (2, 17, 9, 64, 40), (1, 33, 7, 96, 96),
+                                            (3, 15, 25, 160, 48), (80, 16, 8, 32, 72), (300, 2, 2, 64, 64)])
+def test_convolution_tile_edges(pkg, B, H, W, Cin, Cout, path):
+    import torch
+    S = pkg.surrogate
+    lib = S.nn()
+    rng = np.random.default_rng(B * H * W + Cin + Cout)
+    x = U.bf16_round(rng.normal(size=(B, H, W, Cin + 8)))
+    w = U.bf16_round(rng.normal(0, 0.1, size=(Cout, 9, Cin)))
+    bias = rng.normal(size=Cout).astype(np.float32).astype(np.float64)
+    bf = torch.bfloat16
+    xd, wd, bd = up(torch, x, bf), up(torch, w, bf), up(torch, bias)
+    S.timeouts(reset=True)
+    S.set_tensor_path(path)
+    try:
+        got = {}
+        for pad, off in ((0, 0), (3, 1)):  # wide stores; odd strides and offsets
+            z = torch.full((B, H, W, Cout + pad), 7.0, device="cuda")
+            a = torch.full((B, H, W, Cout + pad), 7.0, device="cuda", dtype=bf)
+            acc = torch.ones((B, H, W, Cout + pad), device="cuda")
+            assert lib.lbm_nn_conv3x3(xd.data_ptr(), Cin + 8, 8, wd.data_ptr(), bd.data_ptr(), B, H, W, Cin, Cout,
+                                      z.data_ptr(), Cout + pad, off, 0, a.data_ptr(), Cout + pad, off, 1, None) == 0
+            assert lib.lbm_nn_conv3x3(xd.data_ptr(), Cin + 8, 8, wd.data_ptr(), None, B, H, W, Cin, Cout,
+                                      acc.data_ptr(), Cout + pad, off, 1, None, 0, 0, 0, None) == 0
+            torch.cuda.synchronize()
+            sl = slice(off, off + Cout)
+            keep = [c for c in range(Cout + pad) if not off <= c < off + Cout]
+            assert all((down(t)[..., keep] == v).all() for t, v in ((z, 7.0), (a, 7.0), (acc, 1.0)))
+            got[pad] = tuple(down(t)[..., sl] for t in (z, a, acc))
+    finally:
+        S.set_tensor_path(0)
+    assert S.timeouts(reset=True) == 0
+    for u, v in zip(got[0], got[3]):
+        assert np.array_equal(u, v)
+    z, a, acc = got[0]
+    ref = U.conv3x3(x[..., 8:], w, np.zeros(Cout))
+    size = U.conv3x3(np.abs(x[..., 8:]), np.abs(w), np.zeros(Cout))
+    tol = (9 * Cin + 2) * 2.0 ** -23
+    assert (np.abs(z - (ref + bias)) <= tol * (size + np.abs(bias))).all()
+    assert (np.abs(acc - 1.0 - ref) <= tol * (size + 1.0)).all()
+    s = U.silu(z)
+    assert (np.abs(a - s) <= 2.0 ** -8 * np.abs(s) + 2.0 ** -8 * 2.0 ** -12).all()
+
+
 @pytest.mark.parametrize("B,H,W,Cin,Cout", [(1, 1, 1, 32, 8), (2, 8, 16, 32, 32), (2, 9, 17, 64, 40), (1, 7, 33, 96, 72),
                                             (5, 24, 31, 32, 64), (40, 3, 2, 64, 32)])
 def test_weight_gradient_tile_edges(pkg, B, H, W, Cin, Cout):
