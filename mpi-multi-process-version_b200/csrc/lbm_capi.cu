@@ -325,6 +325,7 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
     const MarchShape ms = march_shape(g.dim, h->p.storage, tx, h->tiley);
     // the fast build's 2D march: one box of all planes per row
     const int wb = g.dim == 2 && h->p.mode != LBM_MODE_EXACT ? march2d_box(h->p.storage, tx ? tx : h->nt) : 0;
+    const bool pairs = g.dim == 3 && h->p.mode != LBM_MODE_EXACT;
     const CUtensorMapDataType dtype =
         h->p.storage == LBM_STORE_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     const cuuint64_t es = h->esize;
@@ -334,14 +335,16 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
                                          : h->l2promo == 1 ? CU_TENSOR_MAP_L2_PROMOTION_L2_64B
                                                            : CU_TENSOR_MAP_L2_PROMOTION_NONE;
     for (int buf = 0; buf < 2; ++buf) {
-        for (int c = 0; c < 4; ++c) {
-            CUtensorMap *m = &out[buf].m[c];
+        for (int k = 0; k < (pairs ? 5 : 4); ++k) {
+            CUtensorMap *m = k < 4 ? &out[buf].m[k] : &out[buf].one;
+            const int c = k & 3;
             CUresult r;
             if (g.dim == 3) {
                 const cuuint64_t dims[4] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz, (cuuint64_t)nplanes};
                 const cuuint64_t strides[3] = {(cuuint64_t)g.pitch * es, (cuuint64_t)g.slab * es,
                                                (cuuint64_t)g.plane * es};
-                const cuuint32_t box[4] = {(cuuint32_t)ms.bx[c], (cuuint32_t)ms.by[c], 1, 1};
+                const cuuint32_t box[4] = {(cuuint32_t)ms.bx[c], (cuuint32_t)ms.by[c], 1,
+                                           pairs && k < 4 ? 2u : 1u};
                 const cuuint32_t estr[4] = {1, 1, 1, 1};
                 r = enc(m, dtype, 4, h->bufs.pop[buf], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_NONE, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -394,8 +397,8 @@ static bool march_supported(const lbm_handle *h)
 }
 
 // tile rows of the 3D march kernel unless LBM_OPT_TILEY says otherwise: 32 x 4
-// tiles run two blocks per SM; measured on B200 at 128^3 FP64 (balanced plan)
-// 13.0 GLUPS against 12.0 GLUPS with 32 x 8 tiles and one block per SM
+// tiles run two blocks per SM (four in FP32); a long run at 128^3 takes 163 us a
+// step in FP64 against 167 with 32 x 8 tiles and one block per SM, FP32 84 against 101
 static constexpr int kDefaultTileY = 4;
 
 // ---------------------------------------------------------------------------

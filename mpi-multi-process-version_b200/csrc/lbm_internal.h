@@ -90,11 +90,13 @@ struct Bufs {
     RunCtl *ctl;           // run state; the step kernels return at once while ctl->active is 0
 };
 
-// TMA descriptors of one population buffer (one per box class) and of the
-// carried-force array that goes with it
+// TMA descriptors of one population buffer, one per box class (the fast build's
+// 3D march: two planes a box), and of the carried-force array that goes with it
+// (right behind m: the exact build's 2D kernels index it as m[4])
 struct alignas(64) TmapSet {
     CUtensorMap m[4];
     CUtensorMap fmap;
+    CUtensorMap one;  // fast 3D march: one plane of the tile alone
 };
 
 // Per-cavity tables of a batch of cavities (device memory)

@@ -813,16 +813,18 @@ k_step3d(const Geo G, const typename Tr<ST>::S *__restrict__ src, const typename
     const int64_t id = (int64_t)k * G.slab + (int64_t)j * G.pitch + i;
     const int64_t xa = off_a(i, G.nx), xb = off_b(i, G.nx);
     const int64_t ya = (int64_t)off_a(j, G.ny) * G.pitch, yb = (int64_t)off_b(j, G.ny) * G.pitch;
-    const int64_t za = (int64_t)off_a(k, G.nz) * G.slab, zb = (int64_t)off_b(k, G.nz) * G.slab;
-    C xp[3], xm[3], yp[3], ym[3], zp[3], zm[3];
+    C xp[3], xm[3], yp[3], ym[3];
     load_w(G.wgt[0], i, xp, xm);
     load_w(G.wgt[1], j, yp, ym);
-    load_w(G.wgt[2], k, zp, zm);
 
     auto LD = [&](int q, int64_t off) -> C {
         C val = tocomp(__ldg(src + q * P + id + off));
         return val;
     };
+#if LBM_EXACT
+    const int64_t za = (int64_t)off_a(k, G.nz) * G.slab, zb = (int64_t)off_b(k, G.nz) * G.slab;
+    C zp[3], zm[3];
+    load_w(G.wgt[2], k, zp, zm);
     auto YI = [&](int q, const C w[3], int64_t c) -> C { return ip(w, LD(q, c + ya), LD(q, c), LD(q, c + yb)); };
     auto ZI = [&](int q, const C w[3], int64_t c) -> C { return ip(w, LD(q, c + za), LD(q, c), LD(q, c + zb)); };
 
@@ -859,6 +861,46 @@ k_step3d(const Geo G, const typename Tr<ST>::S *__restrict__ src, const typename
     gg[4] = ip(ym, LD(23, ya), LD(23, 0), LD(23, yb));
     gg[5] = ip(zp, LD(24, za), LD(24, 0), LD(24, zb));
     gg[6] = ip(zm, LD(25, za), LD(25, 0), LD(25, zb));
+#else
+    // in x or y first, then in z (the march kernel's order: it interpolates a slice
+    // once, when it arrives)
+    C zs[2][3];
+    window_weights(G.wgt[2] + (int64_t)k * 6, k, G.nz, zs[0], zs[1]);
+    const int64_t z0 = (int64_t)(win_lo(k, G.nz) - k) * G.slab;
+    auto XI = [&](int q, const C w[3], int64_t c) -> C { return ip3(w, LD(q, c + xa), LD(q, c), LD(q, c + xb)); };
+    auto YI = [&](int q, const C w[3], int64_t c) -> C { return ip3(w, LD(q, c + ya), LD(q, c), LD(q, c + yb)); };
+    auto ZI = [&](int s, auto slice) -> C { return sym3(zs[s], slice(z0), slice(z0 + G.slab), slice(z0 + 2 * G.slab)); };
+    C f[19], gg[7];
+    f[0] = LD(0, 0);
+    f[1] = XI(1, xp, 0);
+    f[2] = XI(2, xm, 0);
+    f[3] = YI(3, yp, 0);
+    f[4] = YI(4, ym, 0);
+    f[5] = ZI(0, [&](int64_t z) { return LD(5, z); });
+    f[6] = ZI(1, [&](int64_t z) { return LD(6, z); });
+    // xoy plane (3M:807-824): y-interpolation on three x-columns, then x
+    f[7] = ip3(xp, YI(7, yp, xa), YI(7, yp, 0), YI(7, yp, xb));
+    f[8] = ip3(xm, YI(8, yp, xa), YI(8, yp, 0), YI(8, yp, xb));
+    f[9] = ip3(xp, YI(9, ym, xa), YI(9, ym, 0), YI(9, ym, xb));
+    f[10] = ip3(xm, YI(10, ym, xa), YI(10, ym, 0), YI(10, ym, xb));
+    // xoz and yoz planes (3M:767-804)
+    f[11] = ZI(0, [&](int64_t z) { return XI(11, xp, z); });
+    f[12] = ZI(0, [&](int64_t z) { return XI(12, xm, z); });
+    f[13] = ZI(1, [&](int64_t z) { return XI(13, xp, z); });
+    f[14] = ZI(1, [&](int64_t z) { return XI(14, xm, z); });
+    f[15] = ZI(0, [&](int64_t z) { return YI(15, yp, z); });
+    f[16] = ZI(0, [&](int64_t z) { return YI(16, ym, z); });
+    f[17] = ZI(1, [&](int64_t z) { return YI(17, yp, z); });
+    f[18] = ZI(1, [&](int64_t z) { return YI(18, ym, z); });
+    // D3Q7 (3M:831-859)
+    gg[0] = LD(19, 0);
+    gg[1] = XI(20, xp, 0);
+    gg[2] = XI(21, xm, 0);
+    gg[3] = YI(22, yp, 0);
+    gg[4] = YI(23, ym, 0);
+    gg[5] = ZI(0, [&](int64_t z) { return LD(24, z); });
+    gg[6] = ZI(1, [&](int64_t z) { return LD(25, z); });
+#endif
     // deviation from the conduction profile along y (the heated axis)
     C Tc = C(0.0);
     if (Tr<ST>::kDevT) {
@@ -1373,7 +1415,7 @@ int march_blocks_per_sm(const Geo &g, int store, int ty, int nt, int levels)
 
 template <int ST, int TY>
 static cudaError_t launch_march3d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
-                                  const Bufs &b, int wm, const int4 *segs, const int *segoff, int nblocks,
+                                  const Bufs &b, int wm, int rev, const int4 *segs, const int *segoff, int nblocks,
                                   bool pdl, cudaStream_t s)
 {
     using S = typename Tr<ST>::S;
@@ -1381,7 +1423,7 @@ static cudaError_t launch_march3d(const Geo &g, const TmapSet &m, const void *Fi
     cudaError_t e = prepare_march3d<ST, TY>();
     if (e != cudaSuccess) return e;
     return launch_k(k_march3d<ST, TY>, nblocks, L3<ST, TY>::NT, L3<ST, TY>::smem(), s, pdl, m, g, (const C *)Fin,
-                    (S *)pout, (C *)Fout, b, wm, segs, segoff, b.err);
+                    (S *)pout, (C *)Fout, b, wm, rev, segs, segoff, b.err);
 }
 
 #if LBM_EXACT
@@ -1438,9 +1480,10 @@ static cudaError_t launch_march(const Geo &g, const TmapSet &m, const void *Fin,
                                 bool pdl, int nt, int levels, cudaStream_t s)
 {
     cudaError_t e;
+    const int rev = pout == b.pop[0];  // steps that read buffer 1 walk downwards (3D, fast build)
     if (g.dim == 3)
-        e = ty == 4 ? launch_march3d<ST, 4>(g, m, Fin, pout, Fout, b, wm, segs, segoff, nblocks, pdl, s)
-                    : launch_march3d<ST, 8>(g, m, Fin, pout, Fout, b, wm, segs, segoff, nblocks, pdl, s);
+        e = ty == 4 ? launch_march3d<ST, 4>(g, m, Fin, pout, Fout, b, wm, rev, segs, segoff, nblocks, pdl, s)
+                    : launch_march3d<ST, 8>(g, m, Fin, pout, Fout, b, wm, rev, segs, segoff, nblocks, pdl, s);
     else
         e = launch_2d<ST>(g, m, Fin, pout, Fout, b, wm, nblocks, segs, segoff, pdl, nt, levels, s);
     ++g_launches;

@@ -8,7 +8,7 @@
 //   * the domain is cut into cross-section tiles of TX x TY nodes (x, y); a
 //     work item is a tile at one z-slice.  In 3D each persistent CTA runs a
 //     host-made list of segments (tile, first slice, end slice) and marches
-//     along z through each; the host plans the lists so that neighbouring
+//     along z through each (the fast build: up and down in turn); the host plans the lists so that neighbouring
 //     tiles are at the same slice at the same time (their shared halo rows
 //     then come from L2) while every SM has an equal share; in 2D each CTA
 //     takes a contiguous, equal share of the (strip-major, row-minor) items;
@@ -16,9 +16,11 @@
 //     shared memory: a box covers the tile plus the in-plane halo the plane's
 //     interpolation stencil needs (x +-HX columns, y +-1 rows);
 //   * planes whose stencil reaches along z (D3Q19 5,6,11-18; D3Q7 5,6) live in
-//     a 4-slot ring indexed by slice, fetched two slices ahead, so each slice
-//     is read once per tile column and serves the steps k-1, k, k+1 (and the
-//     one-sided stencils at the walls); the other planes use a 2-slot ring;
+//     a ring indexed by slice, fetched two slices ahead, so each slice is read
+//     once per tile column and serves the steps k-1, k, k+1 (and the one-sided
+//     stencils at the walls): four slots in the exact build, which reads all
+//     three at each step, three in the fast build (lbm_march3d.cuh); the other
+//     planes use a 2-slot ring;
 //   * one thread issues the copies (cp.async.bulk.tensor with an mbarrier
 //     transaction count), every thread waits on the slot barriers it needs,
 //     computes its node from shared memory and stores the new post-collision
@@ -191,6 +193,14 @@ __device__ __forceinline__ const Geo *stage_geo(const Geo *src, Geo *dst)
     return dst;
 }
 
+// blocks per SM the registers are bounded for.  FP32 32 x 4 tiles: 128 registers
+// and four blocks; 128^3 takes 81 us a step so, 86 with three blocks, 98 with two
+__host__ __device__ constexpr int march3d_min_blocks(int st, int ty)
+{
+    return ty == 8 ? 1 : (st == kF32 && !LBM_EXACT ? 4 : 2);
+}
+
+#if LBM_EXACT
 template <int ST, int TY_ = 8>
 struct L3 {
     using S = typename Tr<ST>::S;
@@ -262,7 +272,7 @@ struct L3 {
 // descriptors of the buffer read this step, the outputs and the buffers.
 template <int ST, int TY_, bool kStage, class CavFn>
 __device__ __forceinline__ void march3d_run(const int4 *__restrict__ segs, int sbeg, int send, CavFn cavity,
-                                            int write_macro, int *err)
+                                            int write_macro, int, int *err)
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
@@ -517,11 +527,15 @@ __device__ __forceinline__ void march3d_run(const int4 *__restrict__ segs, int s
     }
 }
 
+#else
+#include "lbm_march3d.cuh"
+#endif
+
 template <int ST, int TY_>
-__global__ void __launch_bounds__(32 * TY_, TY_ == 8 ? 1 : 2)
+__global__ void __launch_bounds__(32 * TY_, march3d_min_blocks(ST, TY_))
 k_march3d(const __grid_constant__ TmapSet maps, const __grid_constant__ Geo G,
           const typename Tr<ST>::C *__restrict__ Fin, typename Tr<ST>::S *__restrict__ dst,
-          typename Tr<ST>::C *__restrict__ Fout, const __grid_constant__ Bufs B, int write_macro,
+          typename Tr<ST>::C *__restrict__ Fout, const __grid_constant__ Bufs B, int write_macro, int rev,
           const int4 *__restrict__ segs, const int *__restrict__ seg_off, int *err)
 {
     (void)Fin;
@@ -534,13 +548,13 @@ k_march3d(const __grid_constant__ TmapSet maps, const __grid_constant__ Geo G,
         Fo = Fout;
         Bp = &B;
     };
-    march3d_run<ST, TY_, false>(segs, seg_off[blockIdx.x], seg_off[blockIdx.x + 1], cavity, write_macro, err);
+    march3d_run<ST, TY_, false>(segs, seg_off[blockIdx.x], seg_off[blockIdx.x + 1], cavity, write_macro, rev, err);
 }
 
 // many 3D cavities: segments (tile, z0, z1, cavity) of the batch's work list;
 // `cur` is the ping-pong buffer holding the populations read this step
 template <int ST, int TY_>
-__global__ void __launch_bounds__(32 * TY_, TY_ == 8 ? 1 : 2)
+__global__ void __launch_bounds__(32 * TY_, march3d_min_blocks(ST, TY_))
 k_march3d_batch(const BatchDev D, int cur, int write_macro, int *err)
 {
     using S = typename Tr<ST>::S;
@@ -552,7 +566,7 @@ k_march3d_batch(const BatchDev D, int cur, int write_macro, int *err)
         d = (S *)D.bufs[c].pop[1 - cur];
         Fo = (C *)D.bufs[c].F[1 - cur];
     };
-    march3d_run<ST, TY_, true>(D.segs, D.seg_off[blockIdx.x], D.seg_off[blockIdx.x + 1], cavity, write_macro, err);
+    march3d_run<ST, TY_, true>(D.segs, D.seg_off[blockIdx.x], D.seg_off[blockIdx.x + 1], cavity, write_macro, cur, err);
 }
 
 // ---------------------------------------------------------------------------

@@ -46,6 +46,17 @@ __device__ __forceinline__ C lin2(C w0, C w1, C a, C m) { return fma_(w1, m, mul
 template <class C>
 __device__ __forceinline__ C lin3(const C w[3], C a, C m, C b) { return fma_(w[2], b, lin2(w[0], w[1], a, m)); }
 
+// the same with the operands in table order (a, m, b)
+template <class C>
+__device__ __forceinline__ C ip3(const C w[3], C a, C m, C b) { return fma_(w[2], b, fma_(w[1], m, mul_(w[0], a))); }
+
+// and in an order that is the same from either end of the window
+template <class C>
+__device__ __forceinline__ C sym3(const C w[3], C a, C m, C b)
+{
+    return fma_(w[1], m, add_(mul_(w[0], a), mul_(w[2], b)));
+}
+
 // the collision's constants (relax_setup, lbm_internal.h) in the compute type
 template <class C>
 struct Relax {
