@@ -315,6 +315,8 @@ static EncodeTiledFn encode_fn()
     return fn;
 }
 
+void *lbm::tensor_map_encoder() { return (void *)encode_fn(); }
+
 // Describe a population buffer as a (x, y, [z,] plane) tensor; one descriptor
 // per box class of the march kernel.  Returns false if TMA cannot be used.
 bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])

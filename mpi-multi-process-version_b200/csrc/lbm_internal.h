@@ -227,6 +227,7 @@ extern int64_t g_launches;  // kernels launched by this library
 
 // record a message for lbm_last_error() and return code
 int set_error(int code, const char *fmt, ...);
+void *tensor_map_encoder();  // cuTensorMapEncodeTiled, NULL if there is none
 
 // tile shape of the march kernels (identical in both arithmetic modes); tx
 // selects the tile width of the 2D kernels (0: the single-cavity default),

@@ -14,6 +14,7 @@
 //                (deterministic).
 // Elementwise work (SiLU backward, pooling, upsampling, the 1x1 output layer,
 // the loss, Adam) is plain CUDA-core code.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -25,6 +26,7 @@
 namespace lbm {
 int set_error(int code, const char *fmt, ...);
 extern int64_t g_launches;
+void *tensor_map_encoder();  // cuTensorMapEncodeTiled, NULL if there is none
 }  // namespace lbm
 
 namespace {
@@ -948,14 +950,17 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 //     offset): in this layout without swizzle a tap is a shift of the start
 //     address by whole 16-byte pixels;
 //   * B is the chunk's weights of the nine taps, [tap][panel][BN][16 bytes];
-//   * one thread issues a chunk's 18 tcgen05.mma (K = 16) per tile and commits
-//     them to the stage's mbarrier; the next chunk is copied meanwhile (two
-//     stages; one where Cin = 32 is all there is, then two tiles a block share
-//     the weights);
+//   * one thread issues the copies, one TMA box for a tile's pixels (zero outside
+//     the image) and one for the weights, another a chunk's 18 tcgen05.mma (K =
+//     16) per tile, committed to the stage's mbarrier; copies by all threads took
+//     2000 cycles a chunk for their addresses, as long as the MMAs;
+//   * the launch is a programmatic dependent: its set-up overlaps the end of the
+//     kernel before;
 //   * the epilogue reads the accumulators with tcgen05.ld, a thread one pixel and
 //     16 channels at a time, and stores whole 32-byte sectors.
 // Measured at batch 16 of 128^2 images, all forward and data-gradient layers of
-// a training step: mma.sync kernel 1.64 ms, this kernel 1.01 ms.
+// a training step: mma.sync kernel 1.64 ms, with copies by all threads 1.01 ms,
+// this kernel 0.86 ms; 256 -> 256 at 16 x 16, batch 1: 53, 24 and 14 us.
 // Every mbarrier wait is bounded; on timeout the CTA counts the event in
 // g_nn_timeouts (read by lbm_nn_timeouts), waits (bounded) for its own MMAs,
 // frees its tensor memory and returns.
@@ -1034,14 +1039,38 @@ __device__ __forceinline__ void st_v8(float *p, const float *v)
                  : "memory");
 }
 
+__device__ __forceinline__ void nn_expect(uint64_t *b, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void nn_tma4(void *dst, const CUtensorMap *m, uint64_t *bar, int c1, int c2, int c3)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)), "l"(m), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+        : "memory");
+}
+
+__device__ __forceinline__ void nn_tma5(void *dst, const CUtensorMap *m, uint64_t *bar, int c1, int c2, int c3, int c4)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
+        "%6}], [%7];" ::"r"(smem_u32(dst)), "l"(m), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
+        : "memory");
+}
+
 // vec: the outputs' channel strides, offsets and addresses allow 32-byte stores
 template <int BN, int NM, int NST>
-__global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a, int ntx, int nty, int ntiles, int vec)
+__global__ void __launch_bounds__(TTHREADS)
+k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, int ntx,
+             int nty, int ntiles, int vec)
 {
     using Lt = TcLayout<BN, NM>;
     extern __shared__ unsigned char tc_raw[];
     unsigned char *sm = tc_raw + ((128u - (smem_u32(tc_raw) & 127u)) & 127u);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sm);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm);  // a stage's copies have landed
+    uint64_t *bars = full + NST;                        // the MMAs that read it are complete
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + NST);
     float *sbias = reinterpret_cast<float *>(sm + 128);
     unsigned char *stages = sm + Lt::HEAD;
@@ -1049,77 +1078,58 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a, int n
     const int n0 = blockIdx.y * BN;
     const int nk = a.Cin / TBK;
 
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(Lt::COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid < BN) sbias[tid] = a.bias && n0 + tid < a.Cout ? a.bias[n0 + tid] : 0.0f;
     if (tid == 0) {
-        for (int k = 0; k < NST; ++k) nn_mbar_init(&bars[k], 1);
+        for (int k = 0; k < NST; ++k) {
+            nn_mbar_init(&full[k], 1);
+            nn_mbar_init(&bars[k], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on: what earlier kernels wrote
+    if (tid < BN) sbias[tid] = a.bias && n0 + tid < a.Cout ? a.bias[n0 + tid] : 0.0f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    auto load = [&](int kc) {
-        unsigned char *st = stages + (kc % NST) * Lt::STAGE;
-        const int c0 = kc * TBK;
-#pragma unroll
-        for (int i = 0; i < NM; ++i) {
-            const int t = blockIdx.x * NM + i;
-            const int x0 = (t % ntx) * TTW - 1, y0 = ((t / ntx) % nty) * TTH - 1, b = t / (ntx * nty);
-            for (int v = tid; v < THP * 4; v += TTHREADS) {
-                const int px = v >> 2, q = v & 3;
-                const int xx = x0 + px % THW, yy = y0 + px / THW;
-                const bool ok = t < ntiles && xx >= 0 && xx < a.W && yy >= 0 && yy < a.H;
-                const bf16 *src = a.x + (ok ? (((int64_t)b * a.H + yy) * a.W + xx) * a.xs + a.xo + c0 + q * 8 : 0);
-                cp_async16(st + i * Lt::A_BYTES + q * Lt::PANEL + px * 16, src, ok ? 16 : 0);
-            }
-        }
-        for (int v = tid; v < 9 * BN * 4; v += TTHREADS) {
-            const int q = v & 3, n = (v >> 2) % BN, tap = v / (4 * BN);
-            const bool ok = n0 + n < a.Cout;
-            const bf16 *src = a.w + (ok ? ((int64_t)(n0 + n) * 9 + tap) * a.Cin + c0 + q * 8 : 0);
-            cp_async16(st + Lt::BOFF + tap * Lt::TAP + q * (BN * 16) + n * 16, src, ok ? 16 : 0);
-        }
-    };
-
     constexpr uint32_t idesc = umma_idesc<BN>();
     bool fail = false;
-    int issued = 0;  // K chunks whose MMAs were issued (uniform over the CTA)
-    // copies run AHEAD chunks in front of the MMAs; the stage refilled for chunk kc + AHEAD held chunk
-    // kc + AHEAD - NST, whose MMAs were issued an iteration or more earlier
-    constexpr int AHEAD = NST - 1;
-    if (NST == 1) {
-        load(0);
-        cp_commit();
-    }
-    for (int kc = 0; kc < AHEAD; ++kc) {
-        if (kc < nk) load(kc);
-        cp_commit();
-    }
-    for (int kc = 0; kc < nk; ++kc) {
-        if (NST > 1) {
-            const int nx = kc + AHEAD;
-            if (nx < nk) {
-                if (nx >= NST && !nn_mbar_wait(&bars[nx % NST], uint32_t((nx / NST - 1) & 1))) fail = true;
-                if (!fail) load(nx);
+    if (tid == 32) {  // the copies
+        int kc = 0;
+        for (; kc < nk; ++kc) {
+            const int st = kc % NST;
+            if (kc >= NST && !nn_mbar_wait(&bars[st], uint32_t((kc / NST - 1) & 1))) {
+                fail = true;
+                break;
             }
-            cp_commit();
+            unsigned char *base = stages + st * Lt::STAGE;
+            const int t0 = blockIdx.x * NM, live = NM == 1 || t0 + 1 < ntiles ? NM : 1;
+            nn_expect(&full[st], uint32_t(live * Lt::A_BYTES + 9 * Lt::TAP));
+            for (int i = 0; i < live; ++i) {
+                const int t = t0 + i;
+                nn_tma5(base + i * Lt::A_BYTES, &xmap, &full[st], (t % ntx) * TTW - 1, ((t / ntx) % nty) * TTH - 1,
+                        kc * 4, t / (ntx * nty));
+            }
+            nn_tma4(base + Lt::BOFF, &wmap, &full[st], n0, kc * 4, 0);
         }
-        cp_wait<AHEAD>();
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        tc_fence_before();
-        if (__syncthreads_or(fail)) {
-            fail = true;
-            break;
-        }
-        tc_fence_after();
-        if (tid == 0) {
+        if (fail)  // copies still in flight land before the shared memory is released
+            for (int k = kc > NST ? kc - NST : 0; k < kc; ++k) nn_mbar_wait(&full[k % NST], uint32_t((k / NST) & 1));
+    } else if (tid == 0) {  // the MMAs
+        int kc = 0;
+        for (; kc < nk; ++kc) {
+            if (!nn_mbar_wait(&full[kc % NST], uint32_t((kc / NST) & 1))) {
+                fail = true;
+                break;
+            }
+            tc_fence_after();
             const uint32_t base = smem_u32(stages + (kc % NST) * Lt::STAGE);
 #pragma unroll 1
             for (int tap = 0; tap < 9; ++tap) {
@@ -1146,14 +1156,12 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a, int n
                              smem_u32(&bars[kc % NST]))
                          : "memory");
         }
-        ++issued;
+        // the MMAs that were issued complete before the tensor memory is freed
+        if (fail && kc > 0) nn_mbar_wait(&bars[(kc - 1) % NST], uint32_t(((kc - 1) / NST) & 1));
     }
-    // every MMA of this CTA is complete once the commit of the last issued
-    // chunk arrives (bounded: also on the failure path, before the tensor
-    // memory is freed)
-    bool done = true;
-    if (issued > 0) done = nn_mbar_wait(&bars[(issued - 1) % NST], uint32_t(((issued - 1) / NST) & 1));
-    cp_wait<0>();
+    __syncwarp();
+    // every MMA of this CTA is complete once the commit of the last chunk arrives
+    const bool done = nn_mbar_wait(&bars[(nk - 1) % NST], uint32_t(((nk - 1) / NST) & 1));
     tc_fence_after();
     if (__syncthreads_or(fail || !done)) {
         if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
@@ -1220,41 +1228,80 @@ __global__ void __launch_bounds__(TTHREADS) k_conv3x3_tc(const ConvArgs a, int n
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Lt::COLS) : "memory");
 }
 
+// the input as (channel of 8, x, y, panel of 8 channels, image): a box is a tile with its border in the layout above,
+// zero outside the image; the weights as (channel of 8, output channel, panel, tap)
+bool conv_maps(const ConvArgs &a, int BN, CUtensorMap *xm, CUtensorMap *wm)
+{
+    typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                               const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    const Encode enc = (Encode)lbm::tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+    const cuuint64_t row = (cuuint64_t)a.xs * 2;
+    const cuuint64_t xd[5] = {8, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.Cin / 8, (cuuint64_t)a.B};
+    const cuuint64_t xst[4] = {row, row * a.W, 16, row * a.W * a.H};
+    const cuuint32_t xb[5] = {8, THW, TTH + 2, TBK / 8, 1};
+    const cuuint64_t wd[4] = {8, (cuuint64_t)a.Cout, (cuuint64_t)a.Cin / 8, 9};
+    const cuuint64_t wst[3] = {(cuuint64_t)a.Cin * 18, 16, (cuuint64_t)a.Cin * 2};
+    const cuuint32_t wb[4] = {8, (cuuint32_t)BN, TBK / 8, 9};
+    return enc(xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void *)(a.x + a.xo), xd, xst, xb, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
+           enc(wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.w, wd, wst, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+               CUDA_SUCCESS;
+}
+
 template <int BN, int NM, int NST>
-void launch_conv_tc(const ConvArgs &a, int vec, cudaStream_t s)
+bool launch_conv_tc(const ConvArgs &a, int vec, cudaStream_t s)
 {
     using Lt = TcLayout<BN, NM>;
+    CUtensorMap xm, wm;
+    if (!conv_maps(a, BN, &xm, &wm)) return false;
     const int ntx = (a.W + TTW - 1) / TTW, nty = (a.H + TTH - 1) / TTH, ntiles = a.B * ntx * nty;
     cudaFuncSetAttribute(k_conv3x3_tc<BN, NM, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lt::smem(NST));
-    dim3 grid(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
-    k_conv3x3_tc<BN, NM, NST><<<grid, TTHREADS, Lt::smem(NST), s>>>(a, ntx, nty, ntiles, vec);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
+    cfg.blockDim = dim3(TTHREADS);
+    cfg.dynamicSmemBytes = Lt::smem(NST);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_conv3x3_tc<BN, NM, NST>, a, xm, wm, ntx, nty, ntiles, vec);
+    return true;
 }
 
 int64_t tc_tiles(const ConvArgs &a) { return (int64_t)a.B * ((a.W + TTW - 1) / TTW) * ((a.H + TTH - 1) / TTH); }
 
-// Tiles and channels per block and stages of the ring: where Cin = 32 is one
-// chunk, one stage, and two tiles share the weights if there are tiles enough
-// for every SM; otherwise two stages, so that two blocks share an SM (four
-// stages, one block an SM: 47 us for 256 channels at 16 x 16, batch 16, against
-// 30 us), and 32 channels a block where 64 would leave SMs idle.
-void conv_tc(const ConvArgs &a, cudaStream_t s)
+// Channels and tiles per block and stages of the ring.  An MMA of 128 pixels takes
+// some 100 cycles for 32 or 64 channels alike, so 64 channels a block where that
+// gives a block to every SM; 32 where it does not.  Where more blocks than fit
+// at once keep coming, one stage and many small blocks overlap one another
+// (us, one stage / two / two tiles and two stages: 64 -> 64 at 64 x 64, batch 16,
+// 23.4 / 26.9 / 27.0; 96 -> 32 at 128 x 128 with two tiles 46, one tile and two
+// stages 69); a grid of one wave needs its stages (128 -> 128 at 32 x 32: 34 / 20.7
+// / 18.5), the more the fewer blocks share an SM (256 -> 128 at 16 x 16, 32
+// channels: two 27, four 14; 256 -> 256: three 22, two 31, four 27).
+bool conv_tc(const ConvArgs &a, cudaStream_t s)
 {
     const int64_t tiles = tc_tiles(a);
     const auto ok32 = [](const void *p) { return ((uintptr_t)p & 31u) == 0; };
     const int vec = !a.acc && (!a.of || ((a.os | a.oo) % 8 == 0 && ok32(a.of))) &&
                     (!a.oa || ((a.as | a.ao) % 16 == 0 && ok32(a.oa)));
-    const bool few = tiles * ((a.Cout + 63) / 64) < 148;
-    if (a.Cin == TBK) {
+    const int64_t n64 = tiles * ((a.Cout + 63) / 64), n32 = tiles * ((a.Cout + 31) / 32);
+    const bool wide = a.Cout > 32 && n64 >= 148;
+    if (a.Cin == TBK) {  // one chunk: two tiles share the weights if there are tiles enough for every SM
         const bool two = tiles >= 592;
-        if (a.Cout <= 32 || few)
-            two ? launch_conv_tc<32, 2, 1>(a, vec, s) : launch_conv_tc<32, 1, 1>(a, vec, s);
-        else
-            two ? launch_conv_tc<64, 2, 1>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
-    } else if (a.Cout <= 32 || few) {
-        launch_conv_tc<32, 1, 2>(a, vec, s);
-    } else {
-        launch_conv_tc<64, 1, 2>(a, vec, s);
+        if (!wide) return two ? launch_conv_tc<32, 2, 1>(a, vec, s) : launch_conv_tc<32, 1, 1>(a, vec, s);
+        return two ? launch_conv_tc<64, 2, 1>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
     }
+    if (wide) return n64 <= 296 ? launch_conv_tc<64, 2, 2>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
+    if (n32 <= 148) return launch_conv_tc<32, 1, 4>(a, vec, s);
+    return n32 <= 296 ? launch_conv_tc<32, 1, 3>(a, vec, s) : launch_conv_tc<32, 2, 1>(a, vec, s);
 }
 
 int g_path = 0;            // lbm_nn_set_tensor_path: 0 the faster kernel for the tensors at hand, 1 tcgen05
@@ -1284,13 +1331,14 @@ extern "C" int lbm_nn_conv3x3(const void *x, int64_t xs, int32_t xo, const void 
                (bf16 *)oa, as, ao, act};
     const int64_t M = (int64_t)B * H * W;
     cudaStream_t s = (cudaStream_t)stream;
-    // The tcgen05 kernel is the faster on the network's layers (batch 16: 31 us against 59 for 32 -> 32 channels at
-    // 128 x 128, 29 against 55 for 256 -> 256 at 16 x 16) and on any call of few blocks.  mma.sync takes pixels in a
-    // row, across images, and wins where more than two blocks an SM would mostly hold padding (256 images of 9 x 9,
-    // 64 channels: 27 us against 33; of 2 x 2, 256 channels: 53 against 135; a tile half full: 33 against 17).
+    // The tcgen05 kernel is the faster on the network's layers (batch 16: 30 us against 59 for 32 -> 32 channels at
+    // 128 x 128, 22 against 55 for 256 -> 256 at 16 x 16) and on any call of few blocks.  mma.sync takes pixels in a
+    // row, across images, and wins where more than two blocks an SM would mostly hold padding (256 images of 17 x 3,
+    // 64 channels: 21 us against 30; of 2 x 2, 256 channels: 53 against 100; of 8 x 4, 128: 33 both; a third full, 9 x 9,
+    // 64: 27 against 21).
     const int64_t tiles = tc_tiles(a);
-    if (g_path == 1 || 8 * M >= 3 * tiles * TTW * TTH || tiles * ((Cout + 63) / 64) <= 296) {
-        conv_tc(a, s);
+    if (g_path == 1 || 4 * M >= tiles * TTW * TTH || tiles * ((Cout + 63) / 64) <= 296) {
+        if (!conv_tc(a, s)) return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_conv3x3: no tensor maps on this device");
         return launched("lbm_nn_conv3x3 (tcgen05)");
     }
     if (Cout <= 32) {
