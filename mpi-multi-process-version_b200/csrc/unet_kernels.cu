@@ -35,6 +35,32 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kThreads = 256;
 
+// Every kernel here is launched as a programmatic dependent of the one before: its
+// blocks may be set up while that one still runs, and it reads and writes only
+// after dep_sync.  118 launches a training step (batch 16, 128 x 128): 1.86 ms as ordinary
+// launches, 1.73 so.
+__device__ __forceinline__ void dep_sync()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+void go(void (*k)(KArgs...), dim3 grid, unsigned block, int smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int bytes)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -93,6 +119,7 @@ struct ConvArgs {
 template <int BN>
 __global__ void __launch_bounds__(kThreads) k_conv3x3(const ConvArgs a)
 {
+    dep_sync();
     __shared__ __align__(16) bf16 As[2][CBM * CLD];
     __shared__ __align__(16) bf16 Bs[2][BN * CLD];
     constexpr int NT = BN / 16;  // n8 tiles per warp
@@ -212,6 +239,7 @@ __global__ void __launch_bounds__(kThreads) k_conv3x3(const ConvArgs a)
 
 __global__ void k_flip(const bf16 *__restrict__ w, bf16 *__restrict__ wt, int Cout, int Cin)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t n = (int64_t)Cout * 9 * Cin;
     if (i >= n) return;
@@ -265,6 +293,7 @@ __global__ void __launch_bounds__(BM * 4, BM == 64 ? 2 : 4)
 k_wgrad(const bf16 *__restrict__ dz, const bf16 *__restrict__ x, int64_t xs, int xo, int B, int H, int W, int Cin,
         int Cout, int ntx, int nty, int per, float *__restrict__ ws)
 {
+    dep_sync();
     using L = WgLayout<BM>;
     extern __shared__ __align__(16) unsigned char wg_sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -367,6 +396,7 @@ constexpr int kSumThreads = 1024;
 __global__ void __launch_bounds__(kSumThreads) k_sum_splits(const float *__restrict__ ws, int S, int64_t n,
                                                          float *__restrict__ out)
 {
+    dep_sync();
     __shared__ float sh[kSumThreads / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * 32 + lane;
@@ -396,6 +426,7 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_splits(const float *__restr
 __global__ void __launch_bounds__(kThreads) k_sum_few(const float *__restrict__ ws, int S, int64_t n,
                                                       float *__restrict__ out)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     const float *q = ws + i;
@@ -417,9 +448,9 @@ __global__ void __launch_bounds__(kThreads) k_sum_few(const float *__restrict__ 
 void sum_splits(const float *ws, int S, int64_t n, float *out, cudaStream_t s)
 {
     if (S <= 64)
-        k_sum_few<<<unsigned((n + kThreads - 1) / kThreads), kThreads, 0, s>>>(ws, S, n, out);
+        go(k_sum_few, unsigned((n + kThreads - 1) / kThreads), kThreads, 0, s, ws, S, n, out);
     else
-        k_sum_splits<<<unsigned((n + 31) / 32), kSumThreads, 0, s>>>(ws, S, n, out);
+        go(k_sum_splits, unsigned((n + 31) / 32), kSumThreads, 0, s, ws, S, n, out);
 }
 
 struct WgradPlan {
@@ -522,6 +553,7 @@ __device__ __forceinline__ void col_block(int64_t P, int C, float *__restrict__ 
 __global__ void __launch_bounds__(kThreads) k_colsum8(const bf16 *__restrict__ a, int64_t P, int C,
                                                       float *__restrict__ ws)
 {
+    dep_sync();
     col_block(P, C, ws, [&](int64_t p, int c, float (&v)[8]) { unpack8(*(const uint4 *)(a + p * C + c), v); });
 }
 
@@ -530,6 +562,7 @@ __global__ void __launch_bounds__(kThreads) k_silu_bwd8(const float *__restrict_
                                                         const float *__restrict__ z, int64_t P, int C,
                                                         bf16 *__restrict__ dz, float *__restrict__ ws)
 {
+    dep_sync();
     col_block(P, C, ws, [&](int64_t p, int c, float (&v)[8]) {
         const float4 *d = (const float4 *)(da + p * das + dao + c), *y = (const float4 *)(z + p * C + c);
         const float4 d0 = d[0], d1 = d[1], y0 = y[0], y1 = y[1];
@@ -547,6 +580,7 @@ __global__ void __launch_bounds__(kThreads) k_silu_bwd8(const float *__restrict_
 __global__ void __launch_bounds__(kThreads) k_colsum(const bf16 *__restrict__ a, int64_t P, int C,
                                                      float *__restrict__ ws)
 {
+    dep_sync();
     const int64_t nr = col_rows(P), beg = (int64_t)blockIdx.x * nr;
     const int64_t end = beg + nr < P ? beg + nr : P;
     for (int c = threadIdx.x; c < C; c += kThreads) {
@@ -559,6 +593,7 @@ __global__ void __launch_bounds__(kThreads) k_colsum(const bf16 *__restrict__ a,
 __global__ void k_silu_bwd(const float *__restrict__ da, int64_t das, int dao, const float *__restrict__ z, int64_t P,
                            int C, bf16 *__restrict__ dz)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P * C) return;
     const int64_t p = i / C;
@@ -597,6 +632,7 @@ __device__ __forceinline__ Pix pix_of(int B, int h, int w, int C)
 __global__ void __launch_bounds__(kThreads) k_pool2_v(const bf16 *__restrict__ x, int64_t xs, int xo, int B, int H,
                                                       int W, int C, bf16 *__restrict__ y, int64_t ys, int yo)
 {
+    dep_sync();
     const int h = H / 2, w = W / 2;
     const Pix p = pix_of<8>(B, h, w, C);
     if (!p.in) return;
@@ -614,6 +650,7 @@ __global__ void __launch_bounds__(kThreads) k_pool2_v(const bf16 *__restrict__ x
 __global__ void __launch_bounds__(kThreads) k_up2_v(const bf16 *__restrict__ x, int64_t xs, int xo, int B, int h,
                                                     int w, int C, bf16 *__restrict__ y, int64_t ys, int yo)
 {
+    dep_sync();
     const Pix p = pix_of<8>(B, h, w, C);
     if (!p.in) return;
     const uint4 v = *(const uint4 *)(x + ((int64_t)(p.b * h + p.y) * w + p.x) * xs + xo + p.c);
@@ -628,6 +665,7 @@ __global__ void __launch_bounds__(kThreads) k_pool2_bwd_v(const float *__restric
                                                           int H, int W, int C, float *__restrict__ dx, int64_t dxs,
                                                           int dxo)
 {
+    dep_sync();
     const int h = H / 2, w = W / 2;
     const Pix p = pix_of<4>(B, h, w, C);
     if (!p.in) return;
@@ -646,6 +684,7 @@ __global__ void __launch_bounds__(kThreads) k_up2_bwd_v(const float *__restrict_
                                                         int h, int w, int C, float *__restrict__ dx, int64_t dxs,
                                                         int dxo, int accumulate)
 {
+    dep_sync();
     const Pix p = pix_of<4>(B, h, w, C);
     if (!p.in) return;
     const float *s = dy + ((int64_t)(p.b * 2 * h + 2 * p.y) * 2 * w + 2 * p.x) * dys + dyo + p.c;
@@ -664,6 +703,7 @@ __global__ void __launch_bounds__(kThreads) k_up2_bwd_v(const float *__restrict_
 __global__ void k_pool2(const bf16 *__restrict__ x, int64_t xs, int xo, int B, int H, int W, int C,
                         bf16 *__restrict__ y, int64_t ys, int yo)
 {
+    dep_sync();
     const int h = H / 2, w = W / 2;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)B * h * w * C) return;
@@ -678,6 +718,7 @@ __global__ void k_pool2(const bf16 *__restrict__ x, int64_t xs, int xo, int B, i
 __global__ void k_pool2_bwd(const float *__restrict__ dy, int64_t dys, int dyo, int B, int H, int W, int C,
                             float *__restrict__ dx, int64_t dxs, int dxo)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)B * H * W * C) return;
     const int c = int(i % C);
@@ -690,6 +731,7 @@ __global__ void k_pool2_bwd(const float *__restrict__ dy, int64_t dys, int dyo, 
 __global__ void k_up2(const bf16 *__restrict__ x, int64_t xs, int xo, int B, int h, int w, int C,
                       bf16 *__restrict__ y, int64_t ys, int yo)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int H = 2 * h, W = 2 * w;
     if (i >= (int64_t)B * H * W * C) return;
@@ -702,6 +744,7 @@ __global__ void k_up2(const bf16 *__restrict__ x, int64_t xs, int xo, int B, int
 __global__ void k_up2_bwd(const float *__restrict__ dy, int64_t dys, int dyo, int B, int h, int w, int C,
                           float *__restrict__ dx, int64_t dxs, int dxo, int accumulate)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (int64_t)B * h * w * C) return;
     const int c = int(i % C);
@@ -719,6 +762,7 @@ constexpr int kMaxJ = 8;
 __global__ void k_head(const bf16 *__restrict__ a, int64_t as, int ao, const bf16 *__restrict__ wh,
                        const float *__restrict__ bh, int64_t P, int C, int J, float *__restrict__ y)
 {
+    dep_sync();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     float acc[kMaxJ];
@@ -733,6 +777,7 @@ __global__ void k_head(const bf16 *__restrict__ a, int64_t as, int ao, const bf1
 __global__ void k_head_bwd_da(const float *__restrict__ dy, const bf16 *__restrict__ wh, int64_t P, int C, int J,
                               float *__restrict__ da, int64_t das, int dao)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P * C) return;
     const int64_t p = i / C;
@@ -747,6 +792,7 @@ __global__ void __launch_bounds__(kThreads) k_head3_v(const bf16 *__restrict__ a
                                                       const bf16 *__restrict__ wh, const float *__restrict__ bh,
                                                       int64_t P, int C, float *__restrict__ y)
 {
+    dep_sync();
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     float acc[3];
@@ -766,6 +812,7 @@ __global__ void __launch_bounds__(kThreads) k_head3_bwd_da_v(const float *__rest
                                                              int64_t P, int C, float *__restrict__ da, int64_t das,
                                                              int dao)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int C4 = C / 4;
     if (i >= P * C4) return;
@@ -788,6 +835,7 @@ __global__ void __launch_bounds__(kThreads) k_head_bwd_w(const float *__restrict
                                                          int64_t as, int ao, int64_t P, int C, int J,
                                                          float *__restrict__ ws)
 {
+    dep_sync();
     __shared__ float sh[kThreads / 32][kMaxJ][33];
     const int lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
     const int items = J * C + J;
@@ -825,6 +873,7 @@ __global__ void __launch_bounds__(kThreads) k_head3_bwd_w_v(const float *__restr
                                                             int64_t as, int ao, int64_t P, int C,
                                                             float *__restrict__ ws)
 {
+    dep_sync();
     __shared__ float sh[kThreads * 8], shd[kThreads];
     const int C8 = C / 8, RL = kThreads / C8, rl = threadIdx.x / C8, g = threadIdx.x % C8;
     const int64_t beg = (int64_t)blockIdx.x * kHeadRows;
@@ -873,6 +922,7 @@ constexpr int kMseBlocks = 296;
 __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ cw, int64_t P,
                       int J, float *__restrict__ dy, float *__restrict__ ws)
 {
+    dep_sync();
     __shared__ float sh[kThreads / 32];
     const int64_t n = P * J;
     const float inv = 1.0f / float(n);
@@ -896,6 +946,7 @@ __global__ void k_mse(const float *__restrict__ y, const float *__restrict__ t, 
 
 __global__ void k_mse_final(const float *__restrict__ ws, int nb, int64_t n, float *__restrict__ loss)
 {
+    dep_sync();
     float s = 0.0f;  // one warp: lane l takes every 32nd block's sum, then a fixed tree
     for (int k = threadIdx.x; k < nb; k += 32) s += ws[k];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -906,6 +957,7 @@ __global__ void k_adam(float *__restrict__ p, bf16 *__restrict__ pb, const float
                        float *__restrict__ v, int64_t n, float lr, float b1, float b2, float eps, float c1, float c2,
                        float wd)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float gi = g[i];
@@ -920,6 +972,7 @@ __global__ void k_adam(float *__restrict__ p, bf16 *__restrict__ pb, const float
 
 __global__ void k_to_bf16(const float *__restrict__ x, bf16 *__restrict__ y, int64_t n)
 {
+    dep_sync();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) y[i] = __float2bfloat16_rn(x[i]);
 }
@@ -1261,17 +1314,8 @@ bool launch_conv_tc(const ConvArgs &a, int vec, cudaStream_t s)
     if (!conv_maps(a, BN, &xm, &wm)) return false;
     const int ntx = (a.W + TTW - 1) / TTW, nty = (a.H + TTH - 1) / TTH, ntiles = a.B * ntx * nty;
     cudaFuncSetAttribute(k_conv3x3_tc<BN, NM, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lt::smem(NST));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
-    cfg.blockDim = dim3(TTHREADS);
-    cfg.dynamicSmemBytes = Lt::smem(NST);
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_conv3x3_tc<BN, NM, NST>, a, xm, wm, ntx, nty, ntiles, vec);
+    const dim3 grid(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
+    go(k_conv3x3_tc<BN, NM, NST>, grid, TTHREADS, Lt::smem(NST), s, a, xm, wm, ntx, nty, ntiles, vec);
     return true;
 }
 
@@ -1343,10 +1387,10 @@ extern "C" int lbm_nn_conv3x3(const void *x, int64_t xs, int32_t xo, const void 
     }
     if (Cout <= 32) {
         dim3 grid(unsigned((M + CBM - 1) / CBM), unsigned((Cout + 31) / 32));
-        k_conv3x3<32><<<grid, kThreads, 0, s>>>(a);
+        go(k_conv3x3<32>, grid, kThreads, 0, s, a);
     } else {
         dim3 grid(unsigned((M + CBM - 1) / CBM), unsigned((Cout + 63) / 64));
-        k_conv3x3<64><<<grid, kThreads, 0, s>>>(a);
+        go(k_conv3x3<64>, grid, kThreads, 0, s, a);
     }
     return launched("lbm_nn_conv3x3");
 }
@@ -1355,7 +1399,7 @@ extern "C" int lbm_nn_flip_weights(const void *w, void *wt, int32_t Cout, int32_
 {
     NN_REQUIRE(w && wt && Cout > 0 && Cin > 0, "lbm_nn_flip_weights: bad arguments");
     const int64_t n = (int64_t)Cout * 9 * Cin;
-    k_flip<<<blocks_for(n), kThreads, 0, (cudaStream_t)stream>>>((const bf16 *)w, (bf16 *)wt, Cout, Cin);
+    go(k_flip, blocks_for(n), kThreads, 0, (cudaStream_t)stream, (const bf16 *)w, (bf16 *)wt, Cout, Cin);
     return launched("lbm_nn_flip_weights");
 }
 
@@ -1385,11 +1429,11 @@ extern "C" int lbm_nn_conv3x3_wgrad(const void *dz, const void *x, int64_t xs, i
     dim3 grid(unsigned(Cin / WBN), unsigned((Cout + pl.BM - 1) / pl.BM), unsigned(pl.S));
     if (pl.BM == 64) {
         cudaFuncSetAttribute(k_wgrad<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, WgLayout<64>::SMEM);
-        k_wgrad<64><<<grid, WgLayout<64>::threads, WgLayout<64>::SMEM, s>>>(
+        go(k_wgrad<64>, grid, WgLayout<64>::threads, WgLayout<64>::SMEM, s,
             (const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl.ntx, pl.nty, pl.per, part);
     } else {
         cudaFuncSetAttribute(k_wgrad<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, WgLayout<32>::SMEM);
-        k_wgrad<32><<<grid, WgLayout<32>::threads, WgLayout<32>::SMEM, s>>>(
+        go(k_wgrad<32>, grid, WgLayout<32>::threads, WgLayout<32>::SMEM, s,
             (const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl.ntx, pl.nty, pl.per, part);
     }
     if (pl.S > 1) sum_splits(ws, pl.S, n, dw, s);
@@ -1411,9 +1455,9 @@ extern "C" int lbm_nn_colsum(const void *a, int64_t P, int32_t C, float *ws, flo
     const int64_t S = (P + col_rows(P) - 1) / col_rows(P);
     cudaStream_t s = (cudaStream_t)stream;
     if (C % 8 == 0 && aligned16(a))
-        k_colsum8<<<unsigned(S), kThreads, 0, s>>>((const bf16 *)a, P, C, ws);
+        go(k_colsum8, unsigned(S), kThreads, 0, s, (const bf16 *)a, P, C, ws);
     else
-        k_colsum<<<unsigned(S), kThreads, 0, s>>>((const bf16 *)a, P, C, ws);
+        go(k_colsum, unsigned(S), kThreads, 0, s, (const bf16 *)a, P, C, ws);
     sum_splits(ws, int(S), C, out, s);
     return launched("lbm_nn_colsum", 2);
 }
@@ -1429,10 +1473,10 @@ extern "C" int lbm_nn_silu_backward(const float *da, int64_t das, int32_t dao, c
     NN_REQUIRE(da && z && dz && P > 0 && C > 0 && dao >= 0 && dao + C <= das, "lbm_nn_silu_backward: bad arguments");
     cudaStream_t s = (cudaStream_t)stream;
     if (silu_vec(da, das, dao, z, C, dz))
-        k_silu_bwd8<<<unsigned((P + col_rows(P) - 1) / col_rows(P)), kThreads, 0, s>>>(da, das, dao, z, P, C, (bf16 *)dz,
+        go(k_silu_bwd8, unsigned((P + col_rows(P) - 1) / col_rows(P)), kThreads, 0, s, da, das, dao, z, P, C, (bf16 *)dz,
                                                                                  nullptr);
     else
-        k_silu_bwd<<<blocks_for(P * C), kThreads, 0, s>>>(da, das, dao, z, P, C, (bf16 *)dz);
+        go(k_silu_bwd, blocks_for(P * C), kThreads, 0, s, da, das, dao, z, P, C, (bf16 *)dz);
     return launched("lbm_nn_silu_backward");
 }
 
@@ -1447,7 +1491,7 @@ extern "C" int lbm_nn_silu_backward_bias(const float *da, int64_t das, int32_t d
     }
     const int64_t S = (P + col_rows(P) - 1) / col_rows(P);
     cudaStream_t s = (cudaStream_t)stream;
-    k_silu_bwd8<<<unsigned(S), kThreads, 0, s>>>(da, das, dao, z, P, C, (bf16 *)dz, ws);
+    go(k_silu_bwd8, unsigned(S), kThreads, 0, s, da, das, dao, z, P, C, (bf16 *)dz, ws);
     sum_splits(ws, int(S), C, db, s);
     return launched("lbm_nn_silu_backward_bias", 2);
 }
@@ -1461,9 +1505,9 @@ extern "C" int lbm_nn_pool2(const void *x, int64_t xs, int32_t xo, int32_t B, in
     const int64_t n = (int64_t)B * (H / 2) * (W / 2) * C;
     cudaStream_t s = (cudaStream_t)stream;
     if ((C | xs | xo | ys | yo) % 8 == 0 && aligned16(x) && aligned16(y) && small(n / 8))
-        k_pool2_v<<<blocks_for(n / 8), kThreads, 0, s>>>((const bf16 *)x, xs, xo, B, H, W, C, (bf16 *)y, ys, yo);
+        go(k_pool2_v, blocks_for(n / 8), kThreads, 0, s, (const bf16 *)x, xs, xo, B, H, W, C, (bf16 *)y, ys, yo);
     else
-        k_pool2<<<blocks_for(n), kThreads, 0, s>>>((const bf16 *)x, xs, xo, B, H, W, C, (bf16 *)y, ys, yo);
+        go(k_pool2, blocks_for(n), kThreads, 0, s, (const bf16 *)x, xs, xo, B, H, W, C, (bf16 *)y, ys, yo);
     return launched("lbm_nn_pool2");
 }
 
@@ -1476,9 +1520,9 @@ extern "C" int lbm_nn_pool2_backward(const float *dy, int64_t dys, int32_t dyo, 
     const int64_t n = (int64_t)B * H * W * C;
     cudaStream_t s = (cudaStream_t)stream;
     if ((C | dys | dyo | dxs | dxo) % 4 == 0 && aligned16(dy) && aligned16(dx) && small(n / 16))
-        k_pool2_bwd_v<<<blocks_for(n / 16), kThreads, 0, s>>>(dy, dys, dyo, B, H, W, C, dx, dxs, dxo);
+        go(k_pool2_bwd_v, blocks_for(n / 16), kThreads, 0, s, dy, dys, dyo, B, H, W, C, dx, dxs, dxo);
     else
-        k_pool2_bwd<<<blocks_for(n), kThreads, 0, s>>>(dy, dys, dyo, B, H, W, C, dx, dxs, dxo);
+        go(k_pool2_bwd, blocks_for(n), kThreads, 0, s, dy, dys, dyo, B, H, W, C, dx, dxs, dxo);
     return launched("lbm_nn_pool2_backward");
 }
 
@@ -1490,9 +1534,9 @@ extern "C" int lbm_nn_up2(const void *x, int64_t xs, int32_t xo, int32_t B, int3
     const int64_t n = (int64_t)B * 4 * h * w * C;
     cudaStream_t s = (cudaStream_t)stream;
     if ((C | xs | xo | ys | yo) % 8 == 0 && aligned16(x) && aligned16(y) && small(n / 32))
-        k_up2_v<<<blocks_for(n / 32), kThreads, 0, s>>>((const bf16 *)x, xs, xo, B, h, w, C, (bf16 *)y, ys, yo);
+        go(k_up2_v, blocks_for(n / 32), kThreads, 0, s, (const bf16 *)x, xs, xo, B, h, w, C, (bf16 *)y, ys, yo);
     else
-        k_up2<<<blocks_for(n), kThreads, 0, s>>>((const bf16 *)x, xs, xo, B, h, w, C, (bf16 *)y, ys, yo);
+        go(k_up2, blocks_for(n), kThreads, 0, s, (const bf16 *)x, xs, xo, B, h, w, C, (bf16 *)y, ys, yo);
     return launched("lbm_nn_up2");
 }
 
@@ -1504,9 +1548,9 @@ extern "C" int lbm_nn_up2_backward(const float *dy, int64_t dys, int32_t dyo, in
     const int64_t n = (int64_t)B * h * w * C;
     cudaStream_t s = (cudaStream_t)stream;
     if ((C | dys | dyo | dxs | dxo) % 4 == 0 && aligned16(dy) && aligned16(dx) && small(n / 4))
-        k_up2_bwd_v<<<blocks_for(n / 4), kThreads, 0, s>>>(dy, dys, dyo, B, h, w, C, dx, dxs, dxo, accumulate);
+        go(k_up2_bwd_v, blocks_for(n / 4), kThreads, 0, s, dy, dys, dyo, B, h, w, C, dx, dxs, dxo, accumulate);
     else
-        k_up2_bwd<<<blocks_for(n), kThreads, 0, s>>>(dy, dys, dyo, B, h, w, C, dx, dxs, dxo, accumulate);
+        go(k_up2_bwd, blocks_for(n), kThreads, 0, s, dy, dys, dyo, B, h, w, C, dx, dxs, dxo, accumulate);
     return launched("lbm_nn_up2_backward");
 }
 
@@ -1517,9 +1561,9 @@ extern "C" int lbm_nn_head(const void *a, int64_t as, int32_t ao, const void *wh
     NN_REQUIRE(ao >= 0 && ao + C <= as, "lbm_nn_head: bad channel stride/offset");
     cudaStream_t s = (cudaStream_t)stream;
     if (J == 3 && (C | as | ao) % 8 == 0 && aligned16(a))
-        k_head3_v<<<blocks_for(P), kThreads, 0, s>>>((const bf16 *)a, as, ao, (const bf16 *)wh, bh, P, C, y);
+        go(k_head3_v, blocks_for(P), kThreads, 0, s, (const bf16 *)a, as, ao, (const bf16 *)wh, bh, P, C, y);
     else
-        k_head<<<blocks_for(P), kThreads, 0, s>>>((const bf16 *)a, as, ao, (const bf16 *)wh, bh, P, C, J, y);
+        go(k_head, blocks_for(P), kThreads, 0, s, (const bf16 *)a, as, ao, (const bf16 *)wh, bh, P, C, J, y);
     return launched("lbm_nn_head");
 }
 
@@ -1542,13 +1586,13 @@ extern "C" int lbm_nn_head_backward(const float *dy, const void *a, int64_t as, 
     NN_REQUIRE(ws_elems >= (S + 1) * items, "lbm_nn_head_backward: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
     if (J == 3 && (C | das | dao) % 4 == 0 && aligned16(da))
-        k_head3_bwd_da_v<<<blocks_for(P * C / 4), kThreads, 0, s>>>(dy, (const bf16 *)wh, P, C, da, das, dao);
+        go(k_head3_bwd_da_v, blocks_for(P * C / 4), kThreads, 0, s, dy, (const bf16 *)wh, P, C, da, das, dao);
     else
-        k_head_bwd_da<<<blocks_for(P * C), kThreads, 0, s>>>(dy, (const bf16 *)wh, P, C, J, da, das, dao);
+        go(k_head_bwd_da, blocks_for(P * C), kThreads, 0, s, dy, (const bf16 *)wh, P, C, J, da, das, dao);
     if (J == 3 && (C | as | ao) % 8 == 0 && C <= 256 && aligned16(a))
-        k_head3_bwd_w_v<<<unsigned(S), kThreads, 0, s>>>(dy, (const bf16 *)a, as, ao, P, C, ws);
+        go(k_head3_bwd_w_v, unsigned(S), kThreads, 0, s, dy, (const bf16 *)a, as, ao, P, C, ws);
     else
-        k_head_bwd_w<<<unsigned(S), kThreads, 0, s>>>(dy, (const bf16 *)a, as, ao, P, C, J, ws);
+        go(k_head_bwd_w, unsigned(S), kThreads, 0, s, dy, (const bf16 *)a, as, ao, P, C, J, ws);
     // each split's partials hold dwh (J*C) then dbh (J); their ordered sums go after them
     sum_splits(ws, int(S), items, ws + S * items, s);
     int st = launched("lbm_nn_head_backward", 3);
@@ -1573,8 +1617,8 @@ extern "C" int lbm_nn_mse(const float *y, const float *t, const float *cw, int64
     NN_REQUIRE(y && t && dy && ws && loss && P > 0 && J > 0, "lbm_nn_mse: bad arguments");
     NN_REQUIRE(ws_elems >= kMseBlocks, "lbm_nn_mse: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
-    k_mse<<<kMseBlocks, kThreads, 0, s>>>(y, t, cw, P, J, dy, ws);
-    k_mse_final<<<1, 32, 0, s>>>(ws, kMseBlocks, P * J, loss);
+    go(k_mse, kMseBlocks, kThreads, 0, s, y, t, cw, P, J, dy, ws);
+    go(k_mse_final, 1, 32, 0, s, ws, kMseBlocks, P * J, loss);
     return launched("lbm_nn_mse", 2);
 }
 
@@ -1583,14 +1627,14 @@ extern "C" int lbm_nn_adam(float *p, void *pb, const float *g, float *m, float *
 {
     NN_REQUIRE(p && g && m && v && n > 0, "lbm_nn_adam: bad arguments");
     NN_REQUIRE(c1 > 0.0f && c2 > 0.0f, "lbm_nn_adam: bias corrections must be > 0");
-    k_adam<<<blocks_for(n), kThreads, 0, (cudaStream_t)stream>>>(p, (bf16 *)pb, g, m, v, n, lr, b1, b2, eps, c1, c2, wd);
+    go(k_adam, blocks_for(n), kThreads, 0, (cudaStream_t)stream, p, (bf16 *)pb, g, m, v, n, lr, b1, b2, eps, c1, c2, wd);
     return launched("lbm_nn_adam");
 }
 
 extern "C" int lbm_nn_to_bf16(const float *x, void *y, int64_t n, void *stream)
 {
     NN_REQUIRE(x && y && n > 0, "lbm_nn_to_bf16: bad arguments");
-    k_to_bf16<<<blocks_for(n), kThreads, 0, (cudaStream_t)stream>>>(x, (bf16 *)y, n);
+    go(k_to_bf16, blocks_for(n), kThreads, 0, (cudaStream_t)stream, x, (bf16 *)y, n);
     return launched("lbm_nn_to_bf16");
 }
 
