@@ -106,6 +106,40 @@ int lbm_nn_mse(const float *y, const float *t, const float *cw, int64_t P, int32
 int lbm_nn_adam(float *p, void *pb, const float *g, float *m, float *v, int64_t n, float lr, float b1,
                 float b2, float eps, float c1, float c2, float wd, void *stream);
 
+/* The 4-level U-Net as one call: its 3x3 layers in execution order are
+ *   0 e1a, 1 e1b, 2 e2a, 3 e2b, 4 e3a, 5 e3b, 6 ba, 7 bb, 8 d3a, 9 d3b, 10 d2a,
+ *   11 d2b, 12 d1a, 13 d1b;
+ * ch[l] holds layer l's input and output channels.  pb, wt (flipped, written by
+ * the backward pass), master and grad are flat parameter buffers; layer l's
+ * weights start at off[l][0] and its bias at off[l][1], the 1x1 output layer's
+ * (J outputs) at off[14].  Images: level 1 is R x R, level k R >> (k - 1).
+ *   x     the input, bf16;            p[k]  pooled level k + 1, bf16
+ *   cat[k] level k + 1's [upsampled | skip] buffer, bf16 (the skip half is the
+ *         output of e1b, e2b, e3b);   a[l], z[l]  layer l's activation (bf16;
+ *         not used for layers 1, 3, 5) and pre-activation (FP32)
+ *   y     the output, FP32 (B R R, J)
+ * and for the backward pass, from dy: FP32 da[l], dcat[k], dp[k], bf16 dz[l], and
+ * scratch ws, the largest of the single calls' workspaces. */
+typedef struct lbm_nn_unet {
+    int32_t B, R, J, reserved;
+    int32_t ch[14][2];
+    int64_t off[15][2];
+    const void *pb;
+    void *wt;
+    const float *master;
+    float *grad;
+    const void *x;
+    void *cat[3], *p[3], *a[14];
+    float *z[14], *y;
+    float *dy, *da[14], *dcat[3], *dp[3];
+    void *dz[14];
+    float *ws;
+    int64_t ws_elems;
+} lbm_nn_unet;
+int lbm_nn_unet_forward(const lbm_nn_unet *net, void *stream);
+/* gradients of sum(dy y) into grad, from the buffers the forward pass left */
+int lbm_nn_unet_backward(const lbm_nn_unet *net, void *stream);
+
 /* Which tensor-core path lbm_nn_conv3x3 uses: 0 (the default) the faster one for
  * the tensors at hand: tcgen05 with the accumulators in tensor memory, or
  * mma.sync (m16n8k16) for many images far smaller than its 8 x 16 pixel tiles;

@@ -1660,3 +1660,115 @@ extern "C" int lbm_nn_timeouts(int32_t *count, int32_t reset)
     *count = v;
     return LBM_OK;
 }
+
+// ---------------------------------------------------------------------------
+// the network's passes
+// ---------------------------------------------------------------------------
+// One call issues the pass's launches: from Python each launch is a foreign call
+// of some twenty arguments, 8 us, as much as the kernels take at batch 1.  One
+// prediction at 128 x 128: the host's share 175 -> 91 us, the pass 173 -> 156 us.
+#define NN_DO(call)                   \
+    do {                              \
+        const int st_ = (call);       \
+        if (st_ != LBM_OK) return st_; \
+    } while (0)
+
+namespace {
+
+// a layer's image size, and its input and output tensors
+struct UnetLayer {
+    const void *x;
+    int xs;
+    void *a;
+    int as, ao, H;
+};
+
+void unet_layers(const lbm_nn_unet &n, UnetLayer l[14])
+{
+    const int c1 = n.ch[0][1], c2 = n.ch[2][1], c3 = n.ch[4][1], c4 = n.ch[6][1], R = n.R;
+    const int k1 = c2 + c1, k2 = c3 + c2, k3 = c4 + c3;  // channels of the concat buffers
+    const UnetLayer t[14] = {
+        {n.x, n.ch[0][0], n.a[0], c1, 0, R},         {n.a[0], c1, n.cat[0], k1, c2, R},
+        {n.p[0], c1, n.a[2], c2, 0, R / 2},          {n.a[2], c2, n.cat[1], k2, c3, R / 2},
+        {n.p[1], c2, n.a[4], c3, 0, R / 4},          {n.a[4], c3, n.cat[2], k3, c4, R / 4},
+        {n.p[2], c3, n.a[6], c4, 0, R / 8},          {n.a[6], c4, n.a[7], c4, 0, R / 8},
+        {n.cat[2], k3, n.a[8], c3, 0, R / 4},        {n.a[8], c3, n.a[9], c3, 0, R / 4},
+        {n.cat[1], k2, n.a[10], c2, 0, R / 2},       {n.a[10], c2, n.a[11], c2, 0, R / 2},
+        {n.cat[0], k1, n.a[12], c1, 0, R},           {n.a[12], c1, n.a[13], c1, 0, R}};
+    for (int k = 0; k < 14; ++k) l[k] = t[k];
+}
+
+int unet_check(const lbm_nn_unet *n, const char *what)
+{
+    NN_REQUIRE(n && n->B > 0 && n->R >= 16 && n->R % 8 == 0 && n->J > 0, "%s: bad arguments", what);
+    NN_REQUIRE(n->pb && n->master, "%s: NULL parameters", what);
+    return LBM_OK;
+}
+
+const char *at16(const void *p, int64_t o) { return (const char *)p + 2 * o; }
+
+}  // namespace
+
+extern "C" int lbm_nn_unet_forward(const lbm_nn_unet *net, void *stream)
+{
+    NN_DO(unet_check(net, "lbm_nn_unet_forward"));
+    const lbm_nn_unet &n = *net;
+    const int B = n.B;
+    UnetLayer l[14];
+    unet_layers(n, l);
+    for (int k = 0; k < 14; ++k) {
+        const UnetLayer &t = l[k];
+        const int ci = n.ch[k][0], co = n.ch[k][1], H = t.H;
+        NN_DO(lbm_nn_conv3x3(t.x, t.xs, 0, at16(n.pb, n.off[k][0]), n.master + n.off[k][1], B, H, H, ci, co, n.z[k], co,
+                             0, 0, t.a, t.as, t.ao, 1, stream));
+        if (k == 1 || k == 3 || k == 5)  // the end of an encoder level
+            NN_DO(lbm_nn_pool2(t.a, t.as, t.ao, B, H, H, co, n.p[k / 2], co, 0, stream));
+        if (k == 7 || k == 9 || k == 11) {  // up into the next decoder level
+            const int d = (11 - k) / 2;
+            NN_DO(lbm_nn_up2(t.a, co, 0, B, H, H, co, n.cat[d], l[k + 1].xs, 0, stream));
+        }
+    }
+    return lbm_nn_head(n.a[13], l[13].as, 0, at16(n.pb, n.off[14][0]), n.master + n.off[14][1], (int64_t)B * n.R * n.R,
+                       l[13].as, n.J, n.y, stream);
+}
+
+extern "C" int lbm_nn_unet_backward(const lbm_nn_unet *net, void *stream)
+{
+    NN_DO(unet_check(net, "lbm_nn_unet_backward"));
+    const lbm_nn_unet &n = *net;
+    NN_REQUIRE(n.wt && n.grad && n.dy && n.ws, "lbm_nn_unet_backward: NULL pointer");
+    const int B = n.B;
+    UnetLayer l[14];
+    unet_layers(n, l);
+    for (int k = 0; k < 14; ++k)
+        NN_DO(lbm_nn_flip_weights(at16(n.pb, n.off[k][0]), (char *)n.wt + 2 * n.off[k][0], n.ch[k][1], n.ch[k][0],
+                                  stream));
+    NN_DO(lbm_nn_head_backward(n.dy, n.a[13], l[13].as, 0, at16(n.pb, n.off[14][0]), (int64_t)B * n.R * n.R, l[13].as,
+                               n.J, n.da[13], l[13].as, 0, n.ws, n.ws_elems, n.grad + n.off[14][0],
+                               n.grad + n.off[14][1], stream));
+    // where a layer's input gradient goes, per layer: its tensor and channel stride
+    float *const dx[14] = {nullptr, n.da[0], n.dp[0], n.da[2], n.dp[1], n.da[4], n.dp[2], n.da[6], n.dcat[2], n.da[8],
+                           n.dcat[1], n.da[10], n.dcat[0], n.da[12]};
+    for (int k = 13; k >= 0; --k) {
+        const UnetLayer &t = l[k];
+        const int ci = n.ch[k][0], co = n.ch[k][1], H = t.H;
+        const bool skip = k == 1 || k == 3 || k == 5;  // its output is the skip half of a concat buffer
+        const float *da = skip ? n.dcat[k / 2] : n.da[k];
+        NN_DO(lbm_nn_silu_backward_bias(da, t.as, t.ao, n.z[k], (int64_t)B * H * H, co, n.dz[k], n.ws,
+                                        n.grad + n.off[k][1], stream));
+        NN_DO(lbm_nn_conv3x3_wgrad(n.dz[k], t.x, t.xs, 0, B, H, H, ci, co, n.ws, n.ws_elems, n.grad + n.off[k][0],
+                                   stream));
+        if (dx[k])
+            NN_DO(lbm_nn_conv3x3(n.dz[k], co, 0, (char *)n.wt + 2 * n.off[k][0], nullptr, B, H, H, co, ci, dx[k], t.xs, 0,
+                                 0, nullptr, 0, 0, 0, stream));
+        if (k == 12 || k == 10 || k == 8) {  // the upsampled half of the concat buffer
+            const int up = n.ch[k - 1][1];
+            NN_DO(lbm_nn_up2_backward(dx[k], t.xs, 0, B, H / 2, H / 2, up, n.da[k - 1], up, 0, 0, stream));
+        }
+        if (k == 6 || k == 4 || k == 2) {  // through the pooling into the skip half
+            const int e = k / 2 - 1, c = n.ch[k - 1][1];
+            NN_DO(lbm_nn_pool2_backward(n.dp[e], c, 0, B, 2 * H, 2 * H, c, n.dcat[e], l[k - 1].as, l[k - 1].ao, stream));
+        }
+    }
+    return LBM_OK;
+}

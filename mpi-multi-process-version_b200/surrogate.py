@@ -56,6 +56,8 @@ _SIGS = {
     "lbm_nn_mse": [_dp, _dp, _dp, _i64, _i32, _dp, _dp, _i64, _dp, _dp],
     "lbm_nn_adam": [_dp, _dp, _dp, _dp, _dp, _i64, _f32, _f32, _f32, _f32, _f32, _f32, _f32, _dp],
     "lbm_nn_to_bf16": [_dp, _dp, _i64, _dp],
+    "lbm_nn_unet_forward": [_dp, _dp],
+    "lbm_nn_unet_backward": [_dp, _dp],
     "lbm_nn_set_tensor_path": [_i32],
     "lbm_nn_get_tensor_path": [],
     "lbm_nn_timeouts": [_dp, _i32],
@@ -112,6 +114,17 @@ def _align(n, a=64):
     return (n + a - 1) // a * a
 
 
+_v14, _v3 = _dp * 14, _dp * 3
+
+
+class _Unet(ctypes.Structure):
+    """lbm_nn_unet of include/lbm_surrogate.h."""
+    _fields_ = [("B", _i32), ("R", _i32), ("J", _i32), ("reserved", _i32), ("ch", _i32 * 28), ("off", _i64 * 30),
+                ("pb", _dp), ("wt", _dp), ("master", _dp), ("grad", _dp), ("x", _dp), ("cat", _v3), ("p", _v3),
+                ("a", _v14), ("z", _v14), ("y", _dp), ("dy", _dp), ("da", _v14), ("dcat", _v3), ("dp", _v3),
+                ("dz", _v14), ("ws", _dp), ("ws_elems", _i64)]
+
+
 class Net:
     """Parameters (flat FP32 master, bf16 copy, gradients, Adam moments) and
     per-batch-size activation buffers of the U-Net, on one CUDA device."""
@@ -130,6 +143,8 @@ class Net:
             off = _align(self.off[name][1] + co)
         self.off["head"] = (off, _align(off + OUT_CH * LEVELS[0]))
         self.n_params_padded = _align(self.off["head"][1] + OUT_CH)
+        self._ch = tuple(c for _, ci, co in self.table for c in (ci, co))
+        self._off = tuple(o for name in [n for n, _, _ in self.table] + ["head"] for o in self.off[name])
         f32 = dict(dtype=torch.float32, device=self.dev)
         self.master = torch.zeros(self.n_params_padded, **f32)
         self.grad = torch.zeros_like(self.master)
@@ -188,22 +203,8 @@ class Net:
         _chk(nn().lbm_nn_to_bf16(self.master.data_ptr(), self.pb.data_ptr(), self.n_params_padded, self._s()),
              "lbm_nn_to_bf16")
 
-    # -- pointers ---------------------------------------------------------
     def _s(self):
         return self.torch.cuda.current_stream(self.dev).cuda_stream
-
-    def _w(self, name, flipped=False):
-        t = self.wt if flipped else self.pb
-        return t.data_ptr() + 2 * self.off[name][0]
-
-    def _b(self, name):
-        return self.master.data_ptr() + 4 * self.off[name][1]
-
-    def _gw(self, name):
-        return self.grad.data_ptr() + 4 * self.off[name][0]
-
-    def _gb(self, name):
-        return self.grad.data_ptr() + 4 * self.off[name][1]
 
     # -- buffers ----------------------------------------------------------
     def buffers(self, B):
@@ -249,10 +250,22 @@ class Net:
         return b
 
     # -- kernels ----------------------------------------------------------
-    def _conv(self, B, name, x, xs, xo, of, os_, oo, acc, oa, as_, ao, act, bias, flipped, H, Cin, Cout):
-        st = nn().lbm_nn_conv3x3(x, xs, xo, self._w(name, flipped), self._b(name) if bias else None, B, H, H, Cin,
-                                 Cout, of, os_, oo, acc, oa, as_, ao, act, self._s())
-        _chk(st, f"conv {name}")
+    def _unet(self, b, B, backward):
+        """The passes' descriptor, of the tensors as they are now."""
+        p = lambda key: b[key].data_ptr()  # noqa: E731
+        names = [n for n, _, _ in self.table]
+        d = _Unet(B=B, R=self.R, J=OUT_CH, ch=self._ch, off=self._off, pb=self.pb.data_ptr(),
+                  master=self.master.data_ptr(), x=p("x"), cat=tuple(p(f"cat{k}") for k in (1, 2, 3)),
+                  p=tuple(p(f"p{k}") for k in (1, 2, 3)), a=tuple(p("a_" + n) for n in names),
+                  z=tuple(p("z_" + n) for n in names), y=p("y"))
+        if backward:
+            d.wt, d.grad, d.dy = self.wt.data_ptr(), self.grad.data_ptr(), p("dy")
+            d.da = tuple(p("da_" + n) for n in names)
+            d.dz = tuple(p("dz_" + n) for n in names)
+            d.dcat = tuple(p(f"dcat{k}") for k in (1, 2, 3))
+            d.dp = tuple(p(f"dp{k}") for k in (1, 2, 3))
+            d.ws, d.ws_elems = p("ws"), b["ws"].numel()
+        return d
 
     def forward(self, x=None, B=None):
         """Forward pass on buffers(B)['x'] (or copy x, a bf16 (B, R, R, 32)
@@ -261,53 +274,7 @@ class Net:
             B = x.shape[0]
             self.buffers(B)["x"].copy_(x)
         b = self.buffers(B)
-        R = self.R
-        c1, c2, c3, c4 = LEVELS
-        lib = nn()
-        s = self._s()
-        # (name, input ptr, stride, offset, output bf16 ptr, stride, offset)
-        plan = [
-            ("e1a", b["x"], IN_CH, 0, b["a_e1a"], c1, 0),
-            ("e1b", b["a_e1a"], c1, 0, b["cat1"], c2 + c1, c2),
-            ("e2a", b["p1"], c1, 0, b["a_e2a"], c2, 0),
-            ("e2b", b["a_e2a"], c2, 0, b["cat2"], c3 + c2, c3),
-            ("e3a", b["p2"], c2, 0, b["a_e3a"], c3, 0),
-            ("e3b", b["a_e3a"], c3, 0, b["cat3"], c4 + c3, c4),
-            ("ba", b["p3"], c3, 0, b["a_ba"], c4, 0),
-            ("bb", b["a_ba"], c4, 0, b["a_bb"], c4, 0),
-            ("d3a", b["cat3"], c4 + c3, 0, b["a_d3a"], c3, 0),
-            ("d3b", b["a_d3a"], c3, 0, b["a_d3b"], c3, 0),
-            ("d2a", b["cat2"], c3 + c2, 0, b["a_d2a"], c2, 0),
-            ("d2b", b["a_d2a"], c2, 0, b["a_d2b"], c2, 0),
-            ("d1a", b["cat1"], c2 + c1, 0, b["a_d1a"], c1, 0),
-            ("d1b", b["a_d1a"], c1, 0, b["a_d1b"], c1, 0),
-        ]
-        tab = {n: (ci, co) for n, ci, co in self.table}
-        for name, xin, xs, xo, oa, as_, ao in plan:
-            ci, co = tab[name]
-            H = b["res"][name]
-            self._conv(B, name, xin.data_ptr(), xs, xo, b["z_" + name].data_ptr(), co, 0, 0, oa.data_ptr(), as_, ao,
-                       1, True, False, H, ci, co)
-            if name == "e1b":
-                _chk(lib.lbm_nn_pool2(b["cat1"].data_ptr(), c2 + c1, c2, B, R, R, c1, b["p1"].data_ptr(), c1, 0, s), "pool")
-            elif name == "e2b":
-                _chk(lib.lbm_nn_pool2(b["cat2"].data_ptr(), c3 + c2, c3, B, R // 2, R // 2, c2, b["p2"].data_ptr(), c2, 0,
-                                      s), "pool")
-            elif name == "e3b":
-                _chk(lib.lbm_nn_pool2(b["cat3"].data_ptr(), c4 + c3, c4, B, R // 4, R // 4, c3, b["p3"].data_ptr(), c3, 0,
-                                      s), "pool")
-            elif name == "bb":
-                _chk(lib.lbm_nn_up2(b["a_bb"].data_ptr(), c4, 0, B, R // 8, R // 8, c4, b["cat3"].data_ptr(), c4 + c3, 0,
-                                    s), "up")
-            elif name == "d3b":
-                _chk(lib.lbm_nn_up2(b["a_d3b"].data_ptr(), c3, 0, B, R // 4, R // 4, c3, b["cat2"].data_ptr(), c3 + c2, 0,
-                                    s), "up")
-            elif name == "d2b":
-                _chk(lib.lbm_nn_up2(b["a_d2b"].data_ptr(), c2, 0, B, R // 2, R // 2, c2, b["cat1"].data_ptr(), c2 + c1, 0,
-                                    s), "up")
-        o, ob = self.off["head"]
-        _chk(lib.lbm_nn_head(b["a_d1b"].data_ptr(), c1, 0, self.pb.data_ptr() + 2 * o, self.master.data_ptr() + 4 * ob,
-                             B * R * R, c1, OUT_CH, b["y"].data_ptr(), s), "head")
+        _chk(nn().lbm_nn_unet_forward(ctypes.byref(self._unet(b, B, False)), self._s()), "forward")
         self.launches += 14 + 7
         return b["y"]
 
@@ -324,52 +291,7 @@ class Net:
     def backward(self, B):
         """Gradients of sum(dy * y) (dy in buffers(B)['dy']) into self.grad."""
         b = self.buffers(B)
-        R = self.R
-        c1, c2, c3, c4 = LEVELS
-        lib = nn()
-        s = self._s()
-        tab = {n: (ci, co) for n, ci, co in self.table}
-        for name, ci, co in self.table:
-            _chk(lib.lbm_nn_flip_weights(self._w(name), self._w(name, True), co, ci, s), "flip")
-        ws, wsn = b["ws"].data_ptr(), b["ws"].numel()
-        o, ob = self.off["head"]
-        _chk(lib.lbm_nn_head_backward(b["dy"].data_ptr(), b["a_d1b"].data_ptr(), c1, 0, self.pb.data_ptr() + 2 * o,
-                                      B * R * R, c1, OUT_CH, b["da_d1b"].data_ptr(), c1, 0, ws, wsn,
-                                      self.grad.data_ptr() + 4 * o, self.grad.data_ptr() + 4 * ob, s), "head backward")
-
-        def back(name, da_ptr, das, dao, x_ptr, xs, xo, dx_ptr=None, dxs=0, dxo=0, dx_acc=0):
-            ci, co = tab[name]
-            H = b["res"][name]
-            P = B * H * H
-            dz = b["dz_" + name]
-            _chk(lib.lbm_nn_silu_backward_bias(da_ptr, das, dao, b["z_" + name].data_ptr(), P, co, dz.data_ptr(), ws,
-                                               self._gb(name), s), f"silu backward {name}")
-            _chk(lib.lbm_nn_conv3x3_wgrad(dz.data_ptr(), x_ptr, xs, xo, B, H, H, ci, co, ws, wsn, self._gw(name), s),
-                 f"wgrad {name}")
-            if dx_ptr is not None:
-                self._conv(B, name, dz.data_ptr(), co, 0, dx_ptr, dxs, dxo, dx_acc, None, 0, 0, 0, False, True, H, co, ci)
-
-        p = lambda key: b[key].data_ptr()  # noqa: E731
-        back("d1b", p("da_d1b"), c1, 0, p("a_d1a"), c1, 0, p("da_d1a"), c1, 0)
-        back("d1a", p("da_d1a"), c1, 0, p("cat1"), c2 + c1, 0, p("dcat1"), c2 + c1, 0)
-        _chk(lib.lbm_nn_up2_backward(p("dcat1"), c2 + c1, 0, B, R // 2, R // 2, c2, p("da_d2b"), c2, 0, 0, s), "up bwd")
-        back("d2b", p("da_d2b"), c2, 0, p("a_d2a"), c2, 0, p("da_d2a"), c2, 0)
-        back("d2a", p("da_d2a"), c2, 0, p("cat2"), c3 + c2, 0, p("dcat2"), c3 + c2, 0)
-        _chk(lib.lbm_nn_up2_backward(p("dcat2"), c3 + c2, 0, B, R // 4, R // 4, c3, p("da_d3b"), c3, 0, 0, s), "up bwd")
-        back("d3b", p("da_d3b"), c3, 0, p("a_d3a"), c3, 0, p("da_d3a"), c3, 0)
-        back("d3a", p("da_d3a"), c3, 0, p("cat3"), c4 + c3, 0, p("dcat3"), c4 + c3, 0)
-        _chk(lib.lbm_nn_up2_backward(p("dcat3"), c4 + c3, 0, B, R // 8, R // 8, c4, p("da_bb"), c4, 0, 0, s), "up bwd")
-        back("bb", p("da_bb"), c4, 0, p("a_ba"), c4, 0, p("da_ba"), c4, 0)
-        back("ba", p("da_ba"), c4, 0, p("p3"), c3, 0, p("dp3"), c3, 0)
-        _chk(lib.lbm_nn_pool2_backward(p("dp3"), c3, 0, B, R // 4, R // 4, c3, p("dcat3"), c4 + c3, c4, s), "pool bwd")
-        back("e3b", p("dcat3"), c4 + c3, c4, p("a_e3a"), c3, 0, p("da_e3a"), c3, 0)
-        back("e3a", p("da_e3a"), c3, 0, p("p2"), c2, 0, p("dp2"), c2, 0)
-        _chk(lib.lbm_nn_pool2_backward(p("dp2"), c2, 0, B, R // 2, R // 2, c2, p("dcat2"), c3 + c2, c3, s), "pool bwd")
-        back("e2b", p("dcat2"), c3 + c2, c3, p("a_e2a"), c2, 0, p("da_e2a"), c2, 0)
-        back("e2a", p("da_e2a"), c2, 0, p("p1"), c1, 0, p("dp1"), c1, 0)
-        _chk(lib.lbm_nn_pool2_backward(p("dp1"), c1, 0, B, R, R, c1, p("dcat1"), c2 + c1, c2, s), "pool bwd")
-        back("e1b", p("dcat1"), c2 + c1, c2, p("a_e1a"), c1, 0, p("da_e1a"), c1, 0)
-        back("e1a", p("da_e1a"), c1, 0, p("x"), IN_CH, 0)
+        _chk(nn().lbm_nn_unet_backward(ctypes.byref(self._unet(b, B, True)), self._s()), "backward")
         self.launches += 14 + 3 + 13 * 5 + 4 + 3 + 3
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8, wd=0.0):

@@ -114,3 +114,51 @@ def test_silu_backward_with_bias_gradient(pkg, P, C, off):
     dz = outs[0][0]
     for _, db in outs:
         assert (np.abs(db - dz.sum(0)) <= P * 2.0 ** -23 * np.abs(dz).sum(0)).all()
+
+
+def test_the_network_as_one_call_is_its_layers(pkg):
+    """The forward pass of lbm_nn_unet_forward against the same layers called one by one: the same bits."""
+    import torch
+    S = pkg.surrogate
+    lib = S.nn()
+    B, R = 2, 24
+    net = S.Net(R=R, seed=3)
+    x = torch.randn(B, R, R, S.IN_CH, generator=torch.Generator().manual_seed(1)).cuda().to(torch.bfloat16)
+    y = net.forward(x).clone()
+    c1, c2, c3, c4 = S.LEVELS
+    st = torch.cuda.current_stream().cuda_stream
+    t = {}
+
+    def conv(k, v, xs, out, os_, oo):
+        name, ci, co = net.table[k]
+        o, ob = net.off[name]
+        H = v.shape[1]
+        z = torch.empty(B, H, H, co, device="cuda")
+        assert lib.lbm_nn_conv3x3(v.data_ptr(), xs, 0, net.pb.data_ptr() + 2 * o, net.master.data_ptr() + 4 * ob, B, H, H,
+                                  ci, co, z.data_ptr(), co, 0, 0, out.data_ptr(), os_, oo, 1, st) == 0
+        return out
+
+    def new(H, c):
+        return torch.zeros(B, H, H, c, device="cuda", dtype=torch.bfloat16)
+
+    v, width = x, S.IN_CH
+    for e, (c, up) in enumerate(((c1, c2), (c2, c3), (c3, c4))):
+        H = R >> e
+        t[e] = conv(2 * e + 1, conv(2 * e, v, width, new(H, c), c, 0), c, new(H, up + c), up + c, up)
+        v, width = new(H // 2, c), c
+        assert lib.lbm_nn_pool2(t[e].data_ptr(), up + c, up, B, H, H, c, v.data_ptr(), c, 0, st) == 0
+    v = conv(7, conv(6, v, c3, new(R // 8, c4), c4, 0), c4, new(R // 8, c4), c4, 0)
+    for d, (c, up) in enumerate(((c3, c4), (c2, c3), (c1, c2))):
+        e = 2 - d
+        H = R >> e
+        assert lib.lbm_nn_up2(v.data_ptr(), up, 0, B, H // 2, H // 2, up, t[e].data_ptr(), up + c, 0, st) == 0
+        v = conv(9 + 2 * d, conv(8 + 2 * d, t[e], up + c, new(H, c), c, 0), c, new(H, c), c, 0)
+    o, ob = net.off["head"]
+    want = torch.empty_like(y)
+    assert lib.lbm_nn_head(v.data_ptr(), c1, 0, net.pb.data_ptr() + 2 * o, net.master.data_ptr() + 4 * ob, B * R * R, c1,
+                           S.OUT_CH, want.data_ptr(), st) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    import ctypes
+    bad = ctypes.byref(S._Unet(B=0, R=R, J=3))
+    assert lib.lbm_nn_unet_forward(None, st) < 0 and lib.lbm_nn_unet_backward(bad, st) < 0
