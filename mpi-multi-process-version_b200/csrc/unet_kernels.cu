@@ -35,7 +35,7 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kThreads = 256;
 
-// Every kernel here is launched as a programmatic dependent of the one before: its
+// Every kernel here but k_conv3x3 is launched as a programmatic dependent of the one before: its
 // blocks may be set up while that one still runs, and it reads and writes only
 // after dep_sync.  118 launches a training step (batch 16, 128 x 128): 1.86 ms as ordinary
 // launches, 1.73 so.
@@ -1385,12 +1385,14 @@ extern "C" int lbm_nn_conv3x3(const void *x, int64_t xs, int32_t xo, const void 
         if (!conv_tc(a, s)) return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_conv3x3: no tensor maps on this device");
         return launched("lbm_nn_conv3x3 (tcgen05)");
     }
+    // ordinary launches: set up while another grid runs, a grid below one wave would share few SMs (128 blocks: 106 us
+    // as programmatic dependents of one another, 55 so)
     if (Cout <= 32) {
         dim3 grid(unsigned((M + CBM - 1) / CBM), unsigned((Cout + 31) / 32));
-        go(k_conv3x3<32>, grid, kThreads, 0, s, a);
+        k_conv3x3<32><<<grid, kThreads, 0, s>>>(a);
     } else {
         dim3 grid(unsigned((M + CBM - 1) / CBM), unsigned((Cout + 63) / 64));
-        go(k_conv3x3<64>, grid, kThreads, 0, s, a);
+        k_conv3x3<64><<<grid, kThreads, 0, s>>>(a);
     }
     return launched("lbm_nn_conv3x3");
 }
