@@ -1146,12 +1146,17 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on: what earlier kernels wrote
-    if (tid < BN) sbias[tid] = a.bias && n0 + tid < a.Cout ? a.bias[n0 + tid] : 0.0f;
+    if (tid == 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&wmap) : "memory");
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on: what earlier kernels wrote
+    if (tid >= 64 && tid - 64 < BN)  // read after the next block barrier
+        sbias[tid - 64] = a.bias && n0 + tid - 64 < a.Cout ? a.bias[n0 + tid - 64] : 0.0f;
 
     constexpr uint32_t idesc = umma_idesc<BN>();
     bool fail = false;
