@@ -782,7 +782,8 @@ static int resolve_path(lbm_handle *h)
                                                    : fast::resident_blocks(h->geo, h->p.storage, h->device);
         if (nb > 0 && (int64_t)nb * 256 >= h->geo.nnode) h->resident = nb;
     }
-    return LBM_OK;
+    // a choice that changed after the init call: planned here, so that stepping itself uploads nothing
+    return h->phase && h->owns_stream ? ensure_plan(h) : LBM_OK;
 }
 
 extern "C" int lbm_create(const lbm_params *p, const double *x, const double *y, const double *z, lbm_handle **out)
