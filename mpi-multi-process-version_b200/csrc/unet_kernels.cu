@@ -997,12 +997,15 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // block) in tensor memory.  The kernel was bound by gathering the im2col matrix,
 // nine copies of every pixel; here a K chunk is 32 input channels and all nine
 // taps, and its pixels are staged once, with a one-pixel border:
-//   * A lies as four panels of 8 channels, [panel][18 x 10 pixels][16 bytes].  The
-//     8 pixels of a tile row are a core matrix (8 rows of 16 bytes), the rows of
-//     the tile 160 bytes apart (stride offset) and the panels 2880 (leading
-//     offset): in this layout without swizzle a tap is a shift of the start
-//     address by whole 16-byte pixels;
-//   * B is the chunk's weights of the nine taps, [tap][panel][BN][16 bytes];
+//   * A lies as rows of one pixel's 32 channels, 64 bytes under the 64-byte swizzle,
+//     18 x 10 of them.  The 8 pixels of a tile row are a core matrix, the rows of
+//     the tile 640 bytes apart (stride offset); the swizzle goes by address bits, so
+//     a tap is a shift of the start address by whole pixels;
+//   * B is the chunk's weights of the nine taps, [tap][BN][64 bytes], likewise;
+//   * rows of 64 bytes are what the copies want: a TMA box costs about 1.2 cycles a
+//     row whatever its length, and rows of 16 bytes (8 channels, no swizzle) made
+//     the copies the bottleneck.  us at batch 16, 16-byte rows -> 64: 64 -> 64 channels at
+//     64 x 64 29 -> 14, 192 -> 64 50 -> 22, 32 -> 32 at 128 x 128 34 -> 21;
 //   * one thread issues the copies, one TMA box for a tile's pixels (zero outside
 //     the image) and one for the weights, another a chunk's 18 tcgen05.mma (K =
 //     16) per tile, committed to the stage's mbarrier; copies by all threads took
@@ -1054,12 +1057,12 @@ __device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// shared-memory matrix descriptor: start address, leading / stride byte
-// offsets (>> 4), descriptor version 1, base offset 0, no swizzle
-__device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
+// shared-memory matrix descriptor: start address, byte offset of the next 8 rows
+// (both >> 4), descriptor version 1, base offset 0, rows of 64 bytes, 64-byte swizzle
+__device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t sbo)
 {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
 }
 
 // instruction descriptor of kind::f16: FP32 accumulator, bf16 A and B, both
@@ -1072,15 +1075,17 @@ __host__ __device__ constexpr uint32_t umma_idesc()
 
 template <int BN, int NM>
 struct TcLayout {
-    static constexpr int PANEL = THP * 16;             // 2880: 8 channels of the tile and its border
-    static constexpr int A_BYTES = 4 * PANEL;
-    static constexpr int TAP = 4 * BN * 16;            // a tap's weights
+    static constexpr int ROW = TBK * 2;                // 64: a pixel's, an output channel's input channels
+    static constexpr int A_TX = THP * ROW;             // the tile and its border
+    static constexpr int A_BYTES = (A_TX + 1023) / 1024 * 1024;
+    static constexpr int TAP = BN * ROW;               // a tap's weights
     static constexpr int BOFF = NM * A_BYTES;
     static constexpr int STAGE = BOFF + 9 * TAP;
-    static constexpr int HEAD = 128 + BN * 4;          // mbarriers, the TMEM address, the channels' bias
+    static constexpr int HEAD = 1024;                  // mbarriers, the TMEM address, the channels' bias
+    static_assert(STAGE % 1024 == 0 && 128 + BN * 4 <= HEAD, "the swizzle goes by address bits");
     static constexpr int COLS = NM * BN;               // TMEM columns
     static_assert(COLS == 32 || COLS == 64 || COLS == 128, "TMEM allocations are powers of two >= 32");
-    static constexpr int smem(int stages) { return HEAD + stages * STAGE + 128; }
+    static constexpr int smem(int stages) { return HEAD + stages * STAGE + 1024; }
     // shared memory bounds the CTAs per SM, so their TMEM columns fit the SM's 512
     static_assert((228 * 1024 / smem(1)) * COLS <= 512, "TMEM oversubscription");
 };
@@ -1097,19 +1102,19 @@ __device__ __forceinline__ void nn_expect(uint64_t *b, uint32_t bytes)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void nn_tma4(void *dst, const CUtensorMap *m, uint64_t *bar, int c1, int c2, int c3)
+__device__ __forceinline__ void nn_tma3(void *dst, const CUtensorMap *m, uint64_t *bar, int c0, int c1, int c2)
 {
     asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(smem_u32(dst)), "l"(m), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];" ::"r"(smem_u32(dst)), "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
         : "memory");
 }
 
-__device__ __forceinline__ void nn_tma5(void *dst, const CUtensorMap *m, uint64_t *bar, int c1, int c2, int c3, int c4)
+__device__ __forceinline__ void nn_tma4(void *dst, const CUtensorMap *m, uint64_t *bar, int c0, int c1, int c2, int c3)
 {
     asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-        "%6}], [%7];" ::"r"(smem_u32(dst)), "l"(m), "r"(0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)), "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
         : "memory");
 }
 
@@ -1121,7 +1126,7 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
 {
     using Lt = TcLayout<BN, NM>;
     extern __shared__ unsigned char tc_raw[];
-    unsigned char *sm = tc_raw + ((128u - (smem_u32(tc_raw) & 127u)) & 127u);
+    unsigned char *sm = tc_raw + ((1024u - (smem_u32(tc_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm);  // a stage's copies have landed
     uint64_t *bars = full + NST;                        // the MMAs that read it are complete
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + NST);
@@ -1170,13 +1175,13 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
             }
             unsigned char *base = stages + st * Lt::STAGE;
             const int t0 = blockIdx.x * NM, live = NM == 1 || t0 + 1 < ntiles ? NM : 1;
-            nn_expect(&full[st], uint32_t(live * Lt::A_BYTES + 9 * Lt::TAP));
+            nn_expect(&full[st], uint32_t(live * Lt::A_TX + 9 * Lt::TAP));
             for (int i = 0; i < live; ++i) {
                 const int t = t0 + i;
-                nn_tma5(base + i * Lt::A_BYTES, &xmap, &full[st], (t % ntx) * TTW - 1, ((t / ntx) % nty) * TTH - 1,
-                        kc * 4, t / (ntx * nty));
+                nn_tma4(base + i * Lt::A_BYTES, &xmap, &full[st], kc * TBK, (t % ntx) * TTW - 1,
+                        ((t / ntx) % nty) * TTH - 1, t / (ntx * nty));
             }
-            nn_tma4(base + Lt::BOFF, &wmap, &full[st], n0, kc * 4, 0);
+            nn_tma3(base + Lt::BOFF, &wmap, &full[st], kc * TBK, n0, 0);
         }
         if (fail)  // copies still in flight land before the shared memory is released
             for (int k = kc > NST ? kc - NST : 0; k < kc; ++k) nn_mbar_wait(&full[k % NST], uint32_t((k / NST) & 1));
@@ -1191,16 +1196,14 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
             const uint32_t base = smem_u32(stages + (kc % NST) * Lt::STAGE);
 #pragma unroll 1
             for (int tap = 0; tap < 9; ++tap) {
-                const uint32_t shift = uint32_t((tap / 3) * THW + tap % 3) * 16u;
+                const uint32_t shift = uint32_t((tap / 3) * THW + tap % 3) * Lt::ROW;
 #pragma unroll
                 for (int ks = 0; ks < TBK; ks += 16) {
-                    const uint64_t db =
-                        umma_desc(base + Lt::BOFF + tap * Lt::TAP + (ks / 8) * (BN * 16), BN * 16, 128);
+                    const uint64_t db = umma_desc(base + Lt::BOFF + tap * Lt::TAP + ks * 2, 8 * Lt::ROW);
                     const uint32_t accum = (kc > 0 || tap > 0 || ks > 0) ? 1u : 0u;
 #pragma unroll
                     for (int i = 0; i < NM; ++i) {
-                        const uint64_t da = umma_desc(base + i * Lt::A_BYTES + (ks / 8) * Lt::PANEL + shift,
-                                                      Lt::PANEL, THW * 16);
+                        const uint64_t da = umma_desc(base + i * Lt::A_BYTES + shift + ks * 2, THW * Lt::ROW);
                         asm volatile(
                             "{\n\t.reg .pred p;\n\t"
                             "setp.ne.b32 p, %4, 0;\n\t"
@@ -1286,8 +1289,8 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Lt::COLS) : "memory");
 }
 
-// the input as (channel of 8, x, y, panel of 8 channels, image): a box is a tile with its border in the layout above,
-// zero outside the image; the weights as (channel of 8, output channel, panel, tap)
+// the input as (channel, x, y, image): a box is a tile with its border, zero outside the image; the weights as
+// (input channel, output channel, tap)
 bool conv_maps(const ConvArgs &a, int BN, CUtensorMap *xm, CUtensorMap *wm)
 {
     typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1295,19 +1298,19 @@ bool conv_maps(const ConvArgs &a, int BN, CUtensorMap *xm, CUtensorMap *wm)
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     const Encode enc = (Encode)lbm::tensor_map_encoder();
     if (!enc) return false;
-    const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
     const cuuint64_t row = (cuuint64_t)a.xs * 2;
-    const cuuint64_t xd[5] = {8, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.Cin / 8, (cuuint64_t)a.B};
-    const cuuint64_t xst[4] = {row, row * a.W, 16, row * a.W * a.H};
-    const cuuint32_t xb[5] = {8, THW, TTH + 2, TBK / 8, 1};
-    const cuuint64_t wd[4] = {8, (cuuint64_t)a.Cout, (cuuint64_t)a.Cin / 8, 9};
-    const cuuint64_t wst[3] = {(cuuint64_t)a.Cin * 18, 16, (cuuint64_t)a.Cin * 2};
-    const cuuint32_t wb[4] = {8, (cuuint32_t)BN, TBK / 8, 9};
-    return enc(xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void *)(a.x + a.xo), xd, xst, xb, one,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    const cuuint64_t xd[4] = {(cuuint64_t)a.Cin, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
+    const cuuint64_t xst[3] = {row, row * a.W, row * a.W * a.H};
+    const cuuint32_t xb[4] = {TBK, THW, TTH + 2, 1};
+    const cuuint64_t wd[3] = {(cuuint64_t)a.Cin, (cuuint64_t)a.Cout, 9};
+    const cuuint64_t wst[2] = {(cuuint64_t)a.Cin * 18, (cuuint64_t)a.Cin * 2};
+    const cuuint32_t wb[3] = {TBK, (cuuint32_t)BN, 9};
+    return enc(xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)(a.x + a.xo), xd, xst, xb, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
-           enc(wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.w, wd, wst, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+           enc(wm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)a.w, wd, wst, wb, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
                CUDA_SUCCESS;
 }
 
