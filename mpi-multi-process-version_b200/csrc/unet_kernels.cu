@@ -993,9 +993,9 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // 3x3 convolution on the 5th-generation tensor cores (tcgen05, TMEM)
 // ---------------------------------------------------------------------------
 // The implicit GEMM of k_conv3x3 (M = pixels, N = Cout, K = 9 Cin) on a tile of
-// 8 x 16 pixels, with the accumulators (128 pixels x BN channels, FP32, NM tiles a
-// block) in tensor memory.  The kernel was bound by gathering the im2col matrix,
-// nine copies of every pixel; here a K chunk is 32 input channels and all nine
+// 8 x 16 pixels, with the accumulators (128 pixels x BN channels, FP32) in tensor
+// memory.  The kernel was bound by gathering the im2col matrix, nine copies of
+// every pixel; here a K chunk is 32 input channels and all nine
 // taps, and its pixels are staged once, with a one-pixel border:
 //   * A lies as rows of one pixel's 32 channels, 64 bytes under the 64-byte swizzle,
 //     18 x 10 of them.  The 8 pixels of a tile row are a core matrix, the rows of
@@ -1008,8 +1008,10 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 //     64 x 64 29 -> 14, 192 -> 64 50 -> 22, 32 -> 32 at 128 x 128 34 -> 21;
 //   * one thread issues the copies, one TMA box for a tile's pixels (zero outside
 //     the image) and one for the weights, another a chunk's 18 tcgen05.mma (K =
-//     16) per tile, committed to the stage's mbarrier; copies by all threads took
-//     2000 cycles a chunk for their addresses, as long as the MMAs;
+//     16), committed to the stage's mbarrier; copies by all threads took 2000 cycles
+//     a chunk for their addresses, and the MMAs' descriptors, computed anew for
+//     each, 130 cycles an MMA (us, so and as constants: 384 -> 128 at 32 x 32,
+//     batch 1, 16.5 -> 11.3; 256 -> 256 at 16 x 16 12.4 -> 8.9);
 //   * the launch is a programmatic dependent: its set-up overlaps the end of the
 //     kernel before;
 //   * the epilogue reads the accumulators with tcgen05.ld, a thread one pixel and
@@ -1073,18 +1075,18 @@ __host__ __device__ constexpr uint32_t umma_idesc()
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
 }
 
-template <int BN, int NM>
+template <int BN>
 struct TcLayout {
     static constexpr int ROW = TBK * 2;                // 64: a pixel's, an output channel's input channels
     static constexpr int A_TX = THP * ROW;             // the tile and its border
     static constexpr int A_BYTES = (A_TX + 1023) / 1024 * 1024;
     static constexpr int TAP = BN * ROW;               // a tap's weights
-    static constexpr int BOFF = NM * A_BYTES;
+    static constexpr int BOFF = A_BYTES;
     static constexpr int STAGE = BOFF + 9 * TAP;
     static constexpr int HEAD = 1024;                  // mbarriers, the TMEM address, the channels' bias
     static_assert(STAGE % 1024 == 0 && 128 + BN * 4 <= HEAD, "the swizzle goes by address bits");
-    static constexpr int COLS = NM * BN;               // TMEM columns
-    static_assert(COLS == 32 || COLS == 64 || COLS == 128, "TMEM allocations are powers of two >= 32");
+    static constexpr int COLS = BN;                    // TMEM columns
+    static_assert(COLS == 32 || COLS == 64, "TMEM allocations are powers of two >= 32");
     static constexpr int smem(int stages) { return HEAD + stages * STAGE + 1024; }
     // shared memory bounds the CTAs per SM, so their TMEM columns fit the SM's 512
     static_assert((228 * 1024 / smem(1)) * COLS <= 512, "TMEM oversubscription");
@@ -1119,12 +1121,12 @@ __device__ __forceinline__ void nn_tma4(void *dst, const CUtensorMap *m, uint64_
 }
 
 // vec: the outputs' channel strides, offsets and addresses allow 32-byte stores
-template <int BN, int NM, int NST>
+template <int BN, int NST>
 __global__ void __launch_bounds__(TTHREADS)
 k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, int ntx,
-             int nty, int ntiles, int vec)
+             int nty, int vec)
 {
-    using Lt = TcLayout<BN, NM>;
+    using Lt = TcLayout<BN>;
     extern __shared__ unsigned char tc_raw[];
     unsigned char *sm = tc_raw + ((1024u - (smem_u32(tc_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm);  // a stage's copies have landed
@@ -1174,13 +1176,10 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
                 break;
             }
             unsigned char *base = stages + st * Lt::STAGE;
-            const int t0 = blockIdx.x * NM, live = NM == 1 || t0 + 1 < ntiles ? NM : 1;
-            nn_expect(&full[st], uint32_t(live * Lt::A_TX + 9 * Lt::TAP));
-            for (int i = 0; i < live; ++i) {
-                const int t = t0 + i;
-                nn_tma4(base + i * Lt::A_BYTES, &xmap, &full[st], kc * TBK, (t % ntx) * TTW - 1,
-                        ((t / ntx) % nty) * TTH - 1, t / (ntx * nty));
-            }
+            const int t = blockIdx.x;
+            nn_expect(&full[st], uint32_t(Lt::A_TX + 9 * Lt::TAP));
+            nn_tma4(base, &xmap, &full[st], kc * TBK, (t % ntx) * TTW - 1, ((t / ntx) % nty) * TTH - 1,
+                    t / (ntx * nty));
             nn_tma3(base + Lt::BOFF, &wmap, &full[st], kc * TBK, n0, 0);
         }
         if (fail)  // copies still in flight land before the shared memory is released
@@ -1193,24 +1192,22 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
                 break;
             }
             tc_fence_after();
+            // a descriptor's address field counts 16 bytes: a tap or 16 channels on is a constant more
             const uint32_t base = smem_u32(stages + (kc % NST) * Lt::STAGE);
-#pragma unroll 1
+            const uint64_t da0 = umma_desc(base, THW * Lt::ROW), db0 = umma_desc(base + Lt::BOFF, 8 * Lt::ROW);
+#pragma unroll
             for (int tap = 0; tap < 9; ++tap) {
-                const uint32_t shift = uint32_t((tap / 3) * THW + tap % 3) * Lt::ROW;
 #pragma unroll
                 for (int ks = 0; ks < TBK; ks += 16) {
-                    const uint64_t db = umma_desc(base + Lt::BOFF + tap * Lt::TAP + ks * 2, 8 * Lt::ROW);
-                    const uint32_t accum = (kc > 0 || tap > 0 || ks > 0) ? 1u : 0u;
-#pragma unroll
-                    for (int i = 0; i < NM; ++i) {
-                        const uint64_t da = umma_desc(base + i * Lt::A_BYTES + shift + ks * 2, THW * Lt::ROW);
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + i * BN),
-                            "l"(da), "l"(db), "r"(idesc), "r"(accum)
-                            : "memory");
-                    }
+                    const uint64_t da = da0 + (uint64_t)(((tap / 3) * THW + tap % 3) * Lt::ROW + ks * 2) / 16;
+                    const uint64_t db = db0 + (uint64_t)(tap * Lt::TAP + ks * 2) / 16;
+                    const uint32_t accum = tap > 0 || ks > 0 ? 1u : uint32_t(kc > 0);
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+                        "l"(da), "l"(db), "r"(idesc), "r"(accum)
+                        : "memory");
                 }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -1227,19 +1224,17 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
     if (__syncthreads_or(fail || !done)) {
         if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
     } else {
-        // warp w reads TMEM lanes 32 (w % 4) ..: pixels 4 tile rows; two warpgroups split the tiles (NM = 2) or
-        // the channel slices
+        // warp w reads TMEM lanes 32 (w % 4) ..: pixels 4 tile rows; two warpgroups split the channel slices
         const int wg = warp >> 2;
-        const int t = blockIdx.x * NM + (NM == 2 ? wg : 0);
+        const int t = blockIdx.x;
         const int row = (warp & 3) * 32 + lane;
         const int xx = (t % ntx) * TTW + (row & 7), yy = ((t / ntx) % nty) * TTH + (row >> 3), b = t / (ntx * nty);
-        const bool px = t < ntiles && xx < a.W && yy < a.H;
+        const bool px = xx < a.W && yy < a.H;
         const int64_t m = ((int64_t)b * a.H + yy) * a.W + xx;
 #pragma unroll 1
-        for (int sl = NM == 2 ? 0 : wg; sl < BN / 16; sl += NM == 2 ? 1 : 2) {
+        for (int sl = wg; sl < BN / 16; sl += 2) {
             uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) +
-                                   (uint32_t)((NM == 2 ? wg * BN : 0) + sl * 16);
+            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(sl * 16);
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15},"
                 " [%16];"
@@ -1314,30 +1309,32 @@ bool conv_maps(const ConvArgs &a, int BN, CUtensorMap *xm, CUtensorMap *wm)
                CUDA_SUCCESS;
 }
 
-template <int BN, int NM, int NST>
+template <int BN, int NST>
 bool launch_conv_tc(const ConvArgs &a, int vec, cudaStream_t s)
 {
-    using Lt = TcLayout<BN, NM>;
+    using Lt = TcLayout<BN>;
     CUtensorMap xm, wm;
     if (!conv_maps(a, BN, &xm, &wm)) return false;
-    const int ntx = (a.W + TTW - 1) / TTW, nty = (a.H + TTH - 1) / TTH, ntiles = a.B * ntx * nty;
-    cudaFuncSetAttribute(k_conv3x3_tc<BN, NM, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lt::smem(NST));
-    const dim3 grid(unsigned((ntiles + NM - 1) / NM), unsigned((a.Cout + BN - 1) / BN));
-    go(k_conv3x3_tc<BN, NM, NST>, grid, TTHREADS, Lt::smem(NST), s, a, xm, wm, ntx, nty, ntiles, vec);
+    const int ntx = (a.W + TTW - 1) / TTW, nty = (a.H + TTH - 1) / TTH;
+    cudaFuncSetAttribute(k_conv3x3_tc<BN, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lt::smem(NST));
+    const dim3 grid(unsigned(a.B * ntx * nty), unsigned((a.Cout + BN - 1) / BN));
+    go(k_conv3x3_tc<BN, NST>, grid, TTHREADS, Lt::smem(NST), s, a, xm, wm, ntx, nty, vec);
     return true;
 }
 
 int64_t tc_tiles(const ConvArgs &a) { return (int64_t)a.B * ((a.W + TTW - 1) / TTW) * ((a.H + TTH - 1) / TTH); }
 
-// Channels and tiles per block and stages of the ring.  An MMA of 128 pixels takes
-// some 100 cycles for 32 or 64 channels alike, so 64 channels a block where that
-// gives a block to every SM; 32 where it does not.  Where more blocks than fit
-// at once keep coming, one stage and many small blocks overlap one another
-// (us, one stage / two / two tiles and two stages: 64 -> 64 at 64 x 64, batch 16,
-// 23.4 / 26.9 / 27.0; 96 -> 32 at 128 x 128 with two tiles 46, one tile and two
-// stages 69); a grid of one wave needs its stages (128 -> 128 at 32 x 32: 34 / 20.7
-// / 18.5), the more the fewer blocks share an SM (256 -> 128 at 16 x 16, 32
-// channels: two 27, four 14; 256 -> 256: three 22, two 31, four 27).
+// Channels per block and stages of the ring.  Few blocks are bound by the latency
+// of one block's chunks: as many blocks as there are SMs for, and stages that fill
+// an SM's shared memory, so that the next kernel's blocks, set up early, don't
+// crowd onto some of the SMs (us, 32 channels and 4 / 3 / 2 stages: 128 -> 128 at
+// 32 x 32, batch 1, 32 blocks, 6.5 / 7.3 / 7.3; 64 -> 64 at 64 x 64, batch 4, 256 blocks,
+// - / 6.6 / 8.1).  More blocks than two an SM take 64 channels, which halves the reads of the
+// pixels: up to 296 of those with two stages (64 -> 128 at 32 x 32, batch 16, 256
+// blocks: two 8.9, one 13.2, three 13 and more), beyond it with one, where four
+// blocks an SM overlap one another (64 -> 64 at 64 x 64, batch 16, 512 blocks: one
+// 13.5, two 16.3; 32 channels a block 17.3; 128 -> 384 at 32 x 32: 64 channels 27, 128 31).
+// Two tiles a block that share the weights gain nothing (32 -> 32 at 128 x 128: 28.8 against 23.8).
 bool conv_tc(const ConvArgs &a, cudaStream_t s)
 {
     const int64_t tiles = tc_tiles(a);
@@ -1345,15 +1342,10 @@ bool conv_tc(const ConvArgs &a, cudaStream_t s)
     const int vec = !a.acc && (!a.of || ((a.os | a.oo) % 8 == 0 && ok32(a.of))) &&
                     (!a.oa || ((a.as | a.ao) % 16 == 0 && ok32(a.oa)));
     const int64_t n64 = tiles * ((a.Cout + 63) / 64), n32 = tiles * ((a.Cout + 31) / 32);
-    const bool wide = a.Cout > 32 && n64 >= 148;
-    if (a.Cin == TBK) {  // one chunk: two tiles share the weights if there are tiles enough for every SM
-        const bool two = tiles >= 592;
-        if (!wide) return two ? launch_conv_tc<32, 2, 1>(a, vec, s) : launch_conv_tc<32, 1, 1>(a, vec, s);
-        return two ? launch_conv_tc<64, 2, 1>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
-    }
-    if (wide) return n64 <= 296 ? launch_conv_tc<64, 2, 2>(a, vec, s) : launch_conv_tc<64, 1, 1>(a, vec, s);
-    if (n32 <= 148) return launch_conv_tc<32, 1, 4>(a, vec, s);
-    return n32 <= 296 ? launch_conv_tc<32, 1, 3>(a, vec, s) : launch_conv_tc<32, 2, 1>(a, vec, s);
+    if (n32 <= 148) return launch_conv_tc<32, 4>(a, vec, s);
+    if (n32 <= 296) return launch_conv_tc<32, 3>(a, vec, s);
+    if (a.Cout <= 32) return launch_conv_tc<32, 1>(a, vec, s);
+    return n64 <= 296 ? launch_conv_tc<64, 2>(a, vec, s) : launch_conv_tc<64, 1>(a, vec, s);
 }
 
 int g_path = 0;            // lbm_nn_set_tensor_path: 0 the faster kernel for the tensors at hand, 1 tcgen05
