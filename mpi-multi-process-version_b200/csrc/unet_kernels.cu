@@ -4,14 +4,14 @@
 // (natural-convection_2dim_mono.f90:199-240).
 //
 // 3x3 convolutions are implicit GEMMs on the tensor cores (bf16 inputs, FP32
-// accumulators, mma m16n8k16):
-//   forward      M = pixels, N = Cout, K = 9 Cin;  A = im2col(x) gathered by
-//                cp.async with zero fill at the image border, B = weights
-//                [Cout][9][Cin] (K contiguous), two-stage shared-memory ring;
+// accumulators), from pixel tiles that serve all nine taps (tcgen05, TMA copies):
+//   forward      M = pixels, N = Cout, K = 9 Cin;
 //   data grad    the same kernel on dL/dz with the flipped, transposed weights;
 //   weight grad  M = Cout, N = 9 Cin, K = pixels, split over pixel tiles into
 //                FP32 partials that a second kernel sums in a fixed order
 //                (deterministic).
+// k_conv3x3 (mma.sync) takes pixels in a row, across images, for many images far
+// smaller than a tile.
 // Elementwise work (SiLU backward, pooling, upsampling, the 1x1 output layer,
 // the loss, Adam) is plain CUDA-core code.
 #include <cuda.h>
@@ -251,145 +251,8 @@ __global__ void k_flip(const bf16 *__restrict__ w, bf16 *__restrict__ wt, int Co
 }
 
 // ---------------------------------------------------------------------------
-// 3x3 weight gradient
+// sums of the weight gradient's and the column sums' shares
 // ---------------------------------------------------------------------------
-// dw[co][tap][ci] = sum_p dz[p][co] x[p + offset(tap)][ci]: M = Cout, N = 9 Cin,
-// K = pixels.  A block owns BM output channels x 32 input channels x all nine
-// taps (72 accumulators a thread) and walks over its share of 16 x 8 pixel
-// tiles; a tile's dz and its x with a one-pixel border are staged once
-// (cp.async, two stages) and serve the nine taps, whose operands are the same
-// rows of shared memory at shifted addresses.  Both operands lie pixel-major
-// in memory and K runs over pixels, so both fragments come from transposing
-// ldmatrix; row strides of an odd number of 16-byte units keep it free of bank
-// conflicts.  The shares' partial sums are added in a fixed order.
-// Measured at batch 16 of 128^2 images, one backward pass, B200: the former
-// kernel (one tap and 32 pixels a step, operands transposed by scalar stores)
-// 2.9 ms in all layers, this one 0.46 ms.
-constexpr int GTW = 16, GTH = 8, GPX = GTW * GTH;   // pixel tile
-constexpr int GHW = GTW + 2, GHP = GHW * (GTH + 2);  // its x with the border
-constexpr int WBN = 32;                              // input channels per block
-constexpr int GXP = WBN + 8;                         // elements between x rows
-
-template <int BM>
-struct WgLayout {
-    static constexpr int threads = BM * 4;
-    static constexpr int DP = BM + 8;                // elements between dz rows
-    static constexpr int XOFF = GPX * DP * 2;
-    static constexpr int STAGE = XOFF + GHP * GXP * 2;
-    static constexpr int SMEM = 2 * STAGE;
-    static_assert((DP * 2 / 16) % 2 == 1 && (GXP * 2 / 16) % 2 == 1 && STAGE % 16 == 0, "conflict-free rows");
-};
-
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const bf16 *p)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(s));
-}
-
-template <int BM>
-__global__ void __launch_bounds__(BM * 4, BM == 64 ? 2 : 4)
-k_wgrad(const bf16 *__restrict__ dz, const bf16 *__restrict__ x, int64_t xs, int xo, int B, int H, int W, int Cin,
-        int Cout, int ntx, int nty, int per, float *__restrict__ ws)
-{
-    dep_sync();
-    using L = WgLayout<BM>;
-    extern __shared__ __align__(16) unsigned char wg_sm[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 2, wn = warp & 3;
-    const int c0 = blockIdx.x * WBN, co0 = blockIdx.y * BM;
-    const int ntiles = B * ntx * nty;
-    const int t_beg = blockIdx.z * per, t_end = min(t_beg + per, ntiles);
-
-    auto load = [&](int t, int st) {
-        const int tx = t % ntx, ty = (t / ntx) % nty, b = t / (ntx * nty);
-        const int x0 = tx * GTW, y0 = ty * GTH;
-        const int rows = min(GTH, (H - y0 + 1) & ~1);  // rows the MMAs visit, in pairs
-        bf16 *ds = (bf16 *)(wg_sm + st * L::STAGE), *xsm = (bf16 *)(wg_sm + st * L::STAGE + L::XOFF);
-#pragma unroll
-        for (int k = 0; k < GPX * (BM / 8) / L::threads; ++k) {
-            const int v = tid + k * L::threads, px = v / (BM / 8), q = v % (BM / 8);
-            if (px >= rows * GTW) break;
-            const int xx = x0 + px % GTW, yy = y0 + px / GTW;
-            const bool ok = xx < W && yy < H && co0 + q * 8 < Cout;
-            const bf16 *src = ok ? dz + ((int64_t)(b * H + yy) * W + xx) * Cout + co0 + q * 8 : dz;
-            cp_async16(ds + px * L::DP + q * 8, src, ok ? 16 : 0);
-        }
-        for (int v = tid; v < (rows + 2) * GHW * 4; v += L::threads) {
-            const int px = v >> 2, q = v & 3;
-            const int xx = x0 + px % GHW - 1, yy = y0 + px / GHW - 1;
-            const bool ok = xx >= 0 && xx < W && yy >= 0 && yy < H;
-            const bf16 *src = ok ? x + ((int64_t)(b * H + yy) * W + xx) * xs + xo + c0 + q * 8 : x;
-            cp_async16(xsm + px * GXP + q * 8, src, ok ? 16 : 0);
-        }
-        cp_commit();
-    };
-
-    float acc[2][9][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 9; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.0f;
-
-    // ldmatrix row addresses: A (channels x pixels): matrices (co, px) (co+8, px) (co, px+8) (co+8, px+8);
-    // B (pixels x channels): pixels 0-7 and 8-15 of a tile row, then of the next one
-    const int arow = (lane >> 4) * 8 + (lane & 7), acol = wm * 32 + ((lane >> 3) & 1) * 8;
-    const int brow = (lane >> 4) * GHW + ((lane >> 3) & 1) * 8 + (lane & 7), bcol = wn * 8;
-
-    if (t_beg < t_end) load(t_beg, 0);
-    for (int t = t_beg; t < t_end; ++t) {
-        const int st = (t - t_beg) & 1;
-        if (t + 1 < t_end) {
-            load(t + 1, st ^ 1);
-            cp_wait<1>();
-        } else {
-            cp_wait<0>();
-        }
-        __syncthreads();
-        const bf16 *ds = (const bf16 *)(wg_sm + st * L::STAGE) + arow * L::DP + acol;
-        const bf16 *xb = (const bf16 *)(wg_sm + st * L::STAGE + L::XOFF) + brow * GXP + bcol;
-        const int rows = min(GTH, H - (t / ntx) % nty * GTH);
-#pragma unroll 1
-        for (int r = 0; r < rows; r += 2) {
-            uint32_t af[2][2][4];
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int mt = 0; mt < 2; ++mt) ldsm4t(af[k][mt], ds + (r + k) * GTW * L::DP + mt * 16);
-#pragma unroll
-            for (int tap = 0; tap < 9; ++tap) {
-                uint32_t bfr[4];
-                ldsm4t(bfr, xb + ((r + tap / 3) * GHW + tap % 3) * GXP);
-#pragma unroll
-                for (int k = 0; k < 2; ++k)
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt)
-                        mma16816(acc[mt][tap], af[k][mt][0], af[k][mt][1], af[k][mt][2], af[k][mt][3], bfr[2 * k],
-                                 bfr[2 * k + 1]);
-            }
-        }
-        __syncthreads();
-    }
-    const int64_t K9 = 9 * (int64_t)Cin;
-    const int g = lane >> 2, tq = lane & 3;
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int co = co0 + wm * 32 + mt * 16 + g + h * 8;
-            if (co >= Cout) continue;
-            float *o = ws + ((int64_t)blockIdx.z * Cout + co) * K9 + c0 + wn * 8 + 2 * tq;
-#pragma unroll
-            for (int tap = 0; tap < 9; ++tap) {
-                o[(int64_t)tap * Cin] = acc[mt][tap][h * 2];
-                o[(int64_t)tap * Cin + 1] = acc[mt][tap][h * 2 + 1];
-            }
-        }
-}
-
 // out[i] = sum_{s < S} ws[s*n + i] in a fixed order: 32 columns a block, its 32
 // warps take every 32nd row and their sums are added in warp order
 constexpr int kSumThreads = 1024;
@@ -451,29 +314,6 @@ void sum_splits(const float *ws, int S, int64_t n, float *out, cudaStream_t s)
         go(k_sum_few, unsigned((n + kThreads - 1) / kThreads), kThreads, 0, s, ws, S, n, out);
     else
         go(k_sum_splits, unsigned((n + 31) / 32), kSumThreads, 0, s, ws, S, n, out);
-}
-
-struct WgradPlan {
-    int BM, ntx, nty, S, per;
-};
-
-// output channels per block (64, or 32 where that is all there are) and the
-// tiles' split over blocks: about two 64-channel or four 32-channel blocks per
-// SM, what registers let run at once
-WgradPlan wgrad_plan(int B, int H, int W, int Cin, int Cout)
-{
-    WgradPlan p;
-    p.BM = Cout <= 32 ? 32 : 64;
-    p.ntx = (W + GTW - 1) / GTW;
-    p.nty = (H + GTH - 1) / GTH;
-    const int64_t tiles = (int64_t)B * p.ntx * p.nty;
-    const int64_t bps = (int64_t)((Cin + WBN - 1) / WBN) * ((Cout + p.BM - 1) / p.BM);
-    const int64_t want = p.BM == 64 ? 296 : 592;
-    int64_t S = (want + bps - 1) / bps;
-    if (S > tiles) S = tiles;
-    p.per = int((tiles + S - 1) / S);
-    p.S = int((tiles + p.per - 1) / p.per);
-    return p;
 }
 
 // ---------------------------------------------------------------------------
@@ -1120,6 +960,25 @@ __device__ __forceinline__ void nn_tma4(void *dst, const CUtensorMap *m, uint64_
         : "memory");
 }
 
+// the same for a channel-major operand: mn, k: byte offsets of the next 32 channels and of the next 8 rows
+__device__ __forceinline__ uint64_t wg_desc(uint32_t addr, uint32_t mn, uint32_t k)
+{
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((mn >> 4) & 0x3FFFu) << 16) |
+           ((uint64_t)((k >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+
+// 16 accumulator columns of the warp's 32 lanes
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 // vec: the outputs' channel strides, offsets and addresses allow 32-byte stores
 template <int BN, int NST>
 __global__ void __launch_bounds__(TTHREADS)
@@ -1138,7 +997,6 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
     const int n0 = blockIdx.y * BN;
     const int nk = a.Cin / TBK;
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(Lt::COLS)
@@ -1161,6 +1019,8 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    // only now that this block has its tensor memory: a dependent's block that took it first would wait for this grid
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on: what earlier kernels wrote
     if (tid >= 64 && tid - 64 < BN)  // read after the next block barrier
         sbias[tid - 64] = a.bias && n0 + tid - 64 < a.Cout ? a.bias[n0 + tid - 64] : 0.0f;
@@ -1219,9 +1079,11 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
     }
     __syncwarp();
     // every MMA of this CTA is complete once the commit of the last chunk arrives
+    // (for tid 0, which has seen the stage's earlier use complete; the others go by the block barrier)
     const bool done = nn_mbar_wait(&bars[(nk - 1) % NST], uint32_t(((nk - 1) / NST) & 1));
+    const bool bad = __syncthreads_or(fail || !done);
     tc_fence_after();
-    if (__syncthreads_or(fail || !done)) {
+    if (bad) {
         if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
     } else {
         // warp w reads TMEM lanes 32 (w % 4) ..: pixels 4 tile rows; two warpgroups split the channel slices
@@ -1234,16 +1096,7 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
 #pragma unroll 1
         for (int sl = wg; sl < BN / 16; sl += 2) {
             uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(sl * 16);
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15},"
-                " [%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr)
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(sl * 16), r);
             const int n = n0 + sl * 16;
             if (!px || n >= a.Cout) continue;
             float z[16];
@@ -1348,6 +1201,207 @@ bool conv_tc(const ConvArgs &a, cudaStream_t s)
     return n64 <= 296 ? launch_conv_tc<64, 2>(a, vec, s) : launch_conv_tc<64, 1>(a, vec, s);
 }
 
+// ---------------------------------------------------------------------------
+// 3x3 weight gradient on the 5th-generation tensor cores
+// ---------------------------------------------------------------------------
+// dw[co][tap][ci] = sum_p dz[p][co] x[p + offset(tap)][ci]: M = 128 output channels,
+// N = 32 input channels x 9 taps, K = pixels, a block's share of the pixel tiles
+// after one another.  dz and x lie as in the convolution, rows of 32
+// channels under the 64-byte swizzle, a tile's dz as [32 channels][128 pixels], its
+// x with the border; both operands are channel-major (their K runs over the
+// rows).  A step of 16 pixels is two tile rows.  The next 32 columns of B are the
+// same channels a pixel further right, so one MMA takes the three taps of a tap row
+// (96 columns); the three tap rows have accumulators of their own, 288 columns.
+// Fewer than 128 output channels leave rows of the accumulators unused; their part
+// of A is never loaded.  The shares' partial sums are added in a fixed order.
+// Measured, us with that sum, mma.sync kernel -> this: 32 -> 32 channels at 128 x 128,
+// batch 16, 27.9 -> 20.9, 96 -> 32 64 -> 50, 384 -> 128 at 32 x 32 74 -> 21, 256 -> 256 at 16 x 16
+// 27.8 -> 14.0; batch 1: 13.6 -> 6.5, -, 14.6 -> 9.9, 10.2 -> 10.5; 256 images of 4 x 4, 256
+// channels 109 -> 26.  A training step's 14 layers 0.46 -> 0.25 ms.  Where channels are few
+// the tiles' 128 rows of A are mostly unused and the MMAs (24 a tile) are the
+// bound; at batch 1 the launch, one tile's latency and the sum.  Against 64-bit
+// sums the error is 1e-7 to 6e-6 of the result, as long as a share's chain.
+constexpr int WST = 4, WCOLS = 512;                 // stages; TMEM columns (a power of two)
+constexpr int WA_ATOM = TBM * 64, WA = 4 * WA_ATOM;  // dz: 32 channels of a tile, all
+constexpr int WX_TX = THP * 64, WX = (WX_TX + 1023) / 1024 * 1024;
+constexpr int WSTAGE = WA + WX, WSMEM = 1024 + WST * WSTAGE + 1024;
+
+__global__ void __launch_bounds__(TTHREADS)
+k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap xmap, int H, int Cin, int Cout,
+           int ntx, int nty, int ntiles, int per, int vec, float *__restrict__ ws)
+{
+    extern __shared__ unsigned char tc_raw[];
+    unsigned char *sm = tc_raw + ((1024u - (smem_u32(tc_raw) & 1023u)) & 1023u);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm);  // a stage's copies have landed
+    uint64_t *bars = full + WST;                        // the MMAs that read it are complete
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + WST);
+    unsigned char *stages = sm + 1024;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c0 = blockIdx.x * 32, co0 = blockIdx.y * TBM;
+    const int t0 = blockIdx.z * per, nt = min(per, ntiles - t0);  // at least one tile
+    const int atoms = min(4, (Cout - co0 + 31) / 32);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(WCOLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < WST; ++k) {
+            nn_mbar_init(&full[k], 1);
+            nn_mbar_init(&bars[k], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (tid == 32) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&zmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // after the allocation, as in k_conv3x3_tc
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    // FP32 accumulators, bf16 A and B, both channel-major, M = 128, N = 96
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (12u << 17) | (8u << 24);
+    bool fail = false;
+    if (tid == 32) {  // the copies
+        int k = 0;
+        for (; k < nt; ++k) {
+            const int st = k % WST, t = t0 + k;
+            if (k >= WST && !nn_mbar_wait(&bars[st], uint32_t((k / WST - 1) & 1))) {
+                fail = true;
+                break;
+            }
+            unsigned char *base = stages + st * WSTAGE;
+            const int x0 = (t % ntx) * TTW, y0 = ((t / ntx) % nty) * TTH, b = t / (ntx * nty);
+            nn_expect(&full[st], uint32_t(atoms * WA_ATOM + WX_TX));
+            for (int a = 0; a < atoms; ++a) nn_tma4(base + a * WA_ATOM, &zmap, &full[st], co0 + a * 32, x0, y0, b);
+            nn_tma4(base + WA, &xmap, &full[st], c0, x0 - 1, y0 - 1, b);
+        }
+        if (fail)  // copies still in flight land before the shared memory is released
+            for (int j = k > WST ? k - WST : 0; j < k; ++j) nn_mbar_wait(&full[j % WST], uint32_t((j / WST) & 1));
+    } else if (tid == 0) {  // the MMAs
+        int k = 0;
+        for (; k < nt; ++k) {
+            if (!nn_mbar_wait(&full[k % WST], uint32_t((k / WST) & 1))) {
+                fail = true;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t base = smem_u32(stages + (k % WST) * WSTAGE);
+            // A: the next 32 channels an atom further, the next 8 pixels a tile row; B: a pixel, a row with its border
+            const uint64_t da0 = wg_desc(base, WA_ATOM, 8 * 64), db0 = wg_desc(base + WA, 64, THW * 64);
+            const int steps = (min(TTH, H - ((t0 + k) / ntx) % nty * TTH) + 1) / 2;  // rows past the image are zeros
+#pragma unroll 2
+            for (int r = 0; r < steps; ++r) {
+                const uint32_t accum = k > 0 || r > 0;
+#pragma unroll
+                for (int dy = 0; dy < 3; ++dy)
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + dy * 96),
+                        "l"(da0 + (uint64_t)(r * (2 * 8 * 64 / 16))),
+                        "l"(db0 + (uint64_t)((2 * r + dy) * (THW * 64 / 16))), "r"(idesc), "r"(accum)
+                        : "memory");
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&bars[k % WST]))
+                         : "memory");
+        }
+        if (fail && k > 0) nn_mbar_wait(&bars[(k - 1) % WST], uint32_t(((k - 1) / WST) & 1));
+    }
+    __syncwarp();
+    // every MMA of this block is complete once the commit of the last tile arrives
+    const bool done = nn_mbar_wait(&bars[(nt - 1) % WST], uint32_t(((nt - 1) / WST) & 1));
+    const bool bad = __syncthreads_or(fail || !done);
+    tc_fence_after();
+    if (bad) {
+        if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
+    } else {
+        // a lane one output channel; two warpgroups split the 18 slices of 16 columns
+        const int co = co0 + (warp & 3) * 32 + lane;
+        float *o = ws + ((int64_t)blockIdx.z * Cout + co) * 9 * Cin + c0;
+#pragma unroll 1
+        for (int sl = warp >> 2; sl < 18; sl += 2) {
+            uint32_t r[16];
+            tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(sl * 16), r);
+            if (co >= Cout) continue;
+            float z[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]);
+            float *q = o + (int64_t)(sl >> 1) * Cin + (sl & 1) * 16;
+            if (vec) {
+                st_v8(q, z);
+                st_v8(q + 8, z + 8);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) q[j] = z[j];
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(WCOLS) : "memory");
+}
+
+struct WgradPlan {
+    int ntx, nty, S, per;
+};
+
+// The tiles' split over blocks: one block per SM, what its tensor memory lets run
+// (us, 148 blocks / 74: 32 -> 32 channels at 128 x 128, batch 16, 20.9 / 34.8; 384 -> 128 at
+// 32 x 32 21.5 / 31.9).  A share's length is also the chain its FP32 sums go through.
+WgradPlan wgrad_plan(int B, int H, int W, int Cin, int Cout)
+{
+    WgradPlan p;
+    p.ntx = (W + TTW - 1) / TTW;
+    p.nty = (H + TTH - 1) / TTH;
+    const int64_t tiles = (int64_t)B * p.ntx * p.nty;
+    const int64_t bps = (int64_t)((Cin + 31) / 32) * ((Cout + TBM - 1) / TBM);
+    int64_t S = bps >= 148 ? 1 : 148 / bps;
+    if (S > tiles) S = tiles;
+    p.per = int((tiles + S - 1) / S);
+    p.S = int((tiles + p.per - 1) / p.per);
+    return p;
+}
+
+// an image tensor as (channel, x, y, image): boxes of 32 channels of w x h pixels, zero outside
+bool pixel_map(const void *p, int C, int64_t stride, int B, int H, int W, int w, int h, CUtensorMap *m)
+{
+    typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                               const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    const Encode enc = (Encode)lbm::tensor_map_encoder();
+    const cuuint64_t row = (cuuint64_t)stride * 2;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t str[3] = {row, row * W, row * W * H};
+    const cuuint32_t box[4] = {32, (cuuint32_t)w, (cuuint32_t)h, 1}, one[4] = {1, 1, 1, 1};
+    return enc && enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)p, dims, str, box, one,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool launch_wgrad_tc(const bf16 *dz, const bf16 *x, int64_t xs, int xo, int B, int H, int W, int Cin, int Cout,
+                     const WgradPlan &pl, float *part, cudaStream_t s)
+{
+    CUtensorMap zm, xm;
+    if (!pixel_map(dz, Cout, Cout, B, H, W, TTW, TTH, &zm) ||
+        !pixel_map(x + xo, Cin, xs, B, H, W, THW, TTH + 2, &xm))
+        return false;
+    cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, WSMEM);
+    const dim3 grid(unsigned(Cin / 32), unsigned((Cout + TBM - 1) / TBM), unsigned(pl.S));
+    go(k_wgrad_tc, grid, TTHREADS, WSMEM, s, zm, xm, H, Cin, Cout, pl.ntx, pl.nty, B * pl.ntx * pl.nty, pl.per,
+       int(((uintptr_t)part & 31u) == 0), part);
+    return true;
+}
+
 int g_path = 0;            // lbm_nn_set_tensor_path: 0 the faster kernel for the tensors at hand, 1 tcgen05
 
 }  // namespace
@@ -1418,7 +1472,7 @@ extern "C" int lbm_nn_conv3x3_wgrad(const void *dz, const void *x, int64_t xs, i
 {
     NN_REQUIRE(dz && x && ws && dw, "lbm_nn_conv3x3_wgrad: NULL pointer");
     NN_REQUIRE(B > 0 && H > 0 && W > 0, "lbm_nn_conv3x3_wgrad: empty shape");
-    NN_REQUIRE(Cin > 0 && Cin % WBN == 0, "lbm_nn_conv3x3_wgrad: Cin must be a positive multiple of 32");
+    NN_REQUIRE(Cin > 0 && Cin % 32 == 0, "lbm_nn_conv3x3_wgrad: Cin must be a positive multiple of 32");
     NN_REQUIRE(Cout > 0 && Cout % 8 == 0, "lbm_nn_conv3x3_wgrad: Cout must be a positive multiple of 8");
     NN_REQUIRE(xs % 8 == 0 && xo % 8 == 0 && xo >= 0 && xo + Cin <= xs, "lbm_nn_conv3x3_wgrad: bad channel stride/offset");
     NN_REQUIRE(aligned16(dz) && aligned16(x), "lbm_nn_conv3x3_wgrad: dz and x must be 16-byte aligned");
@@ -1428,16 +1482,8 @@ extern "C" int lbm_nn_conv3x3_wgrad(const void *dz, const void *x, int64_t xs, i
                (long long)ws_elems, (long long)pl.S * n);
     cudaStream_t s = (cudaStream_t)stream;
     float *part = pl.S == 1 ? dw : ws;  // one share is the sum
-    dim3 grid(unsigned(Cin / WBN), unsigned((Cout + pl.BM - 1) / pl.BM), unsigned(pl.S));
-    if (pl.BM == 64) {
-        cudaFuncSetAttribute(k_wgrad<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, WgLayout<64>::SMEM);
-        go(k_wgrad<64>, grid, WgLayout<64>::threads, WgLayout<64>::SMEM, s,
-            (const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl.ntx, pl.nty, pl.per, part);
-    } else {
-        cudaFuncSetAttribute(k_wgrad<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, WgLayout<32>::SMEM);
-        go(k_wgrad<32>, grid, WgLayout<32>::threads, WgLayout<32>::SMEM, s,
-            (const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl.ntx, pl.nty, pl.per, part);
-    }
+    if (!launch_wgrad_tc((const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl, part, s))
+        return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_conv3x3_wgrad: no tensor maps on this device");
     if (pl.S > 1) sum_splits(ws, pl.S, n, dw, s);
     return launched("lbm_nn_conv3x3_wgrad", pl.S > 1 ? 2 : 1);
 }

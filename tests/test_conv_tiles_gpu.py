@@ -87,6 +87,31 @@ def test_weight_gradient_tile_edges(pkg, B, H, W, Cin, Cout):
     assert (np.abs(down(dw).reshape(ref.shape) - ref) <= B * H * W * 2.0 ** -23 * size).all()
 
 
+# one full tile; tiles past the image, several blocks of output channels, one with a remainder; many tiles a share
+@pytest.mark.parametrize("B,H,W,Cin,Cout,off", [(1, 16, 8, 32, 8, 0), (3, 37, 21, 96, 264, 0), (2, 33, 47, 32, 160, 1),
+                                                (20, 64, 64, 32, 32, 0)])
+def test_weight_gradient_channel_blocks_and_shares(pkg, B, H, W, Cin, Cout, off):
+    import torch
+    lib = pkg.surrogate.nn()
+    rng = np.random.default_rng(B * H * W + Cin + Cout)
+    x = U.bf16_round(rng.normal(size=(B, H, W, Cin)))
+    dz = U.bf16_round(rng.normal(size=(B, H, W, Cout)))
+    xd, dzd = up(torch, x, torch.bfloat16), up(torch, dz, torch.bfloat16)
+    n = lib.lbm_nn_wgrad_workspace(B, H, W, Cin, Cout)
+    ws = torch.full((n + off,), float("nan"), device="cuda")
+    dw = torch.full((Cout * 9 * Cin + 2 * off + 1,), 7.0, device="cuda")
+    pkg.surrogate.timeouts(reset=True)
+    assert lib.lbm_nn_conv3x3_wgrad(dzd.data_ptr(), xd.data_ptr(), Cin, 0, B, H, W, Cin, Cout, ws[off:].data_ptr(), n,
+                                    dw[off:].data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert pkg.surrogate.timeouts(reset=True) == 0
+    ref = U.conv3x3_wgrad(dz, x)
+    size = U.conv3x3_wgrad(np.abs(dz), np.abs(x))
+    got = down(dw)
+    assert (got[:off] == 7.0).all() and (got[off + ref.size:] == 7.0).all()
+    assert (np.abs(got[off:off + ref.size].reshape(ref.shape) - ref) <= B * H * W * 2.0 ** -23 * size).all()
+
+
 # channels: one 16-byte group, more groups than a block has threads, no multiple of 8; an offset that allows no
 # wide loads
 @pytest.mark.parametrize("P,C,off", [(1, 8, 0), (1000, 32, 0), (4737, 96, 4), (70, 2056, 0), (333, 36, 0), (333, 32, 1)])
