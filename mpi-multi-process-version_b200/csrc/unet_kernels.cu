@@ -1429,13 +1429,13 @@ extern "C" int lbm_nn_conv3x3(const void *x, int64_t xs, int32_t xo, const void 
                (bf16 *)oa, as, ao, act};
     const int64_t M = (int64_t)B * H * W;
     cudaStream_t s = (cudaStream_t)stream;
-    // The tcgen05 kernel is the faster on the network's layers (batch 16: 30 us against 59 for 32 -> 32 channels at
-    // 128 x 128, 22 against 55 for 256 -> 256 at 16 x 16) and on any call of few blocks.  mma.sync takes pixels in a
-    // row, across images, and wins where more than two blocks an SM would mostly hold padding (256 images of 17 x 3,
-    // 64 channels: 21 us against 30; of 2 x 2, 256 channels: 53 against 100; of 8 x 4, 128: 33 both; a third full, 9 x 9,
-    // 64: 27 against 21).
+    // The tcgen05 kernel is the faster on the network's layers and wherever its blocks are some thousand at most.
+    // mma.sync takes pixels in a row, across images, and wins where more blocks than that would mostly hold padding
+    // (us, tcgen05 / mma.sync: 2000 images of 2 x 2, 64 channels, 31.8 / 19.4; of 1 x 1, 256, 268 / 48; 1000 of 3 x 3, 128,
+    // 7 % full, 46.6 / 30.8; but 1000 of 5 x 5, 32, a fifth full, 11.6 / 11.9; 256 of 2 x 2, 256, 1024 blocks, 40.8 / 52.3;
+    // 256 of 17 x 3, 64, 12.0 / 19.6).
     const int64_t tiles = tc_tiles(a);
-    if (g_path == 1 || 4 * M >= tiles * TTW * TTH || tiles * ((Cout + 63) / 64) <= 296) {
+    if (g_path == 1 || 8 * M >= tiles * TTW * TTH || tiles * ((Cout + 63) / 64) <= 1024) {
         if (!conv_tc(a, s)) return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_conv3x3: no tensor maps on this device");
         return launched("lbm_nn_conv3x3 (tcgen05)");
     }

@@ -67,6 +67,27 @@ def test_convolution_tile_edges(pkg, B, H, W, Cin, Cout, path):
     assert (np.abs(a - s) <= 2.0 ** -8 * np.abs(s) + 2.0 ** -8 * 2.0 ** -12).all()
 
 
+# on both sides of the rule between the two kernels: blocks of tcgen05 (1024 / 1025), how full they are
+@pytest.mark.parametrize("B,H,W,Cin,Cout", [(1024, 1, 2, 32, 32), (1025, 1, 2, 32, 32), (1030, 3, 1, 64, 72),
+                                            (1025, 4, 4, 32, 8), (1025, 3, 5, 32, 8)])
+def test_convolution_of_many_small_images(pkg, B, H, W, Cin, Cout):
+    import torch
+    S = pkg.surrogate
+    rng = np.random.default_rng(B + H * W + Cin + Cout)
+    x = U.bf16_round(rng.normal(size=(B, H, W, Cin)))
+    w = U.bf16_round(rng.normal(0, 0.1, size=(Cout, 9, Cin)))
+    xd, wd = up(torch, x, torch.bfloat16), up(torch, w, torch.bfloat16)
+    z = torch.full((B, H, W, Cout), 7.0, device="cuda")
+    S.timeouts(reset=True)
+    assert S.nn().lbm_nn_conv3x3(xd.data_ptr(), Cin, 0, wd.data_ptr(), None, B, H, W, Cin, Cout, z.data_ptr(), Cout, 0, 0,
+                                 None, 0, 0, 0, None) == 0
+    torch.cuda.synchronize()
+    assert S.timeouts(reset=True) == 0
+    ref = U.conv3x3(x, w, np.zeros(Cout))
+    size = U.conv3x3(np.abs(x), np.abs(w), np.zeros(Cout))
+    assert (np.abs(down(z) - ref) <= (9 * Cin + 2) * 2.0 ** -23 * size).all()
+
+
 @pytest.mark.parametrize("B,H,W,Cin,Cout", [(1, 1, 1, 32, 8), (2, 8, 16, 32, 32), (2, 9, 17, 64, 40), (1, 7, 33, 96, 72),
                                             (5, 24, 31, 32, 64), (40, 3, 2, 64, 32)])
 def test_weight_gradient_tile_edges(pkg, B, H, W, Cin, Cout):
