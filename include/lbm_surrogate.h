@@ -119,7 +119,8 @@ int lbm_nn_adam(float *p, void *pb, const float *g, float *m, float *v, int64_t 
  *         not used for layers 1, 3, 5) and pre-activation (FP32)
  *   y     the output, FP32 (B R R, J)
  * and for the backward pass, from dy: FP32 da[l], dcat[k], dp[k], bf16 dz[l], and
- * scratch ws, the largest of the single calls' workspaces. */
+ * scratch ws of ws_elems, at least the largest of the single calls' workspaces
+ * (lbm_nn_unet_backward refuses less before any launch). */
 typedef struct lbm_nn_unet {
     int32_t B, R, J, reserved;
     int32_t ch[14][2];

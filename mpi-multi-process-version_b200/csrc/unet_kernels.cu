@@ -20,6 +20,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "../../include/lbm_b200.h"
 #include "../../include/lbm_surrogate.h"
 
@@ -1788,6 +1790,14 @@ extern "C" int lbm_nn_unet_backward(const lbm_nn_unet *net, void *stream)
     const int B = n.B;
     UnetLayer l[14];
     unet_layers(n, l);
+    // every pass of the chain uses the one scratch, the column sums without a size of their own
+    int64_t need = lbm_nn_head_workspace((int64_t)B * n.R * n.R, l[13].as, n.J);
+    for (int k = 0; k < 14; ++k) {
+        const int ci = n.ch[k][0], co = n.ch[k][1], H = l[k].H;
+        need = std::max({need, lbm_nn_wgrad_workspace(B, H, H, ci, co), lbm_nn_colsum_workspace((int64_t)B * H * H, co)});
+    }
+    NN_REQUIRE(n.ws_elems >= need, "lbm_nn_unet_backward: workspace too small (%lld < %lld)", (long long)n.ws_elems,
+               (long long)need);
     for (int k = 0; k < 14; ++k)
         NN_DO(lbm_nn_flip_weights(at16(n.pb, n.off[k][0]), (char *)n.wt + 2 * n.off[k][0], n.ch[k][1], n.ch[k][0],
                                   stream));
