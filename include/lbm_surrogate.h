@@ -148,9 +148,14 @@ int lbm_nn_unet_backward(const lbm_nn_unet *net, void *stream);
 int lbm_nn_set_tensor_path(int32_t path);
 int lbm_nn_get_tensor_path(void);
 
-/* Number of tcgen05 convolution blocks that gave up on a bounded wait (their
- * output is then incomplete); reset != 0 clears the count.  Synchronous. */
+/* Number of tcgen05 convolution and weight-gradient blocks on the current device
+ * that gave up on a bounded wait; reset != 0 clears the count.  Synchronous.  Such
+ * a block stores NaN in place of its results. */
 int lbm_nn_timeouts(int32_t *count, int32_t reset);
+
+/* The limit of those waits on the current device, in GPU clock cycles; 0 restores
+ * the default (2e9, about 1 s).  For tests of the error path. */
+int lbm_nn_set_wait_limit(int64_t cycles);
 
 /* Round FP32 to bf16 (n elements). */
 int lbm_nn_to_bf16(const float *x, void *y, int64_t n, void *stream);

@@ -862,12 +862,14 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 // a training step: mma.sync kernel 1.64 ms, with copies by all threads 1.01 ms,
 // this kernel 0.86 ms; 256 -> 256 at 16 x 16, batch 1: 53, 24 and 14 us.
 // Every mbarrier wait is bounded; on timeout the CTA counts the event in
-// g_nn_timeouts (read by lbm_nn_timeouts), waits (bounded) for its own MMAs,
-// frees its tensor memory and returns.
+// g_nn_timeouts (read by lbm_nn_timeouts), waits (bounded) for its own copies and
+// MMAs, stores NaN in place of its results, so that nothing downstream takes what an
+// earlier call left there for an answer, frees its tensor memory and returns.
 constexpr int TBM = 128, TBK = 32, TTHREADS = 256;
 constexpr int TTW = 8, TTH = 16, THW = TTW + 2, THP = THW * (TTH + 2);  // pixel tile, its border, their pixels
 constexpr long long kNnWaitCycles = 2000000000LL;  // ~1 s at 1.9 GHz
 __device__ int g_nn_timeouts;
+__device__ long long g_nn_wait_limit = kNnWaitCycles;  // lbm_nn_set_wait_limit
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -889,13 +891,44 @@ __device__ __forceinline__ bool nn_mbar_test(uint64_t *b, uint32_t parity)
     return ok != 0;
 }
 
-__device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity)
+// try_wait may suspend the thread for a while; limits below this poll with test_wait, so that they can run out before
+// a copy in flight lands (the error path's test)
+constexpr long long kNnShortWait = 1000000LL;
+
+__device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity, long long limit = kNnWaitCycles)
 {
-    if (nn_mbar_test(b, parity)) return true;
     const long long t0 = clock64();
+    if (limit < kNnShortWait) {
+        uint32_t ok = 0;
+        while (true) {
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}\n"
+                : "=r"(ok)
+                : "r"(smem_u32(b)), "r"(parity)
+                : "memory");
+            if (ok) return true;
+            if (clock64() - t0 > limit) return false;
+        }
+    }
     while (!nn_mbar_test(b, parity))
-        if (clock64() - t0 > kNnWaitCycles) return false;
+        if (clock64() - t0 > limit) return false;
     return true;
+}
+
+// a block that gave up: the last `stages` of the `copies` its copying thread (tid 32) issued, and the MMAs of the
+// `chunks` its issuing thread (tid 0) committed, end before the memory they use is released
+__device__ __forceinline__ void nn_drain(int tid, uint64_t *full, uint64_t *bars, int stages, int copies, int chunks)
+{
+    if (tid == 32)
+        for (int k = copies > stages ? copies - stages : 0; k < copies; ++k)
+            nn_mbar_wait(&full[k % stages], uint32_t((k / stages) & 1));
+    if (tid == 0) {
+        if (chunks > 0) nn_mbar_wait(&bars[(chunks - 1) % stages], uint32_t(((chunks - 1) / stages) & 1));
+        atomicAdd(&g_nn_timeouts, 1);
+    }
+    __syncthreads();
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -998,6 +1031,7 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n0 = blockIdx.y * BN;
     const int nk = a.Cin / TBK;
+    const long long limit = g_nn_wait_limit;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -1029,11 +1063,11 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
 
     constexpr uint32_t idesc = umma_idesc<BN>();
     bool fail = false;
+    int kc = 0;  // chunks this thread has issued
     if (tid == 32) {  // the copies
-        int kc = 0;
         for (; kc < nk; ++kc) {
             const int st = kc % NST;
-            if (kc >= NST && !nn_mbar_wait(&bars[st], uint32_t((kc / NST - 1) & 1))) {
+            if (kc >= NST && !nn_mbar_wait(&bars[st], uint32_t((kc / NST - 1) & 1), limit)) {
                 fail = true;
                 break;
             }
@@ -1044,12 +1078,9 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
                     t / (ntx * nty));
             nn_tma3(base + Lt::BOFF, &wmap, &full[st], kc * TBK, n0, 0);
         }
-        if (fail)  // copies still in flight land before the shared memory is released
-            for (int k = kc > NST ? kc - NST : 0; k < kc; ++k) nn_mbar_wait(&full[k % NST], uint32_t((k / NST) & 1));
     } else if (tid == 0) {  // the MMAs
-        int kc = 0;
         for (; kc < nk; ++kc) {
-            if (!nn_mbar_wait(&full[kc % NST], uint32_t((kc / NST) & 1))) {
+            if (!nn_mbar_wait(&full[kc % NST], uint32_t((kc / NST) & 1), limit)) {
                 fail = true;
                 break;
             }
@@ -1076,18 +1107,15 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
                              smem_u32(&bars[kc % NST]))
                          : "memory");
         }
-        // the MMAs that were issued complete before the tensor memory is freed
-        if (fail && kc > 0) nn_mbar_wait(&bars[(kc - 1) % NST], uint32_t(((kc - 1) / NST) & 1));
     }
     __syncwarp();
     // every MMA of this CTA is complete once the commit of the last chunk arrives
     // (for tid 0, which has seen the stage's earlier use complete; the others go by the block barrier)
-    const bool done = nn_mbar_wait(&bars[(nk - 1) % NST], uint32_t(((nk - 1) / NST) & 1));
+    const bool done = nn_mbar_wait(&bars[(nk - 1) % NST], uint32_t(((nk - 1) / NST) & 1), limit);
     const bool bad = __syncthreads_or(fail || !done);
     tc_fence_after();
-    if (bad) {
-        if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
-    } else {
+    if (bad) nn_drain(tid, full, bars, NST, kc, kc);
+    {
         // warp w reads TMEM lanes 32 (w % 4) ..: pixels 4 tile rows; two warpgroups split the channel slices
         const int wg = warp >> 2;
         const int t = blockIdx.x;
@@ -1103,7 +1131,7 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
             if (!px || n >= a.Cout) continue;
             float z[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]) + sbias[sl * 16 + j];
+            for (int j = 0; j < 16; ++j) z[j] = bad ? NAN : __uint_as_float(r[j]) + sbias[sl * 16 + j];
             if (vec && n + 16 <= a.Cout) {
                 if (a.of) {
                     float *p = a.of + m * a.os + a.oo + n;
@@ -1242,6 +1270,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
     const int c0 = blockIdx.x * 32, co0 = blockIdx.y * TBM;
     const int t0 = blockIdx.z * per, nt = min(per, ntiles - t0);  // at least one tile
     const int atoms = min(4, (Cout - co0 + 31) / 32);
+    const long long limit = g_nn_wait_limit;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -1271,11 +1300,11 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
     // FP32 accumulators, bf16 A and B, both channel-major, M = 128, N = 96
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (12u << 17) | (8u << 24);
     bool fail = false;
+    int k = 0;  // tiles this thread has issued
     if (tid == 32) {  // the copies
-        int k = 0;
         for (; k < nt; ++k) {
             const int st = k % WST, t = t0 + k;
-            if (k >= WST && !nn_mbar_wait(&bars[st], uint32_t((k / WST - 1) & 1))) {
+            if (k >= WST && !nn_mbar_wait(&bars[st], uint32_t((k / WST - 1) & 1), limit)) {
                 fail = true;
                 break;
             }
@@ -1285,12 +1314,9 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
             for (int a = 0; a < atoms; ++a) nn_tma4(base + a * WA_ATOM, &zmap, &full[st], co0 + a * 32, x0, y0, b);
             nn_tma4(base + WA, &xmap, &full[st], c0, x0 - 1, y0 - 1, b);
         }
-        if (fail)  // copies still in flight land before the shared memory is released
-            for (int j = k > WST ? k - WST : 0; j < k; ++j) nn_mbar_wait(&full[j % WST], uint32_t((j / WST) & 1));
     } else if (tid == 0) {  // the MMAs
-        int k = 0;
         for (; k < nt; ++k) {
-            if (!nn_mbar_wait(&full[k % WST], uint32_t((k / WST) & 1))) {
+            if (!nn_mbar_wait(&full[k % WST], uint32_t((k / WST) & 1), limit)) {
                 fail = true;
                 break;
             }
@@ -1316,16 +1342,14 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
                              smem_u32(&bars[k % WST]))
                          : "memory");
         }
-        if (fail && k > 0) nn_mbar_wait(&bars[(k - 1) % WST], uint32_t(((k - 1) / WST) & 1));
     }
     __syncwarp();
     // every MMA of this block is complete once the commit of the last tile arrives
-    const bool done = nn_mbar_wait(&bars[(nt - 1) % WST], uint32_t(((nt - 1) / WST) & 1));
+    const bool done = nn_mbar_wait(&bars[(nt - 1) % WST], uint32_t(((nt - 1) / WST) & 1), limit);
     const bool bad = __syncthreads_or(fail || !done);
     tc_fence_after();
-    if (bad) {
-        if (tid == 0) atomicAdd(&g_nn_timeouts, 1);
-    } else {
+    if (bad) nn_drain(tid, full, bars, WST, k, k);
+    {
         // a lane one output channel; two warpgroups split the 18 slices of 16 columns
         const int co = co0 + (warp & 3) * 32 + lane;
         float *o = ws + ((int64_t)blockIdx.z * Cout + co) * 9 * Cin + c0;
@@ -1336,7 +1360,7 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
             if (co >= Cout) continue;
             float z[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]);
+            for (int j = 0; j < 16; ++j) z[j] = bad ? NAN : __uint_as_float(r[j]);
             float *q = o + (int64_t)(sl >> 1) * Cin + (sl & 1) * 16;
             if (vec) {
                 st_v8(q, z);
@@ -1708,6 +1732,15 @@ extern "C" int lbm_nn_timeouts(int32_t *count, int32_t reset)
     }
     if (e != cudaSuccess) return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_timeouts: %s", cudaGetErrorString(e));
     *count = v;
+    return LBM_OK;
+}
+
+extern "C" int lbm_nn_set_wait_limit(int64_t cycles)
+{
+    NN_REQUIRE(cycles >= 0, "lbm_nn_set_wait_limit: the limit must be >= 0");
+    const long long v = cycles > 0 ? cycles : kNnWaitCycles;
+    const cudaError_t e = cudaMemcpyToSymbol(g_nn_wait_limit, &v, sizeof v);
+    if (e != cudaSuccess) return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_set_wait_limit: %s", cudaGetErrorString(e));
     return LBM_OK;
 }
 

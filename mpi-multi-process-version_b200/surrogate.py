@@ -61,6 +61,7 @@ _SIGS = {
     "lbm_nn_set_tensor_path": [_i32],
     "lbm_nn_get_tensor_path": [],
     "lbm_nn_timeouts": [_dp, _i32],
+    "lbm_nn_set_wait_limit": [_i64],
 }
 NN_EXPORTS = list(_SIGS)
 
@@ -79,6 +80,12 @@ def timeouts(reset=False):
     c = ctypes.c_int32()
     _chk(nn().lbm_nn_timeouts(ctypes.byref(c), int(bool(reset))), "lbm_nn_timeouts")
     return int(c.value)
+
+
+def set_wait_limit(cycles):
+    """Limit of the convolutions' bounded waits on the current device (0: the default)."""
+    _chk(nn().lbm_nn_set_wait_limit(int(cycles)), "lbm_nn_set_wait_limit")
+
 
 _bound = False
 
@@ -293,6 +300,18 @@ class Net:
         b = self.buffers(B)
         _chk(nn().lbm_nn_unet_backward(ctypes.byref(self._unet(b, B, True)), self._s()), "backward")
         self.launches += 14 + 3 + 13 * 5 + 4 + 3 + 3
+
+    def check(self):
+        """Raise if a convolution or weight gradient on this device gave up on a
+        bounded wait since the last check: its results are NaN then, and so is
+        what was computed from them.  Call it where the host waits for the
+        results anyway; it synchronises."""
+        with self.torch.cuda.device(self.dev):
+            self.torch.cuda.current_stream(self.dev).synchronize()
+            n = timeouts(reset=True)
+        if n:
+            raise L.LBMError(-5, "Net.check",  # LBM_ERR_TIMEOUT
+                             f"{n} convolution blocks gave up on a bounded wait; their results are NaN")
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8, wd=0.0):
         self.t += 1

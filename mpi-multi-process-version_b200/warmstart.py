@@ -193,6 +193,7 @@ class WarmStart:
             self.net.adam(lr_t)
             if (it + 1) % log_every == 0 or it == steps - 1:
                 val = float(loss.item())
+                self.net.check()
                 hist.append((it + 1, val))
                 if log:
                     log(f"step {it + 1:6d}  loss {val:.5f}  lr {lr_t:.2e}  {time.perf_counter() - t0:.1f}s")
@@ -218,6 +219,7 @@ class WarmStart:
             xb = self._device_inputs(X[k:k + batch])
             y = self.net.forward(xb).reshape(xb.shape[0], self.R, self.R, 3)
             out[k:k + xb.shape[0]] = y.cpu().numpy()
+        self.net.check()
         return out * self.std + self.mean
 
     def predict_fields(self, cases):
