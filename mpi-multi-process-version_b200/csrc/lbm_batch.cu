@@ -3,7 +3,8 @@
 // The reference runs one cavity per program (natural-convection_2dim_mono.f90
 // `program main`, 283-380).  A batch holds many cavities of different size and
 // parameters and advances all of them at once:
-//   * 2D batches: one persistent TMA march kernel per step (k_march2d_batch)
+//   * 2D batches: one persistent TMA march kernel per launch (k_march2d_batch, one step;
+//     k_march2d_levels_batch, two or four)
 //     walks a work list of segments -- (cavity, column strip, row range) --
 //     that splits the total work into equal contiguous shares, one per block;
 //     the per-cavity geometry, TMA descriptors and buffers come from tables
@@ -60,7 +61,8 @@ struct lbm_batch {
     int levels = 1;                // time steps a 2D multi-step launch advances (fast build)
     int pdl = 1;                   // LBM_BATCH_OPT_PDL: programmatic dependent launch of the step kernels
     Geo *d_geo = nullptr;
-    TmapSet *d_maps = nullptr;
+    TmapSet *d_maps = nullptr;     // of every member's two buffers, for the one-level kernels
+    TmapSet *d_rows = nullptr;     // and for the fast build's 2D kernels of several levels
     Bufs *d_bufs = nullptr;
     // one work list per population storage (members may differ while a
     // mixed-precision run hands them from FP32 to FP64 one by one)
@@ -68,9 +70,11 @@ struct lbm_batch {
         int4 *d_segs = nullptr;
         int *d_segoff = nullptr;
         size_t segs_cap = 0, segoff_cap = 0;
-        int nblocks = 0;   // the list's grid (fixed while graphs replay it)
-        int tx = 0;        // the tile width its kernel was captured with
-        BatchDev dev{};
+        // per launch of 1, 2 and 4 steps: grid (fixed while graphs replay it) and plan
+        int nblocks[3] = {0, 0, 0};
+        int tx = 0;        // the tile width its kernels were captured with
+        BatchDev dev[3]{};
+        bool present() const { return nblocks[0] > 0; }
     } wl[2];
     bool run_both = false;         // a mixed run: both storages' kernels launch every step
     cudaStream_t stream2 = nullptr;  // the second branch when both storages' kernels run
@@ -103,7 +107,7 @@ static int batch_levels(const lbm_batch *b)
     return b->storage == LBM_STORE_F32 && nodes >= (1 << 21) ? 2 : 4;
 }
 
-// the kernel's columns for a tile width: the fast build's rows have 64 or 128
+// the multi-level kernel's columns for a tile width: its rows have 64 or 128
 // (tile 32 caps the strips at 32 of the 64)
 static int W_cols(int tile) { return tile < 64 ? 64 : tile; }
 
@@ -128,7 +132,7 @@ extern "C" int lbm_batch_destroy(lbm_batch *b)
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graphs(b);
     for (lbm_handle *h : b->cav) lbm_destroy(h);
-    void *ptrs[] = {b->d_geo, b->d_maps,        b->d_bufs,         b->d_err,        b->d_ctl,
+    void *ptrs[] = {b->d_geo, b->d_maps, b->d_rows,       b->d_bufs,         b->d_err,        b->d_ctl,
                     b->d_idx, b->wl[0].d_segs,  b->wl[0].d_segoff, b->wl[1].d_segs, b->wl[1].d_segoff};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -202,6 +206,8 @@ extern "C" int lbm_batch_create(int32_t n, const lbm_params *params, const doubl
         cudaError_t e = cudaMalloc(&b->d_geo, sizeof(Geo) * n);
         if (e == cudaSuccess) e = cudaMalloc(&b->d_bufs, sizeof(Bufs) * n);
         if (e == cudaSuccess) e = cudaMalloc(&b->d_maps, sizeof(TmapSet) * 2 * n);
+        if (e == cudaSuccess && b->dim == 2 && b->mode != LBM_MODE_EXACT)
+            e = cudaMalloc(&b->d_rows, sizeof(TmapSet) * 2 * n);
         if (e == cudaSuccess) e = cudaMalloc(&b->d_err, 16);
         if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, 16);
         if (e != cudaSuccess) return bail(set_error(LBM_ERR_NOMEM, "batch tables: %s", cudaGetErrorString(e)));
@@ -236,11 +242,15 @@ static int build_tables(lbm_batch *b)
 {
     const bool d3 = b->dim == 3;
     const int TX = d3 ? 32 : b->tile;
-    std::vector<TmapSet> maps(2 * (size_t)b->n);
+    const bool fast2d = !d3 && b->mode != LBM_MODE_EXACT;
+    std::vector<TmapSet> maps(2 * (size_t)b->n), rows(fast2d ? 2 * (size_t)b->n : 0);
     for (int i = 0; i < b->n; ++i)
-        if (!encode_maps_tx(b->cav[i], d3 ? 0 : (b->mode == LBM_MODE_EXACT ? TX : W_cols(TX)), &maps[2 * (size_t)i]))
+        if (!encode_maps_tx(b->cav[i], d3 ? 0 : TX, &maps[2 * (size_t)i]) ||
+            (fast2d && !encode_rows(b->cav[i], W_cols(TX), &rows[2 * (size_t)i])))
             return set_error(LBM_ERR_UNSUPPORTED, "batch: TMA descriptors for cavity %d could not be encoded", i);
     BCU(cudaMemcpyAsync(b->d_maps, maps.data(), sizeof(TmapSet) * maps.size(), cudaMemcpyHostToDevice, b->stream));
+    if (fast2d)
+        BCU(cudaMemcpyAsync(b->d_rows, rows.data(), sizeof(TmapSet) * rows.size(), cudaMemcpyHostToDevice, b->stream));
     {
         // the members' buffers (a storage change gives a member new ones)
         std::vector<Bufs> bufs(b->n);
@@ -248,23 +258,23 @@ static int build_tables(lbm_batch *b)
         BCU(cudaMemcpyAsync(b->d_bufs, bufs.data(), sizeof(Bufs) * b->n, cudaMemcpyHostToDevice, b->stream));
     }
 
-    const bool fast2d = !d3 && b->mode != LBM_MODE_EXACT;
+    bool regraph = b->levels != batch_levels(b);
     b->levels = batch_levels(b);
     struct Col {
         int cav, pos, ny;  // pos: 2D the strip's x-offset, 3D the tile index; ny: items (rows or slices)
     };
     std::vector<Col> cols;
-    std::vector<Strip2> strips;
+    std::vector<Strip2> strips[3];  // of the active members, per launch of 2 and 4 steps ([1], [2])
     size_t ncols_all = 0;  // the columns of every member, active or not: the lists' capacity
     b->active_nodes = 0;
     for (int i = 0; i < b->n; ++i) {
         const Geo &g = b->cav[i]->geo;
-        int nc = d3 ? ((g.nx + 31) / 32) * ((g.ny + kBatchTileY - 1) / kBatchTileY) : (g.nx + TX - 1) / TX;
-        if (fast2d) {
-            const size_t n0 = strips.size();
-            strips_march2d(i, g.nx, 0, g.ny, g.ny, TX, b->levels, strips);
-            nc = (int)(strips.size() - n0);
-            if (!b->active[i]) strips.resize(n0);
+        const int nc = d3 ? ((g.nx + 31) / 32) * ((g.ny + kBatchTileY - 1) / kBatchTileY) : (g.nx + TX - 1) / TX;
+        for (int l = 1; 1 << l <= b->levels; ++l) {
+            const size_t n0 = strips[l].size();
+            strips_march2d(i, g.nx, 0, g.ny, g.ny, TX, 1 << l, strips[l]);
+            ncols_all += strips[l].size() - n0;
+            if (!b->active[i]) strips[l].resize(n0);
         }
         ncols_all += nc;
         if (!b->active[i]) continue;
@@ -273,7 +283,6 @@ static int build_tables(lbm_batch *b)
     }
     int sms = 0;
     BCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
-    bool regraph = false;
     b->nblocks = 0;
     for (int sto = 0; sto < 2; ++sto) {
         lbm_batch::WorkList &W = b->wl[sto];
@@ -285,47 +294,63 @@ static int build_tables(lbm_batch *b)
                 sc.push_back(c);
                 stotal += c.ny;
             }
-        const bool present = !sc.empty() || (b->run_both && b->mode != LBM_MODE_EXACT);
-        if (!present) {
-            if (W.nblocks) regraph = true;
-            W.nblocks = 0;
+        bool members = false;
+        for (int i = 0; i < b->n; ++i) members = members || (b->active[i] && b->cav[i]->p.storage == sto);
+        if (!members && !(b->run_both && b->mode != LBM_MODE_EXACT)) {
+            if (W.present()) regraph = true;
+            for (int &nb : W.nblocks) nb = 0;
             continue;
         }
-        const int bps = d3 ? (b->mode == LBM_MODE_EXACT ? exact::march_batch3d_blocks_per_sm(sto)
-                                                         : fast::march_batch3d_blocks_per_sm(sto))
-                           : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(sto, TX, 1)
-                                                        : fast::march_batch_blocks_per_sm(sto, W_cols(TX), b->levels));
-        if (bps <= 0) return set_error(LBM_ERR_UNSUPPORTED, "batch kernel with tile %d cannot be resident", TX);
-        const int64_t G = b->nblocks_opt > 0 ? b->nblocks_opt : (int64_t)bps * sms;
         // equal contiguous shares of the (column, item) items; blocks past the work get none
         std::vector<int4> segs;
-        std::vector<int> off(G + 1, 0);
-        if (fast2d) {
-            std::vector<Strip2> mine;
-            for (const Strip2 &st : strips)
-                if (b->cav[st.cav]->p.storage == sto) mine.push_back(st);
-            plan_march2d(mine, b->levels, (int)G, segs, off);
-            sc.clear();
-            stotal = 0;
+        std::vector<int> off;
+        size_t off0[3] = {0, 0, 0};
+        int grid[3] = {0, 0, 0}, bps[3] = {0, 0, 0};
+        for (int l = 0; 1 << l <= b->levels; ++l) {
+            bps[l] = d3 ? (b->mode == LBM_MODE_EXACT ? exact::march_batch3d_blocks_per_sm(sto)
+                                                     : fast::march_batch3d_blocks_per_sm(sto))
+                        : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(sto, TX, 1)
+                                                     : fast::march_batch_blocks_per_sm(sto, l ? W_cols(TX) : TX, 1 << l));
+            if (bps[l] <= 0) return set_error(LBM_ERR_UNSUPPORTED, "batch kernel with tile %d cannot be resident", TX);
         }
-        size_t c = 0;
-        int64_t colbase = 0;  // first item of column c
-        for (int64_t blk = 0; blk < G && !fast2d; ++blk) {
-            off[blk] = (int)segs.size();
-            const int64_t lo = stotal * blk / G, hi = stotal * (blk + 1) / G;
-            int64_t u = lo;
-            while (u < hi) {
-                while (c < sc.size() && colbase + sc[c].ny <= u) colbase += sc[c++].ny;
-                const int64_t end = std::min<int64_t>(hi, colbase + sc[c].ny);
-                if (d3)
-                    segs.push_back(make_int4(sc[c].pos, (int)(u - colbase), (int)(end - colbase), sc[c].cav));
-                else
-                    segs.push_back(make_int4(sc[c].cav, sc[c].pos, (int)(u - colbase), (int)(end - colbase)));
-                u = end;
+        const int top = b->levels >> 1;  // the launches of most steps
+        for (int l = 0; 1 << l <= b->levels; ++l) {
+            // a grid that was set is the multi-step launches'; the others, whose blocks are smaller, get the same
+            // share of what the SMs hold
+            const int64_t G = b->nblocks_opt > 0 ? std::max<int64_t>(1, (int64_t)b->nblocks_opt * bps[l] / bps[top])
+                                                 : (int64_t)bps[l] * sms;
+            grid[l] = (int)G;
+            off0[l] = off.size();
+            if (l > 0) {
+                std::vector<Strip2> mine;
+                for (const Strip2 &st : strips[l])
+                    if (b->cav[st.cav]->p.storage == sto) mine.push_back(st);
+                std::vector<int4> sg;
+                std::vector<int> of;
+                plan_march2d(mine, 1 << l, (int)G, sg, of);
+                for (int o : of) off.push_back(o + (int)segs.size());
+                segs.insert(segs.end(), sg.begin(), sg.end());
+                continue;
             }
+            size_t c = 0;
+            int64_t colbase = 0;  // first item of column c
+            for (int64_t blk = 0; blk < G; ++blk) {
+                off.push_back((int)segs.size());
+                const int64_t lo = stotal * blk / G, hi = stotal * (blk + 1) / G;
+                int64_t u = lo;
+                while (u < hi) {
+                    while (c < sc.size() && colbase + sc[c].ny <= u) colbase += sc[c++].ny;
+                    const int64_t end = std::min<int64_t>(hi, colbase + sc[c].ny);
+                    if (d3)
+                        segs.push_back(make_int4(sc[c].pos, (int)(u - colbase), (int)(end - colbase), sc[c].cav));
+                    else
+                        segs.push_back(make_int4(sc[c].cav, sc[c].pos, (int)(u - colbase), (int)(end - colbase)));
+                    u = end;
+                }
+            }
+            off.push_back((int)segs.size());
         }
-        off[G] = (int)segs.size();
-        const size_t seg_need = (size_t)G + ncols_all + 16;
+        const size_t seg_need = off.size() + ncols_all + 16;
         if (W.segs_cap < seg_need) {
             if (W.d_segs) cudaFree(W.d_segs);
             W.d_segs = nullptr;
@@ -344,11 +369,14 @@ static int build_tables(lbm_batch *b)
             BCU(cudaMemcpyAsync(W.d_segs, segs.data(), sizeof(int4) * segs.size(), cudaMemcpyHostToDevice,
                                 b->stream));
         BCU(cudaMemcpyAsync(W.d_segoff, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, b->stream));
-        if (W.nblocks != (int)G || W.tx != TX) regraph = true;
-        W.nblocks = (int)G;
+        for (int l = 0; l < 3; ++l) {
+            if (W.nblocks[l] != grid[l]) regraph = true;
+            W.nblocks[l] = grid[l];
+            W.dev[l] = BatchDev{b->d_geo, l ? b->d_rows : b->d_maps, b->d_bufs, W.d_segs, W.d_segoff + off0[l]};
+        }
+        if (W.tx != TX) regraph = true;
         W.tx = TX;
-        W.dev = BatchDev{b->d_geo, b->d_maps, b->d_bufs, W.d_segs, W.d_segoff};
-        b->nblocks += (int)G;
+        b->nblocks += grid[top];
     }
     BCU(cudaStreamSynchronize(b->stream));
     b->dev = BatchDev{b->d_geo, b->d_maps, b->d_bufs, nullptr, nullptr};
@@ -363,12 +391,13 @@ static int build_tables(lbm_batch *b)
 static cudaError_t launch_list(lbm_batch *b, int sto, int cur, int wm, int levels, bool pdl, cudaStream_t s)
 {
     const lbm_batch::WorkList &W = b->wl[sto];
+    const BatchDev &D = W.dev[levels >> 1];
+    const int G = W.nblocks[levels >> 1];
     if (b->dim == 3)
-        return b->mode == LBM_MODE_EXACT ? exact::march_batch3d(sto, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s)
-                                         : fast::march_batch3d(sto, W.dev, W.nblocks, cur, wm, b->d_err, pdl, s);
-    return b->mode == LBM_MODE_EXACT ? exact::march_batch(sto, W.tx, W.dev, W.nblocks, cur, wm, b->d_err, pdl, 1, s)
-                                     : fast::march_batch(sto, W_cols(W.tx), W.dev, W.nblocks, cur, wm, b->d_err, pdl,
-                                                         levels, s);
+        return b->mode == LBM_MODE_EXACT ? exact::march_batch3d(sto, D, G, cur, wm, b->d_err, pdl, s)
+                                         : fast::march_batch3d(sto, D, G, cur, wm, b->d_err, pdl, s);
+    if (b->mode == LBM_MODE_EXACT) return exact::march_batch(sto, W.tx, D, G, cur, wm, b->d_err, pdl, 1, s);
+    return fast::march_batch(sto, levels > 1 ? W_cols(W.tx) : W.tx, D, G, cur, wm, b->d_err, pdl, levels, s);
 }
 
 // with both storages present the two kernels run side by side (a fork onto
@@ -376,7 +405,7 @@ static cudaError_t launch_list(lbm_batch *b, int sto, int cur, int wm, int level
 // single list's kernels follow one another as programmatic dependents
 static cudaError_t launch_step(lbm_batch *b, int cur, int wm, int levels = 1)
 {
-    const bool a = b->wl[0].nblocks > 0, c = b->wl[1].nblocks > 0;
+    const bool a = b->wl[0].present(), c = b->wl[1].present();
     if (a && c) {
         cudaError_t e = cudaEventRecord(b->ev_fork, b->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream2, b->ev_fork, 0);
@@ -391,20 +420,19 @@ static cudaError_t launch_step(lbm_batch *b, int cur, int wm, int levels = 1)
     return cudaSuccess;
 }
 
-// n steps from buffer `cur`, which ends at (cur + n) & 1: pairs of multi-step
-// launches (each flips the buffers once for its even number of steps), then
-// single steps, the last one alone with the macroscopic fields if with_macro
+// n steps from buffer `cur`, which ends at (cur + n) & 1 (launches_2d), the last
+// one alone with the macroscopic fields if with_macro
 static cudaError_t launch_steps(lbm_batch *b, int cur, int n, bool with_macro)
 {
     int left = with_macro ? n - 1 : n;
-    const int group = 2 * b->levels;
+    const Launches l = launches_2d(left, b->levels);
     cudaError_t e = cudaSuccess;
-    if (b->levels > 1)
-        for (; left >= group && e == cudaSuccess; left -= group)
-            for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-                e = launch_step(b, cur, 0, b->levels);
-                cur = 1 - cur;
-            }
+    for (int k = 0; k < l.four + l.two && e == cudaSuccess; ++k) {
+        const int T = k < l.four ? 4 : 2;
+        e = launch_step(b, cur, 0, T);
+        left -= T;
+        cur = 1 - cur;
+    }
     for (; left > 0 && e == cudaSuccess; --left) {
         e = launch_step(b, cur, 0);
         cur = 1 - cur;

@@ -318,15 +318,14 @@ static EncodeTiledFn encode_fn()
 void *lbm::tensor_map_encoder() { return (void *)encode_fn(); }
 
 // Describe a population buffer as a (x, y, [z,] plane) tensor; one descriptor
-// per box class of the march kernel.  Returns false if TMA cannot be used.
-bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
+// per box class of the march kernel, or (wb > 0) of boxes of wb columns of all
+// planes of a row.  Returns false if TMA cannot be used.
+static bool encode_boxes(const lbm_handle *h, int tx, int wb, TmapSet out[2])
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
     const Geo &g = h->geo;
     const MarchShape ms = march_shape(g.dim, h->p.storage, tx, h->tiley);
-    // the fast build's 2D march: one box of all planes per row
-    const int wb = g.dim == 2 && h->p.mode != LBM_MODE_EXACT ? march2d_box(h->p.storage, tx ? tx : h->nt) : 0;
     const bool pairs = g.dim == 3 && h->p.mode != LBM_MODE_EXACT;
     const CUtensorMapDataType dtype =
         h->p.storage == LBM_STORE_F64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
@@ -384,6 +383,13 @@ bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2])
         if (r != CUDA_SUCCESS) return false;
     }
     return true;
+}
+
+bool lbm::encode_maps_tx(const lbm_handle *h, int tx, TmapSet out[2]) { return encode_boxes(h, tx, 0, out); }
+
+bool lbm::encode_rows(const lbm_handle *h, int nt, TmapSet out[2])
+{
+    return encode_boxes(h, 0, march2d_box(h->p.storage, nt), out);
 }
 
 static bool encode_maps(lbm_handle *h) { return lbm::encode_maps_tx(h, 0, h->tmaps); }
@@ -496,6 +502,20 @@ void lbm::strips_march2d(int cav, int nx, int lo, int hi, int ny, int nt, int le
     int S = std::max(1, nx / nt);
     while (!fits(S)) ++S;
     for (int k = 0; k < S; ++k) out.push_back({cav, cut(k, S), cut(k + 1, S) - cut(k, S), lo, hi, ny});
+}
+
+lbm::Launches lbm::launches_2d(int n, int levels)
+{
+    Launches l{0, 0};
+    const int h = n / 2;  // pairs of steps; an even number of launches takes them
+    if (levels == 4) {
+        l.four = h / 2 - (h / 2 + h) % 2;
+        l.two = h - 2 * l.four;
+        if (l.four < 0) l = {0, 0};
+    } else if (levels == 2) {
+        l.two = h - h % 2;
+    }
+    return l;
 }
 
 int lbm::plan_march2d(const std::vector<Strip2> &strips, int levels, int nblocks, std::vector<int4> &segs,
@@ -652,6 +672,8 @@ static int upload_plan3d(lbm_handle *h, int G)
 // 64x4 / 128x2 / 64x2): 384^2 6.9 / 7.8 / 7.2, 700x900 18.4 / 18.5 / 19.7, 1024^2
 // 29.0 / 28.2 / 30.1, 2048^2 108 / 112 / 106; FP32: 512^2 7.7 / 8.0 / 8.2, 1023x771
 // 17.3 / 16.9 / 17.7, 2048^2 89 / 77 / 79.
+// Two levels have a grid and a plan of their own, as single steps have (a grid made
+// for four levels' blocks leaves their SMs half empty).
 static int resolve_2d(lbm_handle *h)
 {
     const Geo &g = h->geo;
@@ -659,41 +681,48 @@ static int resolve_2d(lbm_handle *h)
     const bool f64 = h->p.storage == LBM_STORE_F64;
     const int levels = slab ? 1 : (g.nnode < (1 << 19) ? 4 : 2);
     const int nt = g.nnode < (1 << 19) || (f64 && g.nnode >= (1 << 21)) ? 64 : 128;
-    const int bps = fast::march_blocks_per_sm(g, h->p.storage, h->tiley, nt, levels);
-    if (bps <= 0 || fast::march_blocks_per_sm(g, h->p.storage, h->tiley, nt, 1) <= 0) {
-        h->levels = 0;
-        return LBM_OK;
-    }
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    h->nt = nt;
-    h->levels = levels;
-    h->slots = h->nblocks_opt > 0 ? h->nblocks_opt : bps * sms;
+    for (March2d &m : h->m2) m = March2d{};
     h->sms = sms;
-    h->segs2.clear();
-    h->plan_dirty = true;  // planned by the init call or the first launch: a batch's members never need it
-    h->march_ok = lbm::encode_maps_tx(h, 0, h->tmaps);
+    for (int k = 0; 2 << k <= levels; ++k) {
+        March2d &m = h->m2[k];
+        m.nt = nt;
+        const int bps = fast::march_blocks_per_sm(g, h->p.storage, h->tiley, nt, 2 << k);
+        if (bps <= 0 || !lbm::encode_rows(h, nt, m.maps)) return LBM_OK;
+        m.slots = h->nblocks_opt > 0 ? h->nblocks_opt : bps * sms;
+        m.levels = 2 << k;
+        h->levels = m.levels;
+        h->plan_dirty = true;  // planned by the init call or the first launch: a batch's members never need it
+    }
     return LBM_OK;
 }
 
-// the plan on the host
-static void plan_2d(lbm_handle *h)
-{
-    if (!h->plan_dirty || !h->segs2.empty()) return;
-    const Geo &g = h->geo;
-    std::vector<lbm::Strip2> strips;
-    lbm::strips_march2d(0, g.nx, g.jlo, g.jhi, g.ny, h->nt, h->levels, strips);
-    h->nblocks = lbm::plan_march2d(strips, h->levels, h->slots, h->segs2, h->segoff2);
-    if (g.jlo == 0 && g.jhi == g.ny && g.nnode <= (1 << 18))
-        h->tile = lbm::plan_tile2d(g.nx, g.ny, (int)h->esize, h->sms);
-}
-
+// the plans of the launches of several steps: tiles, or the march's on the device
 static int ensure_plan(lbm_handle *h)
 {
     if (!h->plan_dirty) return LBM_OK;
-    plan_2d(h);
-    if (h->tile.T > 1 && !h->use_march) return LBM_OK;  // tiles and direct-load single steps only
-    int st = upload_segs(h, h->segs2, h->segoff2);
+    const Geo &g = h->geo;
+    if (g.jlo == 0 && g.jhi == g.ny && g.nnode <= (1 << 18))
+        h->tile = lbm::plan_tile2d(g.nx, g.ny, (int)h->esize, h->sms);
+    if (h->tile.T > 1) {
+        h->plan_dirty = false;
+        return LBM_OK;
+    }
+    std::vector<int4> segs;
+    std::vector<int> off;
+    for (March2d &m : h->m2) {
+        if (!m.levels) continue;
+        std::vector<lbm::Strip2> strips;
+        lbm::strips_march2d(0, g.nx, g.jlo, g.jhi, g.ny, m.nt, m.levels, strips);
+        std::vector<int4> sg;
+        std::vector<int> of;
+        m.nblocks = lbm::plan_march2d(strips, m.levels, m.slots, sg, of);
+        m.off0 = off.size();
+        for (int o : of) off.push_back(o + (int)segs.size());
+        segs.insert(segs.end(), sg.begin(), sg.end());
+    }
+    int st = upload_segs(h, segs, off);
     if (!st) h->plan_dirty = false;
     return st;
 }
@@ -734,15 +763,11 @@ static int resolve_path(lbm_handle *h)
     if (fast2d && ok && h->kernel_opt != 1) {
         int st = resolve_2d(h);
         if (st) return st;
-        if (!h->levels || !h->march_ok) {
-            if (h->kernel_opt == 2) return fail(LBM_ERR_UNSUPPORTED, "march kernel cannot be resident");
-            h->levels = 1;
-            h->use_march = 0;
-        }
-    } else if (h->use_march) {
+    }
+    if (h->use_march) {
         const int bps = h->p.mode == LBM_MODE_EXACT
-                            ? exact::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 128, 1)
-                            : fast::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 128, 1);
+                            ? exact::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 0, 1)
+                            : fast::march_blocks_per_sm(h->geo, h->p.storage, h->tiley, 0, 1);
         if (bps <= 0) {
             if (h->kernel_opt == 2) return fail(LBM_ERR_UNSUPPORTED, "march kernel cannot be resident");
             h->use_march = 0;
@@ -1039,11 +1064,16 @@ static cudaError_t launch_one(lbm_handle *h, int cur, int wm, int levels = 1)
     const bool ex = h->p.mode == LBM_MODE_EXACT;
     Bufs &b = h->bufs;
     const int nxt = 1 - cur;
-    if (h->use_march || levels > 1)
+    if (levels > 1) {
+        const March2d &m = h->m2[levels >> 2];
+        return fast::march(h->geo, h->p.storage, m.maps[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm, m.nblocks, 0,
+                           h->d_msegs, h->d_msegoff + m.off0, h->pdl != 0, m.nt, levels, h->stream);
+    }
+    if (h->use_march)
         return ex ? exact::march(h->geo, h->p.storage, h->tmaps[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm,
-                                 h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->nt, 1, h->stream)
+                                 h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, 0, 1, h->stream)
                   : fast::march(h->geo, h->p.storage, h->tmaps[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm,
-                                h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, h->nt, levels, h->stream);
+                                h->nblocks, h->tiley, h->d_msegs, h->d_msegoff, h->pdl != 0, 0, 1, h->stream);
     return ex ? exact::step(h->geo, h->p.storage, b.pop[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm, h->stream)
               : fast::step(h->geo, h->p.storage, b.pop[cur], b.F[cur], b.pop[nxt], b.F[nxt], b, wm, h->stream);
 }
@@ -1056,9 +1086,13 @@ static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
 {
     int left = with_macro ? n - 1 : n;
     cudaError_t e = cudaSuccess;
+    int k = 0;  // tile launches
     if (h->tile.T > 1 && !h->resident && left > 0) {
-        int k = (left + h->tile.T - 1) / h->tile.T;
+        k = (left + h->tile.T - 1) / h->tile.T;
         k += (k ^ left) & 1;
+        if (k == left && h->use_march) k = 0;  // one step each: the march is the faster there
+    }
+    if (k > 0) {
         for (; k > 0 && e == cudaSuccess; --k) {
             const int T = (left + k - 1) / k;
             Bufs &b = h->bufs;
@@ -1068,12 +1102,13 @@ static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
             cur = 1 - cur;
         }
     } else if (h->levels > 1 && !h->resident) {
-        // an even number of levels: launches in pairs
-        for (; left >= 2 * h->levels && e == cudaSuccess; left -= 2 * h->levels)
-            for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-                e = launch_one(h, cur, 0, h->levels);
-                cur = 1 - cur;
-            }
+        const lbm::Launches n = lbm::launches_2d(left, h->levels);
+        for (int k = 0; k < n.four + n.two && e == cudaSuccess; ++k) {
+            const int T = k < n.four ? 4 : 2;
+            e = launch_one(h, cur, 0, T);
+            left -= T;
+            cur = 1 - cur;
+        }
     }
     for (; left > 0 && e == cudaSuccess; --left) {
         e = launch_one(h, cur, 0);
@@ -1712,10 +1747,7 @@ extern "C" int lbm_get_option(const lbm_handle *h, int32_t option, int64_t *valu
     if (!h || !value) return fail(LBM_ERR_PARAM, "NULL argument");
     switch (option) {
     case LBM_OPT_KERNEL: *value = h->use_march ? 2 : 1; return LBM_OK;
-    case LBM_OPT_NBLOCKS:
-        if (h->use_march) plan_2d(const_cast<lbm_handle *>(h));
-        *value = h->use_march ? h->nblocks : 0;
-        return LBM_OK;
+    case LBM_OPT_NBLOCKS: *value = h->use_march ? h->nblocks : 0; return LBM_OK;
     case LBM_OPT_L2PROMO: *value = h->l2promo; return LBM_OK;
     case LBM_OPT_GRAPHS: *value = h->use_graphs; return LBM_OK;
     case LBM_OPT_RESIDENT: *value = h->resident > 0; return LBM_OK;

@@ -16,6 +16,17 @@ struct Derived {
 // ---------------------------------------------------------------------------
 // handle
 // ---------------------------------------------------------------------------
+// The fast build's 2D march at one number of time levels per launch, 2 or 4
+struct March2d {
+    int levels = 0;              // 0: not used by the handle
+    int nt = 128, slots = 0;     // columns per row, blocks the plan may use
+    int nblocks = 0;             // and the blocks it does use
+    std::vector<int4> segs;      // work plan: segments, and each block's first one in the device's table
+    std::vector<int> off;
+    size_t off0 = 0;             // where off lies in the device's table
+    lbm::TmapSet maps[2];
+};
+
 struct lbm_handle {
     using Geo = lbm::Geo;
     using Bufs = lbm::Bufs;
@@ -50,13 +61,11 @@ struct lbm_handle {
     int4 *d_msegs = nullptr;     // 3D march work plan: segments (tile, z0, z1, -)
     int *d_msegoff = nullptr;    // and each block's first segment
     size_t msegs_cap = 0, msegoff_cap = 0;
-    int nt = 128;                // 2D, fast build: columns per row of the march kernel
-    int levels = 1;              // and the time steps its multi-step launches advance
+    March2d m2[2];               // 2D, fast build: launches of 2 and 4 time steps
+    int levels = 1;              // the most steps a launch advances
     lbm::TilePlan tile{};        // T > 1: small domains step T at a time through the tile kernel instead
-    int slots = 0, sms = 0;      // blocks the march plan may use, SMs of the device
-    std::vector<int4> segs2;     // the march's work plan
-    std::vector<int> segoff2;
-    bool plan_dirty = false;     // it is not on the device yet (the first launch plans and uploads it)
+    int sms = 0;                 // SMs of the device
+    bool plan_dirty = false;     // the march's plans are not on the device yet (the first launch makes and uploads them)
     int l2promo = 0;             // LBM_OPT_L2PROMO
     int use_graphs = 1;          // LBM_OPT_GRAPHS
     int resident_opt = 0;        // LBM_OPT_RESIDENT as set (opt-in)
@@ -80,6 +89,8 @@ namespace lbm {
 // kernel with tile width tx (0: the single-cavity default); false if TMA
 // cannot be used
 bool encode_maps_tx(const lbm_handle *h, int tx, lbm::TmapSet out[2]);
+// the same for the 2D levels' rows of nt columns
+bool encode_rows(const lbm_handle *h, int nt, lbm::TmapSet out[2]);
 // the first collision of a run if h is still in its pre-collision state
 int first_collision(lbm_handle *h);
 // synchronise h's stream and report a kernel's bounded wait that gave up

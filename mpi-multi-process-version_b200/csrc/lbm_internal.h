@@ -91,8 +91,9 @@ struct Bufs {
 };
 
 // TMA descriptors of one population buffer, one per box class (the fast build's
-// 3D march: two planes a box), and of the carried-force array that goes with it
-// (right behind m: the exact build's 2D kernels index it as m[4])
+// 3D march: two planes a box; its 2D levels: m[0], a row of all planes), and of the
+// carried-force array that goes with it (right behind m: the one-level 2D kernels
+// index it as m[4])
 struct alignas(64) TmapSet {
     CUtensorMap m[4];
     CUtensorMap fmap;
@@ -104,7 +105,7 @@ struct BatchDev {
     const Geo *geo;          // [ncav]
     const TmapSet *maps;     // [ncav][2]: descriptors of pop[0], pop[1] (+ their force arrays)
     const Bufs *bufs;        // [ncav]
-    const int4 *segs;        // all segments: 2D (cavity, i0, ja, jb), the fast build's from plan_march2d;
+    const int4 *segs;        // all segments: 2D (cavity, i0, ja, jb), several levels from plan_march2d;
                              // 3D (tile, z0, z1, cavity)
     const int *seg_off;      // [nblocks + 1]
 };
@@ -147,16 +148,16 @@ constexpr int kBatchTileY = 4;
     /* fused step through the TMA-fed persistent march kernel; 3D: tile rows ty (4 or 8)  */ \
     /* and the blocks' segment lists segs[segoff[b] .. segoff[b+1]) (device memory);       */ \
     /* pdl: programmatic dependent launch (overlaps the previous kernel's tail);           */ \
-    /* 2D, fast build: segments of plan_march2d, rows of nt columns (64 or 128), levels    */ \
-    /* time steps in the one launch (1, 2 or 4; write_macro needs 1)                       */ \
+    /* levels: 1, or in the fast build's 2D 2 or 4 time steps in the one launch (segments  */ \
+    /* of plan_march2d, rows of nt columns, 64 or 128, no write_macro)                     */ \
     cudaError_t march(const Geo &g, int store, const TmapSet &src, const void *F_in,          \
                       void *pop_out, void *F_out, const Bufs &b, int write_macro, int nblocks,\
                       int ty, const int4 *segs, const int *segoff, bool pdl, int nt,          \
                       int levels, cudaStream_t s);                                            \
     /* resident blocks per SM of the march kernel (0 if it cannot launch) */                  \
     int march_blocks_per_sm(const Geo &g, int store, int ty, int nt, int levels);             \
-    /* `levels` steps of every cavity of a 2D batch (tile width TX = 32, 64 or 128; the   */  \
-    /* exact build: one step) */                                                              \
+    /* one step of every cavity of a 2D batch (tile width TX = 32, 64 or 128), or in the   */ \
+    /* fast build 2 or 4 (TX = 64 or 128)                                                  */ \
     cudaError_t march_batch(int store, int TX, const BatchDev &D, int nblocks, int cur,       \
                             int write_macro, int *err, bool pdl, int levels, cudaStream_t s); \
     int march_batch_blocks_per_sm(int store, int TX, int levels);                             \
@@ -252,6 +253,14 @@ struct Strip2 {
 // The strips of a cavity nx nodes wide for rows of nt columns and `levels` time
 // levels per launch: as few as fit, of nearly equal width.
 void strips_march2d(int cav, int nx, int lo, int hi, int ny, int nt, int levels, std::vector<Strip2> &out);
+// How n steps are split over launches of 4 (where levels is 4), 2 and 1 steps: as
+// many launches modulo 2 as steps, so that the buffers end as n single steps leave
+// them, and the steps that are left over single (two where n / 2 is odd and two
+// levels are the most; of n = 2 and 3 all).  7 = 4 + 2 + 1, 10 = 4 + 2 + 2 + 2.
+struct Launches {
+    int four, two;
+};
+Launches launches_2d(int n, int levels);
 // Work plan: the strips' rows cut into segments (cav | w << 24, x0, ja, jb) for
 // at most `nblocks` blocks so that the busiest block runs as few iterations as
 // possible (a segment costs its rows and 3 levels - 1 more).  off: each block's

@@ -1310,7 +1310,6 @@ static cudaError_t prepare_march3d()
     return cudaSuccess;
 }
 
-#if LBM_EXACT
 template <int ST, class L>
 static cudaError_t prepare_march2d()
 {
@@ -1323,13 +1322,14 @@ static cudaError_t prepare_march2d()
     }
     return cudaSuccess;
 }
-#else
+
+#if !LBM_EXACT
 template <int ST, int COLS, int T>
-static cudaError_t prepare_march2d()
+static cudaError_t prepare_levels2d()
 {
     static bool done = false;
     if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march2d<ST, COLS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(k_march2d_levels<ST, COLS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              M2<ST, COLS, T>::SMEM);
         if (e != cudaSuccess) return e;
         done = true;
@@ -1338,14 +1338,11 @@ static cudaError_t prepare_march2d()
 }
 
 // CALLT(columns, levels) of the variant asked for
-#define LBM_MARCH2D_CASES(cols, levels, CALLT)   \
+#define LBM_LEVELS2D_CASES(cols, levels, CALLT)  \
     switch ((cols) * 8 + (levels)) {             \
-    case 64 * 8 + 1: return CALLT(64, 1);        \
     case 64 * 8 + 2: return CALLT(64, 2);        \
     case 64 * 8 + 4: return CALLT(64, 4);        \
-    case 128 * 8 + 1: return CALLT(128, 1);      \
     case 128 * 8 + 2: return CALLT(128, 2);      \
-    case 128 * 8 + 4: return CALLT(128, 4);      \
     default: break;                              \
     }
 #endif
@@ -1361,43 +1358,39 @@ static int mbps3(void)
                : 0;
 }
 
-#if LBM_EXACT
 template <int ST, class L>
 static int mbps2(void)
 {
     if (prepare_march2d<ST, L>() != cudaSuccess) return 0;
     int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d<ST, L>, L::NT, L::smem()) == cudaSuccess ? n
-                                                                                                             : 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d<ST, L>, L::NT, L::smem()) == cudaSuccess ? n : 0;
 }
 
-template <int ST>
-static int mbps2d(const Geo &g, int, int)
-{
-    return g.nnode >= kDeepRingNodes ? mbps2<ST, L2d<ST>>() : mbps2<ST, L2s<ST>>();
-}
-#else
+#if !LBM_EXACT
 template <int ST, int COLS, int T>
-static int mbps2(void)
+static int mbps_levels(void)
 {
-    if (prepare_march2d<ST, COLS, T>() != cudaSuccess) return 0;
+    if (prepare_levels2d<ST, COLS, T>() != cudaSuccess) return 0;
     using M = M2<ST, COLS, T>;
     int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d<ST, COLS, T>, M::COLS * T, M::SMEM) ==
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_march2d_levels<ST, COLS, T>, M::COLS * T, M::SMEM) ==
                    cudaSuccess
                ? n
                : 0;
 }
+#endif
 
 template <int ST>
-static int mbps2d(const Geo &, int nt, int levels)
+static int mbps2d(const Geo &g, int nt, int levels)
 {
-#define CALLT(COLS, T) (mbps2<ST, COLS, T>())
-    LBM_MARCH2D_CASES(nt, levels, CALLT)
+    if (levels == 1) return g.nnode >= kDeepRingNodes ? mbps2<ST, L2d<ST>>() : mbps2<ST, L2s<ST>>();
+#if !LBM_EXACT
+#define CALLT(COLS, T) (mbps_levels<ST, COLS, T>())
+    LBM_LEVELS2D_CASES(nt, levels, CALLT)
 #undef CALLT
+#endif
     return 0;
 }
-#endif
 
 template <int ST>
 static int mbps(const Geo &g, int ty, int nt, int levels)
@@ -1426,7 +1419,6 @@ static cudaError_t launch_march3d(const Geo &g, const TmapSet &m, const void *Fi
                     (S *)pout, (C *)Fout, b, wm, rev, segs, segoff, b.err);
 }
 
-#if LBM_EXACT
 template <int ST, class L>
 static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
                                   const Bufs &b, int wm, int nblocks, bool pdl, cudaStream_t s)
@@ -1441,38 +1433,36 @@ static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, const void *Fi
                     wm, total, b.err);
 }
 
-template <int ST>
-static cudaError_t launch_2d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout, const Bufs &b,
-                             int wm, int nblocks, const int4 *, const int *, bool pdl, int, int, cudaStream_t s)
-{
-    return g.nnode >= kDeepRingNodes ? launch_march2d<ST, L2d<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s)
-                                     : launch_march2d<ST, L2s<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s);
-}
-#else
+#if !LBM_EXACT
 template <int ST, int COLS, int T>
-static cudaError_t launch_march2d(const Geo &g, const TmapSet &m, void *pout, void *Fout, const Bufs &b, int wm,
-                                  int nblocks, const int4 *segs, const int *segoff, bool pdl, cudaStream_t s)
+static cudaError_t launch_levels2d(const Geo &g, const TmapSet &m, void *pout, void *Fout, const Bufs &b, int nblocks,
+                                   const int4 *segs, const int *segoff, bool pdl, cudaStream_t s)
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
     using M = M2<ST, COLS, T>;
-    cudaError_t e = prepare_march2d<ST, COLS, T>();
+    cudaError_t e = prepare_levels2d<ST, COLS, T>();
     if (e != cudaSuccess) return e;
-    return launch_k(k_march2d<ST, COLS, T>, nblocks, M::COLS * T, M::SMEM, s, pdl, m.m[0], m.fmap, g, (S *)pout,
-                    (C *)Fout, b, wm, segs, segoff, b.err);
+    return launch_k(k_march2d_levels<ST, COLS, T>, nblocks, M::COLS * T, M::SMEM, s, pdl, m.m[0], m.fmap, g, (S *)pout,
+                    (C *)Fout, b, segs, segoff, b.err);
 }
+#endif
 
 template <int ST>
-static cudaError_t launch_2d(const Geo &g, const TmapSet &m, const void *, void *pout, void *Fout, const Bufs &b,
+static cudaError_t launch_2d(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout, const Bufs &b,
                              int wm, int nblocks, const int4 *segs, const int *segoff, bool pdl, int nt, int levels,
                              cudaStream_t s)
 {
-#define CALLT(COLS, T) (launch_march2d<ST, COLS, T>(g, m, pout, Fout, b, wm, nblocks, segs, segoff, pdl, s))
-    LBM_MARCH2D_CASES(nt, levels, CALLT)
+    if (levels == 1)
+        return g.nnode >= kDeepRingNodes ? launch_march2d<ST, L2d<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s)
+                                         : launch_march2d<ST, L2s<ST>>(g, m, Fin, pout, Fout, b, wm, nblocks, pdl, s);
+#if !LBM_EXACT
+#define CALLT(COLS, T) (launch_levels2d<ST, COLS, T>(g, m, pout, Fout, b, nblocks, segs, segoff, pdl, s))
+    LBM_LEVELS2D_CASES(nt, levels, CALLT)
 #undef CALLT
+#endif
     return cudaErrorInvalidValue;
 }
-#endif
 
 template <int ST>
 static cudaError_t launch_march(const Geo &g, const TmapSet &m, const void *Fin, void *pout, void *Fout,
@@ -1529,58 +1519,89 @@ cudaError_t tile2d(const Geo &g, int store, const void *pop_in, const void *F_in
 }
 #endif
 
-// the 2D batch kernel of COLS columns advancing T time levels (the exact build: one level)
+// the 2D batch kernel of COLS columns advancing T time levels
 template <int ST, int COLS, int T>
 struct BatchK {
 #if LBM_EXACT
-    static constexpr int threads = COLS, smem = L2<ST, COLS>::smem();
-    static auto kernel() { return k_march2d_batch<ST, COLS>; }
+    static_assert(T == 1, "one level");
 #else
     static constexpr int threads = COLS * T, smem = M2<ST, COLS, T>::SMEM;
-    static auto kernel() { return k_march2d_batch<ST, COLS, T>; }
+    static auto kernel() { return k_march2d_levels_batch<ST, COLS, T>; }
+    static cudaError_t go(const BatchDev &D, int nblocks, int cur, int, int *err, bool pdl, cudaStream_t s)
+    {
+        return launch_k(kernel(), nblocks, threads, smem, s, pdl, D, cur, err);
+    }
 #endif
-    static cudaError_t prepare()
+};
+template <int ST, int COLS>
+struct BatchK<ST, COLS, 1> {
+    static constexpr int threads = COLS, smem = L2<ST, COLS>::smem();
+    static auto kernel() { return k_march2d_batch<ST, COLS>; }
+    static cudaError_t go(const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl, cudaStream_t s)
     {
-        static bool done = false;
-        if (!done) {
-            cudaError_t e = cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (e != cudaSuccess) return e;
-            done = true;
-        }
-        return cudaSuccess;
-    }
-    static cudaError_t launch(const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl, cudaStream_t s)
-    {
-        cudaError_t e = prepare();
-        if (e != cudaSuccess) return e;
-        ++g_launches;
         return launch_k(kernel(), nblocks, threads, smem, s, pdl, D, cur, wm, err);
-    }
-    static int blocks()
-    {
-        if (prepare() != cudaSuccess) return 0;
-        int n = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel(), threads, smem) == cudaSuccess ? n : 0;
     }
 };
 
+template <class K>
+static cudaError_t prepare_batch()
+{
+    static bool done = false;
+    if (!done) {
+        // The largest share of the SM for shared memory: a call's launches are of kernels that want different shares,
+        // an SM changes its split only when it is empty, and a dependent's blocks that come in under another
+        // kernel's smaller split don't all fit (16 squares in FP32, calls of five steps: 118 us so, 88 now).  A lone
+        // cavity's launches, tiles and direct-load steps among them, are the slower for it (128^2 2.15 -> 2.3 us a step).
+        cudaError_t e = cudaFuncSetAttribute(K::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, K::smem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(K::kernel(), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+        done = true;
+    }
+    return cudaSuccess;
+}
+
+template <class K>
+static cudaError_t launch_batch(const BatchDev &D, int nblocks, int cur, int wm, int *err, bool pdl, cudaStream_t s)
+{
+    cudaError_t e = prepare_batch<K>();
+    if (e != cudaSuccess) return e;
+    ++g_launches;
+    return K::go(D, nblocks, cur, wm, err, pdl, s);
+}
+
+template <class K>
+static int batch_bps()
+{
+    if (prepare_batch<K>() != cudaSuccess) return 0;
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, K::kernel(), K::threads, K::smem) == cudaSuccess ? n : 0;
+}
+
 #if LBM_EXACT
-#define LBM_BATCH_CASES(cols, levels, CALLB) \
-    switch (cols) {                              \
-    case 32: return CALLB(32, 1);             \
-    case 64: return CALLB(64, 1);             \
-    case 128: return CALLB(128, 1);           \
+#define LBM_BATCH_LEVELS(CALLB)
+#else
+#define LBM_BATCH_LEVELS(CALLB)                  \
+    case 64 * 8 + 2: return CALLB(64, 2);        \
+    case 64 * 8 + 4: return CALLB(64, 4);        \
+    case 128 * 8 + 2: return CALLB(128, 2);      \
+    case 128 * 8 + 4: return CALLB(128, 4);
+#endif
+#define LBM_BATCH_CASES(cols, levels, CALLB)     \
+    switch ((cols) * 8 + (levels)) {             \
+    case 32 * 8 + 1: return CALLB(32, 1);        \
+    case 64 * 8 + 1: return CALLB(64, 1);        \
+    case 128 * 8 + 1: return CALLB(128, 1);      \
+    LBM_BATCH_LEVELS(CALLB)                      \
     default: break;                              \
     }
-#else
-#define LBM_BATCH_CASES(cols, levels, CALLB) LBM_MARCH2D_CASES(cols, levels, CALLB)
-#endif
 
 template <int ST>
 static cudaError_t launch_batch_tx(int cols, int levels, const BatchDev &D, int nblocks, int cur, int wm,
                                    int *err, bool pdl, cudaStream_t s)
 {
-#define CALLB(X, T) (BatchK<ST, X, T>::launch(D, nblocks, cur, wm, err, pdl, s))
+#define CALLB(X, T) (launch_batch<BatchK<ST, X, T>>(D, nblocks, cur, wm, err, pdl, s))
     LBM_BATCH_CASES(cols, levels, CALLB)
 #undef CALLB
     return cudaErrorInvalidValue;
@@ -1589,7 +1610,7 @@ static cudaError_t launch_batch_tx(int cols, int levels, const BatchDev &D, int 
 template <int ST>
 static int batch_bps_tx(int cols, int levels)
 {
-#define CALLB(X, T) (BatchK<ST, X, T>::blocks())
+#define CALLB(X, T) (batch_bps<BatchK<ST, X, T>>())
     LBM_BATCH_CASES(cols, levels, CALLB)
 #undef CALLB
     return 0;

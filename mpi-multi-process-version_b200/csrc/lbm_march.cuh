@@ -650,9 +650,15 @@ using L2d = L2<ST, 128, 6, 4>;
 // nodes from which the single-cavity 2D kernel uses the deep ring
 constexpr int64_t kDeepRingNodes = int64_t(1) << 20;
 
-#if LBM_EXACT
-// The exact build's 2D march: one time level per pass, every node interpolated in
-// the reference's operand order from a ring of rows in shared memory.
+// The 2D march of one time level per pass: every node interpolated from a ring of
+// rows in shared memory, in the reference's operand order (exact build) or in the
+// window order of lbm_node2d.cuh (fast build: the single steps beside the
+// multi-level launches of lbm_march2d.cuh).  A block of the multi-level kernel run
+// with one level reads a row once, but its two filling rows and its four-row
+// segments cost more than that saves where few rows are in flight; us a step,
+// this kernel / that one on a grid of its own: FP64 200x180 5.2 / 8.5, 300^2 7.5 / 9.1,
+// 513^2 14.8 / 12.3, 1024^2 51 / 56, 2048^2 191 / 222, FP32 2048^2 131 / 145, a lone 128^2
+// member of a batch 5.7 / 7.3.
 
 // One node of the 2D march at row j, from the ring slots in shared memory:
 // interpolation, walls, macro, collision, stores.
@@ -669,11 +675,9 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     const int ny = G.ny;
     const int64_t P = G.plane;
     const int64_t id = (int64_t)j * G.pitch + i;
-    const int ja_ = j + off_a(j, ny), jb_ = j + off_b(j, ny);
     const unsigned char *nslot_j = sm + L::YS * L::yslot() + (j % L::NS) * L::nslot();
     const C Fy0 = ((const C *)(nslot_j + L::fo()))[tx];
     const double *wy = (const double *)(nslot_j + L::wo());
-    const C yp[3] = {C(wy[0]), C(wy[1]), C(wy[2])}, ym[3] = {C(wy[3]), C(wy[4]), C(wy[5])};
     auto SV = [&](const unsigned char *box, int idx, int q) -> C {
         (void)q;
         return tocomp(((const S *)box)[idx]);
@@ -681,13 +685,16 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     auto YB = [&](int yi, int s) -> const unsigned char * { return sm + (s % L::YS) * L::yslot() + L::yoff(yi); };
     auto NB = [&](int ni) -> const unsigned char * { return nslot_j + L::noff(ni); };
     auto ix = [&](int c, int dx) -> int { return tx + (c ? HX : 0) + dx; };
+    C f[9], gg[5];
+#if LBM_EXACT
+    const C yp[3] = {C(wy[0]), C(wy[1]), C(wy[2])}, ym[3] = {C(wy[3]), C(wy[4]), C(wy[5])};
+    const int ja_ = j + off_a(j, ny), jb_ = j + off_b(j, ny);
     // y-interpolation of a y-ring plane at x-offset dx
     auto YI = [&](int yi, int q, const C *w, int dx) -> C {
         const int c = L::yc(yi);
         const int e = ix(c, dx);
         return ip(w, SV(YB(yi, ja_), e, q), SV(YB(yi, j), e, q), SV(YB(yi, jb_), e, q));
     };
-    C f[9], gg[5];
     f[0] = SV(NB(0), ix(0, 0), 0);
     f[1] = ip(xp, SV(NB(1), ix(1, xa), 1), SV(NB(1), ix(1, 0), 1), SV(NB(1), ix(1, xb), 1));
     f[2] = YI(0, 2, yp, 0);
@@ -702,13 +709,6 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     gg[2] = YI(6, 11, yp, 0);
     gg[3] = ip(xm, SV(NB(5), ix(1, xa), 12), SV(NB(5), ix(1, 0), 12), SV(NB(5), ix(1, xb), 12));
     gg[4] = YI(7, 13, ym, 0);
-    // deviation from the conduction profile along x (the heated axis)
-    // (Tcn: the conduction profile at the node's x, sT: its streaming shift;
-    // both per column, computed once per segment)
-    if (Tr<ST>::kDevT) {
-        gg[1] -= sT;
-        gg[3] += sT;
-    }
 
     // walls (2B:731-801): centre values of row j
     auto CN = [&](int ni, int q) -> C { return SV(NB(ni), ix(L::nc(ni), 0), q); };
@@ -716,11 +716,11 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     const C two_wT = C(2.0) * C(0.125);
     if (i == 0) {
         f[1] = CN(2, 3); f[5] = CY(4, 7); f[8] = CY(3, 6);
-        gg[1] = -CN(5, 12) + two_wT * (Tr<ST>::kDevT ? C(G.Thot) - Tcn : C(G.Thot));
+        gg[1] = -CN(5, 12) + two_wT * C(G.Thot);
     }
     if (i == G.nx - 1) {
         f[3] = CN(1, 1); f[6] = CY(5, 8); f[7] = CY(2, 5);
-        gg[3] = -CN(4, 10) + two_wT * (Tr<ST>::kDevT ? C(G.Tcold) - Tcn : C(G.Tcold));
+        gg[3] = -CN(4, 10) + two_wT * C(G.Tcold);
     }
     if (j == ny - 1) {
         f[4] = CY(0, 2); f[7] = CY(2, 5); f[8] = CY(3, 6);
@@ -732,22 +732,59 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     }
 
     const C dt = C(G.dt);
-    const C rho = (Tr<ST>::kShift ? C(1.0) : C(0.0)) + (f[0]+f[1]+f[2]+f[3]+f[4]+f[5]+f[6]+f[7]+f[8]);
-#if LBM_EXACT
+    const C rho = f[0]+f[1]+f[2]+f[3]+f[4]+f[5]+f[6]+f[7]+f[8];
     const C u = ( f[1]-f[3]+f[5]-f[6]-f[7]+f[8]+C(0.5)*dt*C(0.0))/rho;
     const C v = ( f[2]-f[4]+f[5]+f[6]-f[7]-f[8]+C(0.5)*dt*Fy0)/rho;
+    const C T = gg[0]+gg[1]+gg[2]+gg[3]+gg[4];
+    C fp[9], gp[5], Fy;
+    collide2d<C, false, false>(f, gg, rho, u, v, T, G, fp, gp, Fy);
 #else
-    const C rinv = C(1.0) / rho;
-    const C u = (f[1]-f[3]+f[5]-f[6]-f[7]+f[8])*rinv;
-    const C v = (f[2]-f[4]+f[5]+f[6]-f[7]-f[8]+C(0.5)*dt*Fy0)*rinv;
+    C yp[3], ym[3];
+    window_weights<C>(wy, j, ny, yp, ym);
+    const int xo = win_lo(i, G.nx) - i, r0 = win_lo(j, ny);
+    // x-interpolation of a plane's row in box b, and of the y-ring's plane yi over the rows of j's window
+    auto XI = [&](const unsigned char *b, const C *w) -> C {
+        const S *p = (const S *)b + ix(1, xo);
+        return lin3(w, tocomp(p[0]), tocomp(p[1]), tocomp(p[2]));
+    };
+    auto YI = [&](int yi, const C *w) -> C {
+        const int e = ix(0, 0);
+        return lin3(w, SV(YB(yi, r0), e, 0), SV(YB(yi, r0 + 1), e, 0), SV(YB(yi, r0 + 2), e, 0));
+    };
+    auto XY = [&](int yi, const C *wx, const C *w) -> C {
+        return lin3(w, XI(YB(yi, r0), wx), XI(YB(yi, r0 + 1), wx), XI(YB(yi, r0 + 2), wx));
+    };
+    f[0] = SV(NB(0), ix(0, 0), 0);
+    f[1] = XI(NB(1), xp);
+    f[2] = YI(0, yp);
+    f[3] = XI(NB(2), xm);
+    f[4] = YI(1, ym);
+    f[5] = XY(2, xp, yp);
+    f[6] = XY(3, xm, yp);
+    f[7] = XY(4, xm, ym);
+    f[8] = XY(5, xp, ym);
+    gg[0] = SV(NB(3), ix(0, 0), 9);
+    gg[1] = XI(NB(4), xp);
+    gg[2] = YI(6, yp);
+    gg[3] = XI(NB(5), xm);
+    gg[4] = YI(7, ym);
+    // deviation from the conduction profile along x, per column (Tcn: its value at the node, sT: its streaming shift)
+    if (Tr<ST>::kDevT) {
+        gg[1] = sub_(gg[1], sT);
+        gg[3] = add_(gg[3], sT);
+    }
+    walls2d<C, Tr<ST>::kDevT>(i, j, G.nx, ny, C(G.Thot), C(G.Tcold), Tcn, [&](int q) -> C {
+        constexpr int at[14] = {0, 1, -1, 2, -2, -3, -4, -5, -6, 3, 4, -7, 5, -8};  // plane q: its row plane, or -1 - its y plane
+        const int a = at[q];
+        return a >= 0 ? SV(NB(a), ix(L::nc(a), 0), q) : SV(YB(-a - 1, j), ix(L::yc(-a - 1), 0), q);
+    }, f, gg);
+    C fp[9], gp[5], Fy, rho, u, v, T;
+    node2d<C, Tr<ST>::kShift, Tr<ST>::kDevT>(f, gg, Fy0, relax_of<C>(G), Tcn, fp, gp, Fy, rho, u, v, T);
 #endif
-    const C T = Tr<ST>::kDevT ? Tcn + (gg[0]+gg[1]+gg[2]+gg[3]+gg[4]) : gg[0]+gg[1]+gg[2]+gg[3]+gg[4];
     if (write_macro) {
         const int64_t mid = (int64_t)j * G.nx + i;
         B.rho[mid] = double(rho); B.u[mid] = double(u); B.v[mid] = double(v); B.T[mid] = double(T);
     }
-    C fp[9], gp[5], Fy;
-    collide2d<C, Tr<ST>::kShift, Tr<ST>::kDevT>(f, gg, rho, u, v, T, G, fp, gp, Fy);
     Fout[id] = Fy;
 #pragma unroll
     for (int q = 0; q < 9; ++q) dst[q * P + id] = tostore<S, C>(fp[q]);
@@ -858,8 +895,12 @@ __device__ __forceinline__ void march2d_run(int nseg, SegFn seg, CavFn cavity, i
         int xa = 0, xb = 0;
         C Tcn = C(0.0), sT = C(0.0);  // conduction profile at the column and its streaming shift
         if (active) {
+#if LBM_EXACT
             load_w(G.wgt[0], i, xp, xm);
             xa = off_a(i, G.nx); xb = off_b(i, G.nx);
+#else
+            window_weights<C>(G.wgt[0] + (int64_t)i * 6, i, G.nx, xp, xm);
+#endif
             if (Tr<ST>::kDevT) {
                 Tcn = C(tc_value(G, i));
                 sT = C(0.125 * G.dt * tc_gradient(G));
@@ -959,4 +1000,3 @@ k_march2d_batch(const BatchDev D, int cur, int write_macro, int *err)
     };
     march2d_run<ST, L2<ST, TX>, true>(s1 - s0, seg, cavity, write_macro, err);
 }
-#endif  // LBM_EXACT

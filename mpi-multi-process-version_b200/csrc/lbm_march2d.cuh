@@ -1,4 +1,4 @@
-// The fast build's 2D march: T time levels per pass over the populations.
+// The fast build's 2D march of T = 2 or 4 time levels per pass over the populations.
 //
 // Included by lbm_kernels.cu inside namespace lbm::LBM_NS, after
 // lbm_node2d.cuh and lbm_march.cuh (barriers, TMA copies, programmatic launch).
@@ -58,7 +58,7 @@ struct M2 {
     static constexpr int K0 = B0 + 64 + kGeoStage;          // a batch's staged geometry, then its Relax
     static constexpr int SMEM = K0 + 128 + 128;
     static constexpr int TX = PLANES + WB * ES + 48;        // bytes of a row's copies
-    static_assert((WB * ES) % 16 == 0 && WB <= 256, "2D march layout");
+    static_assert((WB * ES) % 16 == 0 && WB <= 256 && (T == 2 || T == 4), "2D march layout");
 };
 
 // A segment: columns [x0, x0 + w) of cavity cav, rows [ja, jb).
@@ -72,8 +72,7 @@ __device__ __forceinline__ Seg2 seg2_of(const int4 q)
 }
 
 template <int ST, class M, bool kStage, class CavFn>
-__device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, int sbeg, int send, CavFn cavity,
-                                               int write_macro, int *err)
+__device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, int sbeg, int send, CavFn cavity, int *err)
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
@@ -88,8 +87,8 @@ __device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, in
     Relax<C> *srelax = (Relax<C> *)(sm + M::K0);
 
     const int tid = threadIdx.x;
-    const int s = T == 1 ? 0 : tid / NT;  // the group's time level (warp-uniform)
-    const int t = T == 1 ? tid : tid % NT;
+    const int s = tid / NT;  // the group's time level (warp-uniform)
+    const int t = tid % NT;
     if (tid == 0) {
         for (int k = 0; k < NS; ++k) mbar_init(&bar[k], 1);
         fence_barrier_init();
@@ -193,7 +192,7 @@ __device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, in
             }
             work = work && n <= r1;
             // the input ring: rows below group 0's node row are free
-            if (T == 1 || s == 0) {
+            if (s == 0) {
                 int n0 = work ? n : r1 + 1;
                 if (bottom && !work && q < 4 * (T - 1)) n0 = 3 * (q >> 2) + 3;  // a stall: the next row's node
                 if (tid == 0) issue_to(min(n0 - 1 + NS, row_last));
@@ -203,10 +202,10 @@ __device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, in
                 const bool lo = n == 0 && bottom, hi = n == ny - 1;
                 // ring rows of node row n + k
                 auto rowp = [&](int r) -> const unsigned char * {
-                    if (T == 1 || s == 0) return sm + ((seq + uint32_t(r - row_first)) % NS) * M::ROW;
+                    if (s == 0) return sm + ((seq + uint32_t(r - row_first)) % NS) * M::ROW;
                     return sm + M::E0 + ((s - 1) * 3 + r % 3) * M::ROW;
                 };
-                if (T == 1 || s == 0) {
+                if (s == 0) {
                     auto wait = [&](int r) {
                         const uint32_t k = seq + uint32_t(r - row_first);
                         ok = ok && mbar_wait_lim(&bar[k % NS], (k / NS) & 1u);
@@ -296,11 +295,6 @@ __device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, in
                         node2d<C, DEV, DEVT>(f, g, F0, K, Tcn, fp, gp, Fy, rho, u, v, Tm);
                         if (s == T - 1) {
                             const int64_t id = (int64_t)n * G.pitch + c;
-                            if (T == 1 && write_macro) {
-                                const int64_t mid = (int64_t)n * nx + c;
-                                Bp->rho[mid] = double(rho); Bp->u[mid] = double(u); Bp->v[mid] = double(v);
-                                Bp->T[mid] = double(Tm);
-                            }
                             Fout[id] = Fy;
                             S *o = dst + id;
 #pragma unroll
@@ -353,9 +347,9 @@ constexpr int m2_blocks()
 // one cavity
 template <int ST, int COLS, int T>
 __global__ void __launch_bounds__(COLS * T, (m2_blocks<M2<ST, COLS, T>, ST>()))
-k_march2d(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap fmap,
+k_march2d_levels(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap fmap,
           const __grid_constant__ Geo G, typename Tr<ST>::S *__restrict__ dst, typename Tr<ST>::C *__restrict__ Fout,
-          const __grid_constant__ Bufs B, int write_macro, const int4 *__restrict__ segs,
+          const __grid_constant__ Bufs B, const int4 *__restrict__ segs,
           const int *__restrict__ seg_off, int *err)
 {
     using S = typename Tr<ST>::S;
@@ -370,13 +364,13 @@ k_march2d(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUten
         Bp = &B;
     };
     march2d_levels<ST, M2<ST, COLS, T>, false>(segs, seg_off[blockIdx.x], seg_off[blockIdx.x + 1], cavity,
-                                                   write_macro, err);
+                                               err);
 }
 
 // many cavities; `cur` is the ping-pong buffer holding the populations read
 template <int ST, int COLS, int T>
 __global__ void __launch_bounds__(COLS * T, (m2_blocks<M2<ST, COLS, T>, ST>()))
-k_march2d_batch(const BatchDev D, int cur, int write_macro, int *err)
+k_march2d_levels_batch(const BatchDev D, int cur, int *err)
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
@@ -391,5 +385,5 @@ k_march2d_batch(const BatchDev D, int cur, int write_macro, int *err)
         Fo = (C *)D.bufs[c].F[1 - cur];
     };
     march2d_levels<ST, M2<ST, COLS, T>, true>(D.segs, D.seg_off[blockIdx.x], D.seg_off[blockIdx.x + 1], cavity,
-                                                  write_macro, err);
+                                              err);
 }
