@@ -295,29 +295,38 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
     C xp[3], xm[3], yp[3], ym[3];
     window_weights<C>(G.wgt[0] + (int64_t)i * 6, i, G.nx, xp, xm);
     window_weights<C>(G.wgt[1] + (int64_t)j * 6, j, G.ny, yp, ym);
-    auto XI = [&](int q, const C w[3], int64_t r) -> C {
-        return lin3(w, LD(q, r + xo), LD(q, r + xo + 1), LD(q, r + xo + 2));
+    // the loads first, as many of them in flight as the registers hold: planes 1 3 10 12 along x, 2 4 11 13 along y,
+    // 5 6 7 8 both
+    const C c0 = LD(0, 0), c9 = LD(9, 0);
+    C h[4][3], w[4][3], d[4][3][3];
+    constexpr int hq[4] = {1, 3, 10, 12}, wq[4] = {2, 4, 11, 13};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+            h[k][e] = LD(hq[k], xo + e);
+            w[k][e] = LD(wq[k], yo + e * G.pitch);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) d[k][r][e] = LD(5 + k, yo + r * G.pitch + xo + e);
+        }
+    auto I = [&](const C ww[3], const C v[3]) -> C { return lin3(ww, v[0], v[1], v[2]); };
+    auto XY = [&](int k, const C wx[3], const C wy[3]) -> C {
+        return lin3(wy, I(wx, d[k][0]), I(wx, d[k][1]), I(wx, d[k][2]));
     };
-    auto YI = [&](int q, const C w[3]) -> C {
-        return lin3(w, LD(q, yo), LD(q, yo + G.pitch), LD(q, yo + 2 * G.pitch));
-    };
-    auto XY = [&](int q, const C wx[3], const C wy[3]) -> C {
-        return lin3(wy, XI(q, wx, yo), XI(q, wx, yo + G.pitch), XI(q, wx, yo + 2 * G.pitch));
-    };
-    f[0] = LD(0, 0);
-    f[1] = XI(1, xp, 0);
-    f[2] = YI(2, yp);
-    f[3] = XI(3, xm, 0);
-    f[4] = YI(4, ym);
-    f[5] = XY(5, xp, yp);
-    f[6] = XY(6, xm, yp);
-    f[7] = XY(7, xm, ym);
-    f[8] = XY(8, xp, ym);
-    gg[0] = LD(9, 0);
-    gg[1] = XI(10, xp, 0);
-    gg[2] = YI(11, yp);
-    gg[3] = XI(12, xm, 0);
-    gg[4] = YI(13, ym);
+    f[0] = c0;
+    f[1] = I(xp, h[0]);
+    f[2] = I(yp, w[0]);
+    f[3] = I(xm, h[1]);
+    f[4] = I(ym, w[1]);
+    f[5] = XY(0, xp, yp);
+    f[6] = XY(1, xm, yp);
+    f[7] = XY(2, xm, ym);
+    f[8] = XY(3, xp, ym);
+    gg[0] = c9;
+    gg[1] = I(xp, h[2]);
+    gg[2] = I(yp, w[2]);
+    gg[3] = I(xm, h[3]);
+    gg[4] = I(ym, w[3]);
     // deviation from the conduction profile: the departure point of g1 / g3
     // lies dt behind / ahead along x
     C Tc = C(0.0);
@@ -359,8 +368,16 @@ __device__ __forceinline__ void step2d_node(const Geo &G, const typename Tr<ST>:
     for (int q = 0; q < 5; ++q) ST_(9 + q, gp[q]);
 }
 
-template <int ST, int KIND>
-__global__ void __launch_bounds__(256)
+// MINB, the direct-load kernels' blocks per SM that the registers are bounded for
+// (0: the compiler's own choice).  The compiler takes few registers and with them
+// few loads in flight where nothing is asked of it; a domain of a wave or less
+// wants the loads in flight, a larger one the blocks.  us a step in graphs of
+// single steps, 0 -> this: 2D FP64 (two blocks, 128 registers) 128^2 6.1 -> 4.0,
+// 2048^2 320 -> 223; FP32 up to 2^16 nodes (two, 112) 128^2 6.2 -> 3.5, above (0) 2048^2
+// 147 against 166; 3D FP32 up to 2^15 nodes (one, 198) 32 x 24 x 16 5.1 -> 4.7, above (0)
+// 128^3 187 against 227.
+template <int ST, int KIND, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 k_step2d(const Geo G, const typename Tr<ST>::S *__restrict__ src, const typename Tr<ST>::C *__restrict__ Fin,
          typename Tr<ST>::S *__restrict__ dst, typename Tr<ST>::C *__restrict__ Fout, const Bufs B,
          int write_macro)
@@ -410,7 +427,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned *gen, uns
 // before the next step reads what its neighbours wrote.  The macroscopic
 // fields are written by the last step.
 template <int ST>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, LBM_EXACT ? 0 : 2)
 k_steps2d_resident(const Geo G, typename Tr<ST>::S *p0, typename Tr<ST>::S *p1, typename Tr<ST>::C *F0,
                    typename Tr<ST>::C *F1, const Bufs B, int cur, int nsteps, unsigned *bar, int *err)
 {
@@ -796,8 +813,8 @@ __device__ __forceinline__ void node3d(const C f[19], const C gg[7], C Fz0, cons
 #endif
 }
 
-template <int ST, int KIND>
-__global__ void __launch_bounds__(256)
+template <int ST, int KIND, int MINB>
+__global__ void __launch_bounds__(256, MINB)
 k_step3d(const Geo G, const typename Tr<ST>::S *__restrict__ src, const typename Tr<ST>::C *__restrict__ Fin,
          typename Tr<ST>::S *__restrict__ dst, typename Tr<ST>::C *__restrict__ Fout, const Bufs B,
          int write_macro)
@@ -1152,16 +1169,14 @@ static cudaError_t launch_step(const Geo &g, const void *pin, const void *Fin, v
     dim3 blk(32, 8, 1);
     if (g.dim == 2) {
         dim3 grd((g.nx + 31) / 32, (g.ny + 7) / 8, 1);
-        if (kind == 0)
-            k_step2d<ST, 0><<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
-        else
-            k_step2d<ST, 1><<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
+        constexpr int few = LBM_EXACT ? 0 : 2, many = LBM_EXACT || ST == kF32 ? 0 : 2;
+        const auto k = kind ? k_step2d<ST, 1, many> : (g.nnode <= (1 << 16) ? k_step2d<ST, 0, few> : k_step2d<ST, 0, many>);
+        k<<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
     } else {
         dim3 grd((g.nx + 31) / 32, (g.ny + 7) / 8, g.khi - g.klo);
-        if (kind == 0)
-            k_step3d<ST, 0><<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
-        else
-            k_step3d<ST, 1><<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
+        constexpr int few = LBM_EXACT || ST == kF64 ? 0 : 1;
+        const auto k = kind ? k_step3d<ST, 1, 0> : (g.nnode <= (1 << 15) ? k_step3d<ST, 0, few> : k_step3d<ST, 0, 0>);
+        k<<<grd, blk, 0, s>>>(g, (const S *)pin, (const C *)Fin, (S *)pout, (C *)Fout, b, wm);
     }
     ++g_launches;
     return cudaGetLastError();
