@@ -369,7 +369,8 @@ int lbm_batch_run_mixed(lbm_batch *b, const int32_t *mask, int32_t max_steps, in
 /* The autotuner: time each storage LBM_BATCH_OPT_STORAGES allows (the
  * batch's state is converted in place, lbm_batch_set_storage) x each tile
  * width and grid size on the batch itself (the timed steps advance the
- * members) and keep the fastest; reports the tile, grid and rate
+ * members: `steps`, or as many as eight of the launches a run is made of take,
+ * whichever is more, and a few to warm up) and keep the fastest; reports the tile, grid and rate
  * (lbm_batch_get_option(LBM_BATCH_OPT_STORAGE) the storage).  No counterpart
  * in the reference. */
 int lbm_batch_tune(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nblocks, double *mlups);

@@ -943,6 +943,9 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
     if (!b->persistent || !b->march_ok)
         return set_error(LBM_ERR_UNSUPPORTED, "lbm_batch_tune: the batch does not use the persistent kernel");
     if (steps < 2) steps = 2;
+    // the launches a run is made of: eight multi-step ones before the single last step
+    const int lev = batch_levels(b);
+    if (lev > 1) steps = std::max(steps, 8 * lev + 1);
     BCU(cudaSetDevice(b->device));
     int sms = 0;
     BCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
@@ -956,12 +959,20 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
     BCU(cudaEventCreate(&e0));
     BCU(cudaEventCreate(&e1));
     const int keep_nb = b->nblocks_opt;
+    const int keep_graphs = b->use_graphs;
+    b->use_graphs = 0;  // a capture would count as time
+    auto done = [&](int st) {
+        b->use_graphs = keep_graphs;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        return st;
+    };
     for (int ti = 0; ti < ntile; ++ti) {
         const int t = tiles[ti];
         const int bps = b->dim == 3 ? (b->mode == LBM_MODE_EXACT ? exact::march_batch3d_blocks_per_sm(b->storage)
                                                                  : fast::march_batch3d_blocks_per_sm(b->storage))
                                     : (b->mode == LBM_MODE_EXACT ? exact::march_batch_blocks_per_sm(b->storage, t, 1)
-                                                                 : fast::march_batch_blocks_per_sm(b->storage, W_cols(t), batch_levels(b)));
+                                                                 : fast::march_batch_blocks_per_sm(b->storage, W_cols(t), lev));
         if (bps <= 0) continue;
         const int cands[2] = {bps, bps > 1 ? bps / 2 : 0};
         for (int c : cands) {
@@ -969,14 +980,14 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
             b->tile = t;
             b->nblocks_opt = c * sms;
             b->dirty = true;
-            int st = lbm_batch_step(b, 2);  // warm-up, builds the tables
-            if (st) return st;
+            int st = lbm_batch_step(b, lev > 1 ? 2 * lev + 2 : 2);  // warm-up, builds the tables
+            if (st) return done(st);
             BCU(cudaEventRecord(e0, b->stream));
             st = lbm_batch_step(b, steps);
-            if (st) return st;
+            if (st) return done(st);
             BCU(cudaEventRecord(e1, b->stream));
             st = lbm_batch_synchronize(b);
-            if (st) return st;
+            if (st) return done(st);
             float ms = 0.f;
             BCU(cudaEventElapsedTime(&ms, e0, e1));
             const double v = (double)b->active_nodes * steps / (ms * 1e-3) / 1e6;
@@ -987,8 +998,7 @@ static int tune_storage(lbm_batch *b, int32_t steps, int32_t *tile, int32_t *nbl
             }
         }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    done(LBM_OK);
     b->tile = best_tile;
     b->tile_opt = best_tile;
     b->nblocks_opt = keep_nb > 0 ? keep_nb : best_nb;
