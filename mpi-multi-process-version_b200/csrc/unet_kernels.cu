@@ -1251,15 +1251,48 @@ bool conv_tc(const ConvArgs &a, cudaStream_t s)
 // the tiles' 128 rows of A are mostly unused and the MMAs (24 a tile) are the
 // bound; at batch 1 the launch, one tile's latency and the sum.  Against 64-bit
 // sums the error is 1e-7 to 6e-6 of the result, as long as a share's chain.
-constexpr int WST = 4, WCOLS = 512;                 // stages; TMEM columns (a power of two)
+//
+// A tile that reaches past the image multiplies zeros of dz by x, and next to the
+// border that is an x of the image: the pixel right of the last column meets it in
+// the taps to the left, the row below the last one in the taps above.  An
+// infinity there must not turn into a NaN of taps that don't use it (RAG): tiles at
+// the right edge take the left taps from a second copy of x without the last column,
+// and a step whose second row is outside takes that row's x from zeros.
+constexpr int WCOLS = 512;                          // TMEM columns (a power of two)
 constexpr int WA_ATOM = TBM * 64, WA = 4 * WA_ATOM;  // dz: 32 channels of a tile, all
 constexpr int WX_TX = THP * 64, WX = (WX_TX + 1023) / 1024 * 1024;
-constexpr int WSTAGE = WA + WX, WSMEM = 1024 + WST * WSTAGE + 1024;
+constexpr int WZERO = (8 + 2) * 64;                 // a row of x with its border
+template <bool RAG>
+struct WgLayout {
+    static constexpr int ST = RAG ? 3 : 4;          // stages
+    static constexpr int STAGE = WA + (RAG ? 2 : 1) * WX, ZERO = 1024 + ST * STAGE;
+    static constexpr int SMEM = ZERO + (RAG ? 1024 : 0) + 1024;
+    static_assert(WZERO <= 1024 && SMEM <= 227 * 1024 && ST * STAGE < (1 << 18), "strides have 14 bits of 16 bytes");
+};
 
-__global__ void __launch_bounds__(TTHREADS)
-k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap xmap, int H, int Cin, int Cout,
-           int ntx, int nty, int ntiles, int per, int vec, float *__restrict__ ws)
+// FP32 accumulators, bf16 A and B, both channel-major, M = 128, N
+__host__ __device__ constexpr uint32_t wg_idesc(int N)
 {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(N >> 3) << 17) | (8u << 24);
+}
+
+__device__ __forceinline__ void wg_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accum)
+        : "memory");
+}
+
+template <bool RAG>
+__global__ void __launch_bounds__(TTHREADS)
+k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUtensorMap xmap,
+           const __grid_constant__ CUtensorMap emap, int H, int W, int Cin, int Cout, int ntx, int nty, int ntiles, int per,
+           int vec, float *__restrict__ ws)
+{
+    constexpr int WST = WgLayout<RAG>::ST, WSTAGE = WgLayout<RAG>::STAGE;
     extern __shared__ unsigned char tc_raw[];
     unsigned char *sm = tc_raw + ((1024u - (smem_u32(tc_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t *>(sm);  // a stage's copies have landed
@@ -1290,6 +1323,10 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
         asm volatile("prefetch.tensormap [%0];" ::"l"(&zmap) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
     }
+    if (RAG && tid >= 64 && tid < 64 + WZERO / 16) {
+        *reinterpret_cast<uint4 *>(sm + WgLayout<RAG>::ZERO + (tid - 64) * 16) = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1297,8 +1334,6 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // after the allocation, as in k_conv3x3_tc
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    // FP32 accumulators, bf16 A and B, both channel-major, M = 128, N = 96
-    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (12u << 17) | (8u << 24);
     bool fail = false;
     int k = 0;  // tiles this thread has issued
     if (tid == 32) {  // the copies
@@ -1310,9 +1345,11 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
             }
             unsigned char *base = stages + st * WSTAGE;
             const int x0 = (t % ntx) * TTW, y0 = ((t / ntx) % nty) * TTH, b = t / (ntx * nty);
-            nn_expect(&full[st], uint32_t(atoms * WA_ATOM + WX_TX));
+            const bool edge = RAG && x0 + TTW > W;
+            nn_expect(&full[st], uint32_t(atoms * WA_ATOM + (edge ? 2 : 1) * WX_TX));
             for (int a = 0; a < atoms; ++a) nn_tma4(base + a * WA_ATOM, &zmap, &full[st], co0 + a * 32, x0, y0, b);
             nn_tma4(base + WA, &xmap, &full[st], c0, x0 - 1, y0 - 1, b);
+            if (edge) nn_tma4(base + WA + WX, &emap, &full[st], c0, W > 1 ? x0 - 1 : 1, y0 - 1, b);
         }
     } else if (tid == 0) {  // the MMAs
         for (; k < nt; ++k) {
@@ -1324,19 +1361,31 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
             const uint32_t base = smem_u32(stages + (k % WST) * WSTAGE);
             // A: the next 32 channels an atom further, the next 8 pixels a tile row; B: a pixel, a row with its border
             const uint64_t da0 = wg_desc(base, WA_ATOM, 8 * 64), db0 = wg_desc(base + WA, 64, THW * 64);
-            const int steps = (min(TTH, H - ((t0 + k) / ntx) % nty * TTH) + 1) / 2;  // rows past the image are zeros
+            const int rows = min(TTH, H - ((t0 + k) / ntx) % nty * TTH), steps = (rows + 1) / 2;  // past them: zeros
+            const bool edge = RAG && ((t0 + k) % ntx) * TTW + TTW > W;
+            // the second row of a step from zeros: the K stride of a start address leads there
+            const uint32_t zero = smem_u32(sm + WgLayout<RAG>::ZERO);
+            auto to_zero = [&](uint64_t d) -> uint64_t {
+                const uint64_t stride = (zero >> 4) - (uint32_t)(d & 0x3FFFu);
+                return (d & ~((uint64_t)0x3FFFu << 32)) | (stride << 32);
+            };
 #pragma unroll 2
             for (int r = 0; r < steps; ++r) {
                 const uint32_t accum = k > 0 || r > 0;
+                const uint64_t da = da0 + (uint64_t)(r * (2 * 8 * 64 / 16));
+                const bool half = RAG && 2 * r + 1 == rows;
 #pragma unroll
-                for (int dy = 0; dy < 3; ++dy)
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem + dy * 96),
-                        "l"(da0 + (uint64_t)(r * (2 * 8 * 64 / 16))),
-                        "l"(db0 + (uint64_t)((2 * r + dy) * (THW * 64 / 16))), "r"(idesc), "r"(accum)
-                        : "memory");
+                for (int dy = 0; dy < 3; ++dy) {
+                    const uint64_t db = db0 + (uint64_t)((2 * r + dy) * (THW * 64 / 16));
+                    const bool z = half && dy == 0;
+                    if (!edge) {
+                        wg_mma(tmem + dy * 96, da, z ? to_zero(db) : db, wg_idesc(96), accum);
+                    } else {
+                        const uint64_t dl = db + WX / 16, dc = db + 64 / 16;
+                        wg_mma(tmem + dy * 96, da, z ? to_zero(dl) : dl, wg_idesc(32), accum);
+                        wg_mma(tmem + dy * 96 + 32, da, z ? to_zero(dc) : dc, wg_idesc(64), accum);
+                    }
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                              smem_u32(&bars[k % WST]))
@@ -1398,15 +1447,16 @@ WgradPlan wgrad_plan(int B, int H, int W, int Cin, int Cout)
     return p;
 }
 
-// an image tensor as (channel, x, y, image): boxes of 32 channels of w x h pixels, zero outside
-bool pixel_map(const void *p, int C, int64_t stride, int B, int H, int W, int w, int h, CUtensorMap *m)
+// an image tensor (H x W pixels in memory, the first Hv x Wv of them seen) as (channel, x, y, image): boxes of 32
+// channels of w x h pixels, zero outside
+bool pixel_map(const void *p, int C, int64_t stride, int B, int Hv, int Wv, int H, int W, int w, int h, CUtensorMap *m)
 {
     typedef CUresult (*Encode)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     const Encode enc = (Encode)lbm::tensor_map_encoder();
     const cuuint64_t row = (cuuint64_t)stride * 2;
-    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)B};
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)Wv, (cuuint64_t)Hv, (cuuint64_t)B};
     const cuuint64_t str[3] = {row, row * W, row * W * H};
     const cuuint32_t box[4] = {32, (cuuint32_t)w, (cuuint32_t)h, 1}, one[4] = {1, 1, 1, 1};
     return enc && enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)p, dims, str, box, one,
@@ -1414,16 +1464,20 @@ bool pixel_map(const void *p, int C, int64_t stride, int B, int H, int W, int w,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <bool RAG>
 bool launch_wgrad_tc(const bf16 *dz, const bf16 *x, int64_t xs, int xo, int B, int H, int W, int Cin, int Cout,
                      const WgradPlan &pl, float *part, cudaStream_t s)
 {
-    CUtensorMap zm, xm;
-    if (!pixel_map(dz, Cout, Cout, B, H, W, TTW, TTH, &zm) ||
-        !pixel_map(x + xo, Cin, xs, B, H, W, THW, TTH + 2, &xm))
+    CUtensorMap zm, xm, em;
+    if (!pixel_map(dz, Cout, Cout, B, H, W, H, W, TTW, TTH, &zm) ||
+        !pixel_map(x + xo, Cin, xs, B, H, W, H, W, THW, TTH + 2, &xm))
         return false;
-    cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, WSMEM);
+    if (!RAG) em = xm;
+    else if (!pixel_map(x + xo, Cin, xs, B, H, W > 1 ? W - 1 : 1, H, W, THW, TTH + 2, &em)) return false;
+    constexpr int smem = WgLayout<RAG>::SMEM;
+    cudaFuncSetAttribute(k_wgrad_tc<RAG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const dim3 grid(unsigned(Cin / 32), unsigned((Cout + TBM - 1) / TBM), unsigned(pl.S));
-    go(k_wgrad_tc, grid, TTHREADS, WSMEM, s, zm, xm, H, Cin, Cout, pl.ntx, pl.nty, B * pl.ntx * pl.nty, pl.per,
+    go(k_wgrad_tc<RAG>, grid, TTHREADS, smem, s, zm, xm, em, H, W, Cin, Cout, pl.ntx, pl.nty, B * pl.ntx * pl.nty, pl.per,
        int(((uintptr_t)part & 31u) == 0), part);
     return true;
 }
@@ -1508,7 +1562,9 @@ extern "C" int lbm_nn_conv3x3_wgrad(const void *dz, const void *x, int64_t xs, i
                (long long)ws_elems, (long long)pl.S * n);
     cudaStream_t s = (cudaStream_t)stream;
     float *part = pl.S == 1 ? dw : ws;  // one share is the sum
-    if (!launch_wgrad_tc((const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin, Cout, pl, part, s))
+    const bool rag = W % TTW != 0 || H % 2 != 0;
+    if (!(rag ? launch_wgrad_tc<true> : launch_wgrad_tc<false>)((const bf16 *)dz, (const bf16 *)x, xs, xo, B, H, W, Cin,
+                                                                Cout, pl, part, s))
         return lbm::set_error(LBM_ERR_CUDA, "lbm_nn_conv3x3_wgrad: no tensor maps on this device");
     if (pl.S > 1) sum_splits(ws, pl.S, n, dw, s);
     return launched("lbm_nn_conv3x3_wgrad", pl.S > 1 ? 2 : 1);
