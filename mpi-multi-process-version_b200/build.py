@@ -42,7 +42,7 @@ UNITS = [
     ("unet.o", "unet_kernels.cu", []),
 ]
 
-HEADERS = ["lbm_internal.h", "lbm_handle.h", "lbm_march.cuh", "lbm_march2d.cuh", "lbm_march3d.cuh", "lbm_node2d.cuh", "lbm_tile2d.cuh"]
+HEADERS = ["lbm_internal.h", "lbm_shared.h", "lbm_handle.h", "lbm_march.cuh", "lbm_march2d.cuh", "lbm_march3d.cuh", "lbm_node2d.cuh", "lbm_tile2d.cuh"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:

@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include "lbm_internal.h"
+#include "lbm_shared.h"
 
 #ifndef LBM_EXACT
 #define LBM_EXACT 0
@@ -1312,44 +1313,39 @@ static cudaError_t launch_k(void (*k)(KArgs...), int grid, int block, int smem, 
     return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// -1 (nothing is remembered for it) if there is none
+static int this_device()
+{
+    int d = -1;
+    return cudaGetDevice(&d) == cudaSuccess ? d : -1;
+}
+
+template <class K>
+static cudaError_t max_smem(K k, int bytes)
+{
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 template <int ST, int TY>
 static cudaError_t prepare_march3d()
 {
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march3d<ST, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             L3<ST, TY>::smem());
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
-    return cudaSuccess;
+    static OncePerDevice once;
+    return once.run(this_device(), [] { return max_smem(k_march3d<ST, TY>, L3<ST, TY>::smem()); });
 }
 
 template <int ST, class L>
 static cudaError_t prepare_march2d()
 {
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march2d<ST, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             L::smem());
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
-    return cudaSuccess;
+    static OncePerDevice once;
+    return once.run(this_device(), [] { return max_smem(k_march2d<ST, L>, L::smem()); });
 }
 
 #if !LBM_EXACT
 template <int ST, int COLS, int T>
 static cudaError_t prepare_levels2d()
 {
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march2d_levels<ST, COLS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             M2<ST, COLS, T>::SMEM);
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
-    return cudaSuccess;
+    static OncePerDevice once;
+    return once.run(this_device(), [] { return max_smem(k_march2d_levels<ST, COLS, T>, M2<ST, COLS, T>::SMEM); });
 }
 
 // CALLT(columns, levels) of the variant asked for
@@ -1512,12 +1508,9 @@ static cudaError_t launch_tile2d(const Geo &g, const void *pin, const void *Fin,
 {
     using S = typename Tr<ST>::S;
     using C = typename Tr<ST>::C;
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_tile2d<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem);
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
+    static OncePerDevice once;
+    cudaError_t e = once.run(this_device(), [] { return max_smem(k_tile2d<ST>, kTileSmem); });
+    if (e != cudaSuccess) return e;
     TilePlan q = pl;
     q.T = T;
     ++g_launches;
@@ -1561,20 +1554,18 @@ struct BatchK<ST, COLS, 1> {
 template <class K>
 static cudaError_t prepare_batch()
 {
-    static bool done = false;
-    if (!done) {
+    static OncePerDevice once;
+    return once.run(this_device(), [] {
         // The largest share of the SM for shared memory: a call's launches are of kernels that want different shares,
         // an SM changes its split only when it is empty, and a dependent's blocks that come in under another
         // kernel's smaller split don't all fit (16 squares in FP32, calls of five steps: 118 us so, 88 now).  A lone
         // cavity's launches, tiles and direct-load steps among them, are the slower for it (128^2 2.15 -> 2.3 us a step).
-        cudaError_t e = cudaFuncSetAttribute(K::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, K::smem);
+        cudaError_t e = max_smem(K::kernel(), K::smem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(K::kernel(), cudaFuncAttributePreferredSharedMemoryCarveout,
                                      cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
-    return cudaSuccess;
+        return e;
+    });
 }
 
 template <class K>
@@ -1649,14 +1640,8 @@ int march_batch_blocks_per_sm(int store, int cols, int levels)
 template <int ST>
 static cudaError_t prepare_batch3d()
 {
-    static bool done = false;
-    if (!done) {
-        cudaError_t e = cudaFuncSetAttribute(k_march3d_batch<ST, kBatchTileY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             L3<ST, kBatchTileY>::smem());
-        if (e != cudaSuccess) return e;
-        done = true;
-    }
-    return cudaSuccess;
+    static OncePerDevice once;
+    return once.run(this_device(), [] { return max_smem(k_march3d_batch<ST, kBatchTileY>, L3<ST, kBatchTileY>::smem()); });
 }
 
 template <int ST>

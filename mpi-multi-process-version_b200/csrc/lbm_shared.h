@@ -1,0 +1,29 @@
+// Host-side bookkeeping that handles on several devices and threads share.
+#ifndef LBM_SHARED_H
+#define LBM_SHARED_H
+#include <stdint.h>
+
+#include <atomic>
+
+namespace lbm {
+
+// A set-up call that holds for one device only (cudaFuncSetAttribute): made once
+// for each device, and again as long as it fails.
+class OncePerDevice {
+    std::atomic<uint64_t> done_{0};
+
+public:
+    template <class F>
+    auto run(int device, F call) -> decltype(call())
+    {
+        using E = decltype(call());
+        const uint64_t bit = device >= 0 && device < 64 ? uint64_t(1) << device : 0;
+        if (done_.load(std::memory_order_acquire) & bit) return E(0);
+        const E e = call();
+        if (e == E(0)) done_.fetch_or(bit, std::memory_order_release);
+        return e;
+    }
+};
+
+}  // namespace lbm
+#endif
