@@ -897,8 +897,8 @@ constexpr long long kNnShortWait = 1000000LL;
 
 __device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity, long long limit = kNnWaitCycles)
 {
-    const long long t0 = clock64();
     if (limit < kNnShortWait) {
+        const long long t0 = clock64();
         uint32_t ok = 0;
         while (true) {
             asm volatile(
@@ -912,6 +912,8 @@ __device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity, long 
             if (clock64() - t0 > limit) return false;
         }
     }
+    if (nn_mbar_test(b, parity)) return true;
+    const long long t0 = clock64();
     while (!nn_mbar_test(b, parity))
         if (clock64() - t0 > limit) return false;
     return true;
@@ -1131,7 +1133,10 @@ k_conv3x3_tc(const ConvArgs a, const __grid_constant__ CUtensorMap xmap, const _
             if (!px || n >= a.Cout) continue;
             float z[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) z[j] = bad ? NAN : __uint_as_float(r[j]) + sbias[sl * 16 + j];
+            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]) + sbias[sl * 16 + j];
+            if (bad)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) z[j] = NAN;
             if (vec && n + 16 <= a.Cout) {
                 if (a.of) {
                     float *p = a.of + m * a.os + a.oo + n;
@@ -1409,7 +1414,10 @@ k_wgrad_tc(const __grid_constant__ CUtensorMap zmap, const __grid_constant__ CUt
             if (co >= Cout) continue;
             float z[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) z[j] = bad ? NAN : __uint_as_float(r[j]);
+            for (int j = 0; j < 16; ++j) z[j] = __uint_as_float(r[j]);
+            if (bad)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) z[j] = NAN;
             float *q = o + (int64_t)(sl >> 1) * Cin + (sl & 1) * 16;
             if (vec) {
                 st_v8(q, z);
