@@ -449,12 +449,11 @@ static int get_graph(lbm_batch *b, int cur, cudaGraphExec_t *out)
 {
     if (!b->graph[cur]) {
         cudaGraph_t g = nullptr;
-        const int64_t launches0 = g_launches;
+        const int64_t launches0 = g_launches.mark();
         BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         const cudaError_t e1 = launch_steps(b, cur, graph_steps(b), false);
         const cudaError_t e3 = cudaStreamEndCapture(b->stream, &g);
-        b->graph_launches = g_launches - launches0;
-        g_launches = launches0;  // counted when replayed
+        b->graph_launches = g_launches.take(launches0);  // counted when replayed
         if (e1 != cudaSuccess || e3 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             return set_error(LBM_ERR_CUDA, "batch graph capture failed: %s",
@@ -603,13 +602,12 @@ static int batch_period_graph(lbm_batch *b, int cur, int period, cudaGraphExec_t
     }
     if (!b->run_graph[cur]) {
         cudaGraph_t g = nullptr;
-        const int64_t launches0 = g_launches;
+        const int64_t launches0 = g_launches.mark();
         BCU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = launch_steps(b, cur, period, true);
         if (e == cudaSuccess) e = run_check_batch(b->dev, b->d_idx, b->nidx, period, b->stream);
         const cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-        b->run_graph_launches = g_launches - launches0;
-        g_launches = launches0;  // counted when replayed
+        b->run_graph_launches = g_launches.take(launches0);  // counted when replayed
         if (e != cudaSuccess || e2 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             return set_error(LBM_ERR_CUDA, "batch check-period graph capture: %s",

@@ -81,7 +81,7 @@ extern "C" const char *lbm_error_string(int status)
 
 extern "C" const char *lbm_last_error(void) { return t_last_error.c_str(); }
 
-extern "C" int64_t lbm_kernel_launches(void) { return g_launches; }
+extern "C" int64_t lbm_kernel_launches(void) { return g_launches.total(); }
 
 // ---------------------------------------------------------------------------
 // mesh() and initial() host arithmetic
@@ -1139,14 +1139,13 @@ static int graph_steps(const lbm_handle *h) { return 8 * (h->tile.T > 1 ? h->til
 
 // end the capture begun on h's stream: *out holds the instantiated graph and
 // *launches the kernels one replay launches.  e: the captured launches' status,
-// launches0: g_launches before them
+// launches0: this thread's mark (LaunchCount) before them
 static int end_capture(lbm_handle *h, cudaError_t e, int64_t launches0, cudaGraphExec_t *out, int64_t *launches,
                        const char *what)
 {
     cudaGraph_t g = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
-    *launches = lbm::g_launches - launches0;
-    lbm::g_launches = launches0;  // counted when replayed
+    *launches = lbm::g_launches.take(launches0);  // counted when replayed
     if (e != cudaSuccess || e2 != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
         return fail(LBM_ERR_CUDA, "%s graph capture: %s", what, cudaGetErrorString(e != cudaSuccess ? e : e2));
@@ -1161,7 +1160,7 @@ static int end_capture(lbm_handle *h, cudaError_t e, int64_t launches0, cudaGrap
 static int step_graph(lbm_handle *h, int cur, cudaGraphExec_t *out)
 {
     if (!h->graph[cur]) {
-        const int64_t l0 = lbm::g_launches;
+        const int64_t l0 = lbm::g_launches.mark();
         CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         const cudaError_t e = launch_steps(h, cur, graph_steps(h), false);
         int st = end_capture(h, e, l0, &h->graph[cur], &h->graph_launches, "step");
@@ -1266,7 +1265,7 @@ static int period_graph(lbm_handle *h, int cur, int period, cudaGraphExec_t *out
         h->run_graph_period = period;
     }
     if (!h->run_graph[cur]) {
-        const int64_t l0 = lbm::g_launches;
+        const int64_t l0 = lbm::g_launches.mark();
         CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = launch_steps(h, cur, period, true);
         if (e == cudaSuccess) e = run_check(h->geo, h->bufs, period, h->stream);

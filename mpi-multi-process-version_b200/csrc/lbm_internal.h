@@ -7,6 +7,8 @@
 
 #include <vector>
 
+#include "lbm_shared.h"
+
 namespace lbm {
 
 // Geometry and physics constants a kernel needs, passed by value.
@@ -224,7 +226,7 @@ cudaError_t convert_state(const Geo &g, int src_store, int dst_store, int nq, co
 cudaError_t macro_from_pops(const Geo &g, int store, const void *pop, const Bufs &b,
                             cudaStream_t s);
 
-extern int64_t g_launches;  // kernels launched by this library
+extern LaunchCount g_launches;  // kernels launched by this library
 
 // record a message for lbm_last_error() and return code
 int set_error(int code, const char *fmt, ...);

@@ -27,7 +27,6 @@
 #include <stdint.h>
 
 #include "lbm_internal.h"
-#include "lbm_shared.h"
 
 #ifndef LBM_EXACT
 #define LBM_EXACT 0

@@ -39,10 +39,11 @@
 #include <mutex>
 
 #include "../../include/lbm_b200.h"
+#include "lbm_shared.h"
 
 namespace lbm {
 int set_error(int code, const char *fmt, ...);
-extern int64_t g_launches;
+extern LaunchCount g_launches;
 }
 
 namespace {

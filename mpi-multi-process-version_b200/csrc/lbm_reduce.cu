@@ -12,7 +12,7 @@
 
 namespace lbm {
 
-int64_t g_launches = 0;
+LaunchCount g_launches;
 
 static constexpr int kRedBlocks = 592;  // 4 x 148 SMs
 static constexpr int kRedThreads = 256;

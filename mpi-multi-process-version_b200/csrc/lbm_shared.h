@@ -25,5 +25,33 @@ public:
     }
 };
 
+// Kernels launched, by all threads.  A thread that captures a graph takes its own
+// launches since a mark out of the count again: they count when the graph is
+// replayed, and other threads' launches in the meantime count as ever.
+class LaunchCount {
+    std::atomic<int64_t> total_{0};
+    static int64_t &mine()
+    {
+        static thread_local int64_t n = 0;
+        return n;
+    }
+
+public:
+    void operator+=(int64_t n)
+    {
+        total_ += n;
+        mine() += n;
+    }
+    void operator++() { *this += 1; }
+    int64_t total() const { return total_; }
+    int64_t mark() const { return mine(); }
+    int64_t take(int64_t mark)
+    {
+        const int64_t n = mine() - mark;
+        *this += -n;
+        return n;
+    }
+};
+
 }  // namespace lbm
 #endif

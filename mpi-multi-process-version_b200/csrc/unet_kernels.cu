@@ -24,10 +24,11 @@
 
 #include "../../include/lbm_b200.h"
 #include "../../include/lbm_surrogate.h"
+#include "lbm_shared.h"
 
 namespace lbm {
 int set_error(int code, const char *fmt, ...);
-extern int64_t g_launches;
+extern LaunchCount g_launches;
 void *tensor_map_encoder();  // cuTensorMapEncodeTiled, NULL if there is none
 }  // namespace lbm
 

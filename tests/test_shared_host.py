@@ -1,5 +1,6 @@
 """The library's shared host-side bookkeeping (csrc/lbm_shared.h), compiled by
-itself: set-up calls that hold for one device are made for each device."""
+itself: set-up calls that hold for one device are made for each device, and
+launches counted by one thread survive another thread's graph capture."""
 import os
 import subprocess
 
@@ -10,6 +11,7 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 PROGRAM = r"""
 #include "lbm_shared.h"
 #include <stdio.h>
+#include <thread>
 enum Err { kOk = 0, kBad = 1 };
 int main()
 {
@@ -21,6 +23,16 @@ int main()
     if (once.run(0, bad) != kOk || calls != 2) return 2;                                  // done on device 0
     if (once.run(1, ok) != kOk || calls != 3 || once.run(1, bad) != kOk || calls != 3) return 3;  // device 1: its own
     if (once.run(70, ok) != kOk || once.run(70, ok) != kOk || calls != 5) return 4;       // beyond the mask: every time
+    lbm::LaunchCount n;
+    n += 2;
+    const int64_t mark = n.mark();
+    ++n;
+    std::thread other([&] { for (int k = 0; k < 1000; ++k) ++n; const int64_t m = n.mark(); n += 5; if (n.take(m) != 5) ++n; });
+    n += 3;
+    other.join();
+    if (n.take(mark) != 4) return 5;          // this thread's own
+    if (n.total() != 1002) return 6;          // the other thread's stay
+    if (n.mark() != mark) return 7;
     puts("ok");
     return 0;
 }
