@@ -59,7 +59,10 @@ extern "C" {
                               bit-identical to the CPU restatement */
 
 /* options for lbm_set_option / lbm_get_option */
-#define LBM_OPT_KERNEL   1  /* step kernel: 0 automatic, 1 direct-load, 2 TMA march */
+#define LBM_OPT_KERNEL   1  /* step kernel: 0 automatic, 1 direct-load, 2 TMA march.  Automatic: the
+                               march from 2^15 nodes on, else direct-load (lbm_get_option names
+                               this one); 2D fast domains of up to some 10^5 nodes advance several
+                               steps at a time in shared memory beside it */
 #define LBM_OPT_NBLOCKS  2  /* persistent blocks of the march kernel (0 = automatic) */
 #define LBM_OPT_L2PROMO  3  /* L2 fetch promotion of the march kernel's TMA boxes:
                                0 none, 1 64 B, 2 128 B, 3 256 B */

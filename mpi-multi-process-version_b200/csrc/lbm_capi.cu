@@ -703,7 +703,8 @@ static int ensure_plan(lbm_handle *h)
 {
     if (!h->plan_dirty) return LBM_OK;
     const Geo &g = h->geo;
-    if (g.jlo == 0 && g.jhi == g.ny && g.nnode <= (1 << 18))
+    // a march that was asked for is one
+    if (h->kernel_opt != 2 && g.jlo == 0 && g.jhi == g.ny && g.nnode <= (1 << 18))
         h->tile = lbm::plan_tile2d(g.nx, g.ny, (int)h->esize, h->sms);
     if (h->tile.T > 1) {
         h->plan_dirty = false;
