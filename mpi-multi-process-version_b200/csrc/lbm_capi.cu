@@ -723,6 +723,11 @@ static int ensure_plan(lbm_handle *h)
         for (int o : of) off.push_back(o + (int)segs.size());
         segs.insert(segs.end(), sg.begin(), sg.end());
     }
+    // a stream that is being captured (a batch member's first steps; other handles planned at their init call) takes no
+    // upload: single steps until there is one
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(h->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return LBM_OK;
     int st = upload_segs(h, segs, off);
     if (!st) h->plan_dirty = false;
     return st;
@@ -1102,7 +1107,7 @@ static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
             left -= T;
             cur = 1 - cur;
         }
-    } else if (h->levels > 1 && !h->resident) {
+    } else if (h->levels > 1 && !h->plan_dirty && !h->resident) {
         const lbm::Launches n = lbm::launches_2d(left, h->levels);
         for (int k = 0; k < n.four + n.two && e == cudaSuccess; ++k) {
             const int T = k < n.four ? 4 : 2;
