@@ -105,7 +105,7 @@ def nn():
 
 def _chk(st, what):
     if st != 0:
-        raise L.LBMError(st, f"{what}: {L.lib().lbm_last_error().decode()}")
+        raise L.LBMError(st, what, L.lib().lbm_last_error().decode())
 
 
 def layer_table():

@@ -27,6 +27,13 @@ def descriptor(pkg, B, R):
     return d
 
 
+def test_a_refused_call_raises_the_librarys_error(pkg):
+    S = pkg.surrogate
+    with pytest.raises(pkg.LBMError, match="path must be 0") as e:
+        S.set_tensor_path(7)
+    assert e.value.status == ERR_PARAM
+
+
 # the scratch is set by the weight gradient; by the column sums, of which the calls before them know nothing
 @pytest.mark.parametrize("B,R", [(1, 16), (1, 128), (40, 16), (3, 24)])
 def test_backward_refuses_a_small_workspace(pkg, B, R):
