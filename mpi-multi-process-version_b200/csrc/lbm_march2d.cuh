@@ -315,7 +315,13 @@ __device__ __forceinline__ void march2d_levels(const int4 *__restrict__ segs, in
             }
             // a wait that ran out in iteration it is noted in word it & 1 and acted on, by every thread alike,
             // at the end of the next one (the test stays off the row's critical path)
-            if (!ok) iss[2 + (it & 1)] = 1;
+            if (!ok) {
+                iss[2 + (it & 1)] = 1;
+                if (tid == 0) {  // and no copy into a slot whose last one this thread has not seen land; their number stays
+                    iss[1] = iss[1] + iss[0] - (1 << 30);
+                    iss[0] = 1 << 30;
+                }
+            }
             const int failed = iss[2 + ((it + 1) & 1)];
             __syncthreads();
             if (failed) {

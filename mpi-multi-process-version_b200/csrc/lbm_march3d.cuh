@@ -257,9 +257,10 @@ __device__ __forceinline__ void march3d_run(const int4 *__restrict__ segs, int s
 
         for (int m = ka; m < kb; ++m) {
             const int k = slice(m);
-            // refill the slots of the slices read last step: z-slice m - 1, plane slice m - 1
-            if (zissued < min(seg_hi, m + ZS - 1)) issue_z(++zissued);
-            if (nissued < min(kb - 1, m + NS - 1)) issue_n(++nissued);
+            // refill the slots of the slices read last step: z-slice m - 1, plane slice m - 1 (not after a wait above
+            // that gave up: a slot takes no copy before its last one was seen to land)
+            if (ok && zissued < min(seg_hi, m + ZS - 1)) issue_z(++zissued);
+            if (ok && nissued < min(kb - 1, m + NS - 1)) issue_n(++nissued);
 
             const int64_t id = (int64_t)k * G.slab + (int64_t)j * G.pitch + i;
             const bool end = m == 0 || m == nz - 1;
