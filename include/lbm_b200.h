@@ -419,6 +419,18 @@ int lbm_march_plan3d(int32_t ntiles, int32_t nz, int32_t nblocks, int32_t kind,
                      int32_t *seg_count, int32_t *segs, int32_t *off,
                      int32_t *blocks_used);
 
+/* The same of the 2D launches of several steps (fast build).  lbm_march_plan2d:
+ * `levels` (2 or 4) steps of a domain of nx x ny nodes by at most `nblocks`
+ * blocks whose rows have at most `columns` nodes; segs receives (first column,
+ * columns, first row, end row) per segment.  lbm_tile_plan2d: the tiles of a
+ * small domain for values of esize bytes (4 or 8) on a device of `sms` SMs:
+ * tiles in x and in y, steps of a launch (0: the march is the better choice),
+ * nodes a patch has room for, threads and bytes of shared memory of a block. */
+int lbm_march_plan2d(int32_t nx, int32_t ny, int32_t columns, int32_t levels, int32_t nblocks,
+                     int32_t *seg_count, int32_t *segs, int32_t *off,
+                     int32_t *blocks_used);
+int lbm_tile_plan2d(int32_t nx, int32_t ny, int32_t esize, int32_t sms, int32_t plan[6]);
+
 #ifdef __cplusplus
 }
 #endif

@@ -755,6 +755,42 @@ extern "C" int lbm_march_plan3d(int32_t ntiles, int32_t nz, int32_t nblocks, int
     return LBM_OK;
 }
 
+extern "C" int lbm_march_plan2d(int32_t nx, int32_t ny, int32_t columns, int32_t levels, int32_t nblocks,
+                                int32_t *seg_count, int32_t *segs, int32_t *off, int32_t *blocks_used)
+{
+    if (nx < 3 || ny < 3 || (columns != 32 && columns != 64 && columns != 128) || (levels != 2 && levels != 4) ||
+        nblocks < 1 || !seg_count)
+        return fail(LBM_ERR_PARAM, "lbm_march_plan2d: bad arguments");
+    std::vector<lbm::Strip2> strips;
+    lbm::strips_march2d(0, nx, 0, ny, ny, columns, levels, strips);
+    std::vector<int4> sg;
+    std::vector<int> of;
+    const int nb = lbm::plan_march2d(strips, levels, nblocks, sg, of);
+    const int cap = *seg_count;
+    *seg_count = (int32_t)sg.size();
+    if (blocks_used) *blocks_used = nb;
+    if (!segs || !off) return LBM_OK;  // size query
+    if ((int)sg.size() > cap) return fail(LBM_ERR_PARAM, "lbm_march_plan2d: %d segments do not fit", (int)sg.size());
+    for (size_t i = 0; i < sg.size(); ++i) {
+        segs[4 * i] = sg[i].y;
+        segs[4 * i + 1] = (int32_t)((uint32_t)sg[i].x >> 24);
+        segs[4 * i + 2] = sg[i].z;
+        segs[4 * i + 3] = sg[i].w;
+    }
+    for (int b = 0; b <= nb; ++b) off[b] = of[b];
+    return LBM_OK;
+}
+
+extern "C" int lbm_tile_plan2d(int32_t nx, int32_t ny, int32_t esize, int32_t sms, int32_t plan[6])
+{
+    if (nx < 3 || ny < 3 || (esize != 4 && esize != 8) || sms < 1 || !plan)
+        return fail(LBM_ERR_PARAM, "lbm_tile_plan2d: bad arguments");
+    const lbm::TilePlan t = lbm::plan_tile2d(nx, ny, esize, sms);
+    const int32_t v[6] = {t.ntx, t.nty, t.T, t.en, t.threads, t.smem};
+    for (int k = 0; k < 6; ++k) plan[k] = v[k];
+    return LBM_OK;
+}
+
 static int resolve_path(lbm_handle *h)
 {
     lbm::drop_graphs(h);
