@@ -39,11 +39,11 @@ class LaunchCount {
 public:
     void operator+=(int64_t n)
     {
-        total_ += n;
+        total_.fetch_add(n, std::memory_order_relaxed);
         mine() += n;
     }
     void operator++() { *this += 1; }
-    int64_t total() const { return total_; }
+    int64_t total() const { return total_.load(std::memory_order_relaxed); }
     int64_t mark() const { return mine(); }
     int64_t take(int64_t mark)
     {

@@ -879,43 +879,26 @@ __device__ __forceinline__ void nn_mbar_init(uint64_t *b, uint32_t n)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
 }
 
-__device__ __forceinline__ bool nn_mbar_test(uint64_t *b, uint32_t parity)
+// a wait suspends the thread until the phase completes, `hint` ns at most
+__device__ __forceinline__ bool nn_mbar_test(uint64_t *b, uint32_t parity, uint32_t hint)
 {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(smem_u32(b)), "r"(parity)
+        : "r"(smem_u32(b)), "r"(parity), "r"(hint)
         : "memory");
     return ok != 0;
 }
 
-// try_wait may suspend the thread for a while; limits below this poll with test_wait, so that they can run out before
-// a copy in flight lands (the error path's test)
-constexpr long long kNnShortWait = 1000000LL;
-
 __device__ __forceinline__ bool nn_mbar_wait(uint64_t *b, uint32_t parity, long long limit = kNnWaitCycles)
 {
-    if (limit < kNnShortWait) {
-        const long long t0 = clock64();
-        uint32_t ok = 0;
-        while (true) {
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}\n"
-                : "=r"(ok)
-                : "r"(smem_u32(b)), "r"(parity)
-                : "memory");
-            if (ok) return true;
-            if (clock64() - t0 > limit) return false;
-        }
-    }
-    if (nn_mbar_test(b, parity)) return true;
+    const uint32_t hint = limit < kNnWaitCycles ? 1u : 1000000u;  // short limits must be able to run out (tests)
+    if (nn_mbar_test(b, parity, hint)) return true;
     const long long t0 = clock64();
-    while (!nn_mbar_test(b, parity))
+    while (!nn_mbar_test(b, parity, hint))
         if (clock64() - t0 > limit) return false;
     return true;
 }
