@@ -1143,7 +1143,7 @@ static cudaError_t launch_steps(lbm_handle *h, int cur, int n, bool with_macro)
             left -= T;
             cur = 1 - cur;
         }
-    } else if (h->levels > 1 && !h->plan_dirty && !h->resident) {
+    } else if (h->levels > 1 && h->tile.T <= 1 && !h->plan_dirty && !h->resident) {
         const lbm::Launches n = lbm::launches_2d(left, h->levels);
         for (int k = 0; k < n.four + n.two && e == cudaSuccess; ++k) {
             const int T = k < n.four ? 4 : 2;

@@ -740,7 +740,15 @@ __device__ __forceinline__ void march2d_node(const unsigned char *sm, const Geo 
     collide2d<C, false, false>(f, gg, rho, u, v, T, G, fp, gp, Fy);
 #else
     C yp[3], ym[3];
-    window_weights<C>(wy, j, ny, yp, ym);
+    if (j > 0 && j < ny - 1) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            yp[k] = C(wy[k]);
+            ym[k] = C(wy[3 + k]);
+        }
+    } else {
+        window_weights<C>(wy, j, ny, yp, ym);
+    }
     const int xo = win_lo(i, G.nx) - i, r0 = win_lo(j, ny);
     // x-interpolation of a plane's row in box b, and of the y-ring's plane yi over the rows of j's window
     auto XI = [&](const unsigned char *b, const C *w) -> C {
