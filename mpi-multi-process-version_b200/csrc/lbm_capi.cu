@@ -646,11 +646,33 @@ static int upload_segs(lbm_handle *h, const std::vector<int4> &segs, const std::
     return LBM_OK;
 }
 
-// plan the 3D march for grid G and upload it; sets h->nblocks
-static int upload_plan3d(lbm_handle *h, int G)
+// The blocks of the 3D march of `slots` that are resident at once, for ntiles tile
+// columns.  The fast build in FP64 reaches the copy bandwidth with fewer: blocks
+// whose segments lie across the others' slices (the plan's tails) then cost it
+// more than they carry.  Up to 2^20 nodes (the state partly in L2) all slots; beyond,
+// whole chunks alone where they fill 85 % of them, else nine tenths.  us a step, in
+// a burst of 100 / in a run of seconds at the board's power limit: 128^3 all 167 / 163,
+// this 156 / 167 (three slices read per output: 156 / 174); 160^3 327 / 322, this 315 / 330
+// (314 / 350); 144 x 140 x 130 214 / 224, this 205 / 224 (222 / 245); 192 x 160 x 100 243 / 235,
+// this 233 / 247 (225 / 256).  FP32 is bound by issue and takes them all (128^3 84 / 90,
+// nine tenths 86 / 95), except where one chunk a column fills them: 256 x 256 x 64 191 / 179,
+// this 182 / 188 (178 / 198).
+static int march3d_blocks(const lbm_handle *h, int ntiles, int slots)
+{
+    const int grid = slots / ntiles * ntiles;
+    if (h->p.mode == LBM_MODE_EXACT || h->geo.nnode < (1 << 20) || grid == 0) return slots;
+    const bool f64 = h->p.storage == LBM_STORE_F64;
+    if (grid * 20 >= slots * 17 && (f64 || grid == ntiles)) return grid;
+    return f64 ? std::max(grid, slots * 9 / 10) : slots;
+}
+
+// plan the 3D march for at most `slots` blocks, or as many as LBM_OPT_NBLOCKS says,
+// and upload it; sets h->nblocks
+static int upload_plan3d(lbm_handle *h, int slots)
 {
     const MarchShape ms = march_shape(3, h->p.storage, 0, h->tiley);
     const int ntiles = ((h->geo.nx + ms.TX - 1) / ms.TX) * ((h->geo.ny + ms.TY - 1) / ms.TY);
+    const int G = h->nblocks_opt > 0 ? h->nblocks_opt : march3d_blocks(h, ntiles, slots);
     std::vector<int4> segs;
     std::vector<int> off;
     // the slices the handle computes: all of them, or a slab's own [klo, khi)
@@ -819,8 +841,7 @@ static int resolve_path(lbm_handle *h)
         CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
         const int slots = bps * sms;
         if (h->geo.dim == 3) {
-            // one full wave, planned
-            int st = upload_plan3d(h, h->nblocks_opt > 0 ? h->nblocks_opt : slots);
+            int st = upload_plan3d(h, slots);  // one wave, planned
             if (st) return st;
         } else if (h->nblocks_opt > 0) {
             h->nblocks = h->nblocks_opt;
