@@ -96,9 +96,9 @@ struct lbm_batch {
 // time steps of a multi-step launch of the 2D kernel (the exact build and 3D: 1).
 // Four levels share the launch and a segment's pipeline fill; large FP32 batches,
 // bound by issue rather than by HBM, do better with the narrower halo of two.
-// Measured, us a step at 1 / 2 / 4 levels (64 columns): FP64 sweep of 32 cavities
-// 390 / 237 / 206, 16 squares 25.1 / 20.3 / 19.2, one 7.27 / 5.26 / 4.78; FP32
-// 244 / 158 / 165, 17.5 / 15.9 / 15.5, 7.26 / 4.76 / 4.02.
+// Measured, us a step, single steps / 2 / 4 levels (64 columns): FP64 sweep of 32
+// cavities 401 / 237 / 206, 16 squares 32 / 20.3 / 19.2, one 5.3 / 5.26 / 4.78; FP32
+// 235 / 158 / 165, 25 / 15.9 / 15.5, 5.4 / 4.76 / 4.02.
 static int batch_levels(const lbm_batch *b)
 {
     if (b->dim != 2 || b->mode == LBM_MODE_EXACT) return 1;
@@ -231,6 +231,36 @@ extern "C" int lbm_batch_create(int32_t n, const lbm_params *params, const doubl
     return LBM_OK;
 }
 
+// a column of the work list; pos: 2D the strip's x-offset, 3D the tile index; ny: items (rows or slices)
+struct Col {
+    int cav, pos, ny;
+};
+
+// One chunk a block (3D, fast build): the shortest length that cuts the columns into at
+// most G chunks, 0 where that leaves the blocks idle.  Chunks that start together keep
+// neighbouring tiles at the same slice, so that their halos come from L2, and a segment's
+// start is the dearer since a slice is interpolated once; equal contiguous shares do
+// neither.  us a step, shares with three slices read per output / with one / chunks:
+// eight cubes of 64^3 FP64 187 / 199 / 158, FP32 119 / 119 / 100; two of 128^3 FP32 229 /
+// 256 / 193; three of 80^3 FP32 107 / 120 / 86.  The line lies at 5/8 of the blocks' time:
+// four unlike boxes that fill 0.64 of it 140 / 148 / 142, six that fill 0.63 137 / 138 / 134,
+// but three of 80^3 FP64, 0.61 of it in 180 chunks for 296 blocks, 155 / 163 / 188.
+static int chunk_length(const std::vector<Col> &cols, int64_t total, int64_t G)
+{
+    if (cols.empty() || (int64_t)cols.size() > G) return 0;
+    int hi = 1;
+    for (const Col &q : cols) hi = std::max(hi, q.ny);
+    int lo = 1;
+    while (lo < hi) {
+        const int m = (lo + hi) / 2;
+        int64_t n = 0;
+        for (const Col &q : cols) n += (q.ny + m - 1) / m;
+        if (n <= G) hi = m;
+        else lo = m + 1;
+    }
+    return total * 8 >= G * lo * 5 ? lo : 0;
+}
+
 // descriptors for the tile width, and the work lists of the active cavities.
 // A column is one march: 2D a TX-wide strip of rows, 3D a 32 x kBatchTileY tile
 // of slices.  Each storage's list keeps a fixed grid (a full wave, or the
@@ -260,9 +290,6 @@ static int build_tables(lbm_batch *b)
 
     bool regraph = b->levels != batch_levels(b);
     b->levels = batch_levels(b);
-    struct Col {
-        int cav, pos, ny;  // pos: 2D the strip's x-offset, 3D the tile index; ny: items (rows or slices)
-    };
     std::vector<Col> cols;
     std::vector<Strip2> strips[3];  // of the active members, per launch of 2 and 4 steps ([1], [2])
     size_t ncols_all = 0;  // the columns of every member, active or not: the lists' capacity
@@ -330,6 +357,16 @@ static int build_tables(lbm_batch *b)
                 plan_march2d(mine, 1 << l, (int)G, sg, of);
                 for (int o : of) off.push_back(o + (int)segs.size());
                 segs.insert(segs.end(), sg.begin(), sg.end());
+                continue;
+            }
+            const int len = d3 && b->mode != LBM_MODE_EXACT ? chunk_length(sc, stotal, G) : 0;
+            if (len > 0) {
+                for (const Col &q : sc)
+                    for (int n = (q.ny + len - 1) / len, k = 0; k < n; ++k) {
+                        off.push_back((int)segs.size());
+                        segs.push_back(make_int4(q.pos, (int)((int64_t)k * q.ny / n), (int)((int64_t)(k + 1) * q.ny / n), q.cav));
+                    }
+                off.resize(off0[l] + (size_t)G + 1, (int)segs.size());
                 continue;
             }
             size_t c = 0;

@@ -18,15 +18,16 @@
 //     reads a node instead of 62, 48 multiply-adds instead of 84);
 //   * one tensor copy fetches all 14 population planes of a row (one more the
 //     carried force).
-// Measured, FP64, us a step, one level per pass in the earlier kernel (62 reads a
-// node, one copy per plane) against this one: 513^2 13.5 -> 9.9, 700x900 27.5 ->
-// 18.5, 1024^2 48.0 -> 28.1, 2048^2 178 -> 105 (9.6 TB/s of the 240 bytes an update
-// moves at one level); FP32: 512^2 9.2 -> 7.7, 1023x771 23.7 -> 17.0, 2048^2 106 ->
-// 78; a batch of 32 cavities FP64 404 -> 206.  What bounds it now: 440 instructions
-// a row and warp (164 FP64, 54 shared-memory) at 16 warps per SM issue 53 % of the
-// time; HBM is at 42 %.  Two columns per thread (300 instructions) needed 254
-// registers and was no faster; 16 warps in blocks of two 64-column levels with a
-// three-slot input ring neither.
+// Measured, FP64, us a step, one level per pass (k_march2d: 62 reads a node, one
+// copy per plane) against this one: 513^2 13.5 -> 9.9, 700x900 27.5 ->
+// 18.5, 1024^2 48.0 -> 28.1, 2048^2 178 -> 105 (1.46 times what one pass per step
+// could reach); FP32: 512^2 9.2 -> 7.7, 1023x771 23.7 -> 17.0, 2048^2 106 ->
+// 78; a batch of 32 cavities FP64 404 -> 206.  What bounds it now: 470 instructions
+// per 32 updates at 2048^2 (185 FP64; 519 and 202 in a batch at four levels, halo
+// included) issue 54 to 56 % of the time at 12 to 15 warps per SM, in FP32 65 to
+// 71 %; HBM is at 55 % there and at 34 % in the batch.  Two columns per thread needed
+// 254 registers and was no faster; 16 warps in blocks of two 64-column levels with
+// a three-slot input ring neither.
 // Level s of rows [ja, jb) x columns [x0, x0 + w) needs T - s more nodes on
 // each side; those are computed twice (by the neighbouring segment too): 2 of
 // 126 columns and 2 rows per segment at T = 2.

@@ -8,7 +8,7 @@
 // once, when a slice arrives; a thread keeps the values of the last two slices
 // in registers.  Reading all three slices for every output instead (as the
 // direct-load kernel does) takes 84 loads from shared memory where this takes
-// 28, 152 against 96 in all, and a 9 % lower instruction count.  Two planes a
+// 28, 152 against 96 in all: 63.5 M warp instructions a launch at 128^3 instead of 70.0 M.  Two planes a
 // TMA copy halve the copies, which one thread issues (FP64 128^3: 16 copies a
 // slice instead of 30; single planes cost 3 % in FP32, 9 % at 61 x 50 x 47).
 //
@@ -16,8 +16,8 @@
 // (1000 W, the clock down to 1.6 GHz), so work saved is time saved even where
 // memory bandwidth would hide it; in L2 the latency of a slice, 2.4 us with two
 // blocks an SM.  Measured, us a step, all three slices read -> this: long runs at
-// 128^3 FP64 175 -> 163, FP32 102 -> 88, 96^3 FP64 75 -> 69; short ones 61 x 50 x 47
-// FP64 15.6 -> 14.2, 131 x 118 x 125 FP64 214 -> 195, FP32 107 -> 100.
+// 128^3 FP64 169 -> 164, FP32 96 -> 85, 96^3 FP64 74 -> 69; shorter ones 61 x 50 x 47
+// FP64 16.6 -> 14.8, 131 x 118 x 125 FP64 215 -> 199, FP32 110 -> 101.
 //
 // Steps that read buffer 1 walk downwards (`rev`): the slices the last step
 // wrote last, partly still in L2, are read first (1 to 2 % in long runs at 128^3;

@@ -40,8 +40,8 @@ constexpr int kThreads = 256;
 
 // Every kernel here but k_conv3x3 is launched as a programmatic dependent of the one before: its
 // blocks may be set up while that one still runs, and it reads and writes only
-// after dep_sync.  118 launches a training step (batch 16, 128 x 128): 1.86 ms as ordinary
-// launches, 1.73 so.
+// after dep_sync.  The 118 launches that a training step (batch 16, 128 x 128) then had:
+// 1.86 ms as ordinary launches, 1.73 so.
 __device__ __forceinline__ void dep_sync()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -859,9 +859,9 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 //     kernel before;
 //   * the epilogue reads the accumulators with tcgen05.ld, a thread one pixel and
 //     16 channels at a time, and stores whole 32-byte sectors.
-// Measured at batch 16 of 128^2 images, all forward and data-gradient layers of
+// Measured at batch 16 of 128^2 images, all 27 forward and data-gradient layers of
 // a training step: mma.sync kernel 1.64 ms, with copies by all threads 1.01 ms,
-// this kernel 0.86 ms; 256 -> 256 at 16 x 16, batch 1: 53, 24 and 14 us.
+// this kernel 0.54 ms; 256 -> 256 at 16 x 16, batch 1: 53, 24 and 8.9 us.
 // Every mbarrier wait is bounded; on timeout the CTA counts the event in
 // g_nn_timeouts (read by lbm_nn_timeouts), waits (bounded) for its own copies and
 // MMAs, stores NaN in place of its results, so that nothing downstream takes what an
@@ -1797,7 +1797,8 @@ extern "C" int lbm_nn_set_wait_limit(int64_t cycles)
 // ---------------------------------------------------------------------------
 // One call issues the pass's launches: from Python each launch is a foreign call
 // of some twenty arguments, 8 us, as much as the kernels take at batch 1.  One
-// prediction at 128 x 128: the host's share 175 -> 91 us, the pass 173 -> 156 us.
+// prediction at 128 x 128: the host's share 175 -> 91 us, the pass 173 -> 156 us
+// (with the kernels since: 78 and 112).
 #define NN_DO(call)                   \
     do {                              \
         const int st_ = (call);       \
