@@ -66,12 +66,13 @@ extern "C" {
 #define LBM_OPT_NBLOCKS  2  /* persistent blocks of the march kernel (0 = automatic) */
 #define LBM_OPT_L2PROMO  3  /* L2 fetch promotion of the march kernel's TMA boxes:
                                0 none, 1 64 B, 2 128 B, 3 256 B */
-#define LBM_OPT_GRAPHS   4  /* 1 (default): lbm_step replays captured 8-step CUDA graphs */
+#define LBM_OPT_GRAPHS   4  /* 1 (default): lbm_step replays captured CUDA graphs of eight launches
+                               (eight iterations; in 2D, fast build, up to 64) */
 #define LBM_OPT_RESIDENT 5  /* 0 (default) / 1: 2D domains of one resident wave run all iterations
                                of an lbm_step call in one cooperative launch with a bounded grid
-                               barrier between iterations.  Measured at 128^2 on B200: 3.87 us per
-                               iteration in FP32 (4.10 with graph-replayed launches) but 4.85 us
-                               in FP64, hence opt-in.  Batch members always step per iteration. */
+                               barrier between iterations.  Measured at 128^2 on B200, fast build:
+                               4.7 us per iteration in FP64, 4.2 in FP32, where the default's tiles
+                               take 2.1 and 1.8, hence opt-in.  Batch members never do. */
 #define LBM_OPT_TILEY    6  /* 3D march kernel tile rows: 0 automatic (4), 4 (two blocks per SM) or 8 */
 #define LBM_OPT_PLAN     7  /* 3D march work plan: 0 (default) every tile column in equal z-chunks
                                run side by side (neighbours share halo rows through L2), the blocks

@@ -405,8 +405,9 @@ static bool march_supported(const lbm_handle *h)
 }
 
 // tile rows of the 3D march kernel unless LBM_OPT_TILEY says otherwise: 32 x 4
-// tiles run two blocks per SM (four in FP32); a long run at 128^3 takes 163 us a
-// step in FP64 against 167 with 32 x 8 tiles and one block per SM, FP32 84 against 101
+// tiles run two blocks per SM (four in FP32); with every resident block a long run
+// at 128^3 takes 163 us a step in FP64 against 167 with 32 x 8 tiles and one block per
+// SM, FP32 84 against 101
 static constexpr int kDefaultTileY = 4;
 
 // ---------------------------------------------------------------------------

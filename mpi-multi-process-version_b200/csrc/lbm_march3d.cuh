@@ -15,9 +15,10 @@
 // What bounds it: at sizes past L2 a long run sits at the board's power limit
 // (1000 W, the clock down to 1.6 GHz), so work saved is time saved even where
 // memory bandwidth would hide it; in L2 the latency of a slice, 2.4 us with two
-// blocks an SM.  Measured, us a step, all three slices read -> this: long runs at
-// 128^3 FP64 169 -> 164, FP32 96 -> 85, 96^3 FP64 74 -> 69; shorter ones 61 x 50 x 47
-// FP64 16.6 -> 14.8, 131 x 118 x 125 FP64 215 -> 199, FP32 110 -> 101.
+// blocks an SM.  Measured, us a step, all three slices read -> this: runs of seconds
+// at 128^3 FP64 175 -> 167, FP32 102 -> 90; bursts of 100 steps 128^3 FP64 157 -> 156,
+// FP32 92 -> 85, 61 x 50 x 47 FP64 16.3 -> 14.7, 131 x 118 x 125 FP64 215 -> 191, FP32
+// 108 -> 101.  On how many blocks: march3d_blocks.
 //
 // Steps that read buffer 1 walk downwards (`rev`): the slices the last step
 // wrote last, partly still in L2, are read first (1 to 2 % in long runs at 128^3;
